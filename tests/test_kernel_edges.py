@@ -1,0 +1,94 @@
+"""Kernels and dispatch rules at the sizes where they can go wrong: host emulations of their
+index logic (CPU), and the device against the oracle or the general path (GPU)."""
+import numpy as np
+import pytest
+import torch
+
+import moraine_b200 as mb
+from oracle import oracle as O
+
+
+# ----------------------------------------------------------------------------- KS statistic
+def _merge_k(a, b):
+    """The reference's merge statistic (moraine/shp.py:36-44)."""
+    n, j1, j2, k = len(a), 0, 0, 0
+    while j1 < n and j2 < n:
+        le, ge = a[j1] <= b[j2], a[j1] >= b[j2]
+        j1 += le
+        j2 += ge
+        k = max(k, abs(j2 - j1))
+    return k
+
+
+def test_ks_walk_and_threshold_equal_the_merge():
+    """One-sided walks and the threshold test give the merge's statistic, ties and infinities
+    included, reading only inside a row of shared memory."""
+    rng = np.random.default_rng(3)
+    for n in (1, 2, 3, 4, 5, 7, 16, 17, 33, 50):
+        row = 4 * (((n + 11) >> 2) | 1)
+        for trial in range(60):
+            levels = (2, 5, 1000)[trial % 3]
+            a = np.sort(rng.integers(0, levels, n)).astype(np.float64)
+            b = np.sort(rng.integers(0, levels, n) + (trial % 4) * levels // 4).astype(np.float64)
+            if trial % 7 == 0:
+                b[-1] = np.inf
+            if trial % 11 == 0:
+                b = a.copy()
+            k = _merge_k(a, b)
+            t = [0, 0]
+            for s in range(n):
+                assert max(t) <= s
+                t = [t[0] + (not b[s] < a[t[0]]), t[1] + (not a[s] < b[t[1]])]
+            assert n - min(t) == k
+            assert (k == 0) == np.array_equal(a, b)
+            pad = np.full(row, np.inf)  # the sentinel: nothing lies below it
+            pa, pb = pad.copy(), pad.copy()
+            pa[:n], pb[:n] = a, b
+            for kth in range(1, n + 2):
+                groups = max(0, (n - kth + 4) >> 2)
+                assert 4 * ((kth - 1) >> 2) + 3 < row  # the first shifted word, read before the loop
+                hit = False
+                for g in range(groups):
+                    assert 4 * (g + ((kth - 1) >> 2) + 1) + 3 < row
+                    for i in range(4 * g, 4 * g + 4):
+                        hit |= pb[i + kth - 1] < pa[i] or pa[i + kth - 1] < pb[i]
+                assert hit == (k >= kth)
+
+
+def _select(x, azh, rh, p_max):
+    """mr_ks_test without p or dist: the chain's selection."""
+    from moraine_b200 import _dev, _lib
+    nl, w, n = x.shape
+    win = (2 * azh + 1) * (2 * rh + 1)
+    is_shp = torch.full((nl, w, win), 7, dtype=torch.uint8, device=x.device)
+    num = torch.full((nl, w), -1, dtype=torch.int32, device=x.device)
+    ws = _dev.workspace(_lib.load().mr_ks_workspace_bytes(nl, w, n), x.device)
+    _lib.call("mr_ks_test", x.data_ptr(), nl, w, n, azh, rh, None, None, p_max, is_shp.data_ptr(), num.data_ptr(),
+              ws.data_ptr(), ws.numel(), _dev.stream())
+    return is_shp.cpu().numpy().reshape(nl, w, 2 * azh + 1, 2 * rh + 1), num.cpu().numpy()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,azh,rh", [(1, 1, 1), (2, 2, 3), (5, 5, 5), (17, 5, 5), (32, 5, 10), (41, 7, 15),
+                                      (101, 5, 10), (150, 2, 15), (257, 1, 10), (512, 0, 4)])
+def test_ks_selection_without_p(cuda, n, azh, rh):
+    """The mask-only path equals p < p_max of the oracle's p, for every kind of threshold: the
+    usual ones, none or all accepted, and tables that accept neither an interval from above."""
+    rng = np.random.default_rng(n)
+    nl, w = (19, 37) if n < 200 else (7, 35)
+    x = rng.exponential(size=(nl, w, n)).astype(np.float32)
+    x[:, w // 2:] *= 2.5
+    x[3, 5] = x[3, 6]                # an identical neighbour: k = 0 off the centre
+    x[4, 7] = np.round(x[4, 7], 1)   # ties
+    x[4, 8] = np.round(x[4, 8], 1)
+    x[5, 9, 0] = np.nan
+    x[6, 3, -1] = np.inf
+    p = O.ks_test(x, azh, rh)
+    t = torch.from_numpy(x).to(cuda)
+    for p_max in (0.05, 0.5, 1e-6, 0.0, -1.0, 1.0, 2.5):
+        ref, num = O.select_shp(p, p_max)
+        got, got_num = _select(t, azh, rh, p_max)
+        np.testing.assert_array_equal(got.astype(bool), ref)
+        np.testing.assert_array_equal(got_num, num)
+        assert got.max() <= 1
+    np.testing.assert_array_equal(mb.ks_test(x, azh, rh), p)
