@@ -8,18 +8,19 @@
 //                          summed in window order (row-major over the az x r window)
 //   moraine/co.py:83-110   raster: cov = sum / n_shp, coh as above, every (m, j)
 #include <algorithm>
+#include <vector>
 
 #include "common.cuh"
 
 namespace mr {
 namespace {
 
-constexpr int kGramThreads = 256;
-constexpr int kChunk = 32;  // SHP rows staged per pass
-
-template <typename A> struct Acc2;
-template <> struct Acc2<float> { using type = float2; };
-template <> struct Acc2<double> { using type = double2; };
+// SHP rows staged per pass: `most`, or fewer (a power of two, at least 4) where `row_bytes` each
+// would take more than 64 KiB.
+int chunk_rows(int most, size_t row_bytes) {
+  while (most > 4 && most * row_bytes > 64 * 1024) most >>= 1;
+  return most;
+}
 
 // Block-wide compaction of a window mask into the linear pixel indices of the SHPs that
 // lie inside the image, in window order. Returns the count (same in every thread).
@@ -29,11 +30,12 @@ __device__ int collect_shps(const uint8_t* __restrict__ mask, int az_win, int r_
   const int azh = az_win / 2, rh = r_win / 2;
   const int per = (win + blockDim.x - 1) / blockDim.x;
   const int e0 = threadIdx.x * per, e1 = min(win, e0 + per);
+  const int k0 = e0 / r_win, l0 = e0 - k0 * r_win;
   int c = 0;
-  for (int e = e0; e < e1; ++e) {
-    int k = e / r_win, l = e - k * r_win;
-    int sa = ra - azh + k, sr = rr - rh + l;
+  for (int e = e0, k = k0, l = l0; e < e1; ++e) {
+    const int sa = ra - azh + k, sr = rr - rh + l;
     c += (mask[e] && sa >= 0 && sa < nlines && sr >= 0 && sr < width);
+    if (++l == r_win) { l = 0; ++k; }
   }
   // block exclusive scan of c
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -44,48 +46,113 @@ __device__ int collect_shps(const uint8_t* __restrict__ mask, int az_win, int r_
   }
   if (lane == 31) s_tmp[wid] = incl;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { int t = s_tmp[w]; s_tmp[w] = run; run += t; }
-    s_tmp[32] = run;
+  int before = 0, total = 0;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+    if (w < wid) before += s_tmp[w];
+    total += s_tmp[w];
   }
-  __syncthreads();
-  int pos = s_tmp[wid] + incl - c;
-  for (int e = e0; e < e1; ++e) {
-    int k = e / r_win, l = e - k * r_win;
-    int sa = ra - azh + k, sr = rr - rh + l;
+  int pos = before + incl - c;
+  for (int e = e0, k = k0, l = l0; e < e1; ++e) {
+    const int sa = ra - azh + k, sr = rr - rh + l;
     if (mask[e] && sa >= 0 && sa < nlines && sr >= 0 && sr < width) s_pos[pos++] = sa * width + sr;
+    if (++l == r_win) { l = 0; ++k; }
   }
-  __syncthreads();
-  int total = s_tmp[32];
   __syncthreads();
   return total;
 }
 
-// One CTA per point (grid-stride). Each thread accumulates a 4x4 block of the N x N
-// Gram over the point's SHPs, staged kChunk rows at a time in shared memory.
-// kFull = false: upper-triangle blocks, writes coh (n_pc, Q) in triu order.
-// kFull = true : all blocks, writes cov and coh (npix, N, N) (raster form).
+__device__ __forceinline__ void copy8(float2* dst, const float2* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// One CTA per point (grid-stride), a 4 x 4 block of the Gram's upper triangle per thread and
+// round, over the point's SHPs staged kc rows at a time. The launch gives a point only as many
+// warps as its blocks fill; several CTAs share an SM.
+// kFull = false: writes coh (n_pc, Q) in triu order.
+// kFull = true : writes cov and coh (npix, N, N) (raster form), the lower blocks as conjugates.
+//
+// A staged row holds its images in the arithmetic A, permuted so that the 16-byte words
+// that a thread reads lie 16 bytes from its neighbour's (no bank conflict): image 4 b + r at
+// position (r / V) V nb + V b + r % V, V images to a word.
+// FP32: cp.async into two buffers; the products re re, im im, im re and re im are summed apart, S
+// roundings each on partial sums of half the size: four FMAs per complex product (the sum of both
+// products rounded into one accumulator took six instructions and was less exact). FP64: fetched
+// by cp.async as stored, widened once when staged (at 16 conversions per clock and SM, widening at
+// each use cost as much time as the products themselves), one FMA chain per component. The sums
+// |z|^2 are the Gram's own diagonal: blocks (b, b) come first, in round 0.
+// FP32 is bound by its issue slots, FP64 by shared memory (eight 16-byte reads, four wavefronts
+// each, take as long as their 64 FP64 FMAs). FP32, N = 50, 15 x 31 window, 30,011 points: 1.65 ms
+// against 2.9 with a separate pass for |z|^2 and 256-thread CTAs; N = 20 raster of 123 x 131: 0.16
+// against 0.38 ms. FP64 at N = 150, 5,224 points of 166 SHPs: 5.2 against 5.4 ms.
+constexpr int kMaxGramThreads = 192;
+
+template <typename A> struct GramAcc;
+template <> struct GramAcc<float> {
+  float rr, ii, ir, ri;
+  __device__ __forceinline__ void add(float2 m, float2 j) {  // z_m conj(z_j)
+    rr = fmaf(m.x, j.x, rr);
+    ii = fmaf(m.y, j.y, ii);
+    ir = fmaf(m.y, j.x, ir);
+    ri = fmaf(m.x, j.y, ri);
+  }
+  __device__ __forceinline__ float re() const { return rr + ii; }
+  __device__ __forceinline__ float im() const { return ir - ri; }
+};
+template <> struct GramAcc<double> {
+  double x, y;
+  __device__ __forceinline__ void add(double2 m, double2 j) {
+    x = fma(m.x, j.x, x);
+    x = fma(m.y, j.y, x);
+    y = fma(m.y, j.x, y);
+    y = fma(-m.x, j.y, y);
+  }
+  __device__ __forceinline__ double re() const { return x; }
+  __device__ __forceinline__ double im() const { return y; }
+};
+
+// Images 4 b .. 4 b + 3 of a staged row.
+__device__ __forceinline__ void load_block(const float2* row, int nb, int b, float2 (&z)[4]) {
+  const float4 u = reinterpret_cast<const float4*>(row)[b], v = reinterpret_cast<const float4*>(row)[nb + b];
+  z[0] = make_float2(u.x, u.y);
+  z[1] = make_float2(u.z, u.w);
+  z[2] = make_float2(v.x, v.y);
+  z[3] = make_float2(v.z, v.w);
+}
+__device__ __forceinline__ void load_block(const double2* row, int nb, int b, double2 (&z)[4]) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r) z[r] = row[r * nb + b];
+}
+
 template <typename A, bool kFull>
-__global__ void __launch_bounds__(kGramThreads) gram_kernel(
+__global__ void __launch_bounds__(kMaxGramThreads, sizeof(A) == 8 ? 2 : 3) gram_kernel(
     const float2* __restrict__ rslc, int nlines, int width, int n, const int32_t* __restrict__ idx,
     int64_t n_pc, const uint8_t* __restrict__ mask, int mask_stride, int az_win, int r_win,
-    float2* __restrict__ coh, float2* __restrict__ cov, const int64_t* __restrict__ dcount, int64_t doff) {
-  using C = typename Acc2<A>::type;
+    float2* __restrict__ coh, float2* __restrict__ cov, const int64_t* __restrict__ dcount, int64_t doff, int kc) {
+  using C = typename cplx<A>::type;
+  constexpr bool kWide = sizeof(A) == 8;
+  constexpr int V = 16 / sizeof(C);  // images per 16-byte word
   if (dcount) {  // points doff .. doff + n_pc - 1 of a count held on the device
     const int64_t c = *dcount - doff;
     n_pc = c < 0 ? 0 : (c < n_pc ? c : n_pc);
   }
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int win = az_win * r_win;
-  const int npad = (n + 3) & ~3;
-  float2* zc = reinterpret_cast<float2*>(smem_raw);                  // kChunk x npad
-  A* amp2 = reinterpret_cast<A*>(zc + kChunk * npad);                 // npad
+  const int nb = (n + 3) >> 2, npad = 4 * nb;
+  C* zc = reinterpret_cast<C*>(smem_raw);                             // FP32: 2 x kc x npad; FP64: kc x npad
+  float2* raw = reinterpret_cast<float2*>(zc + (kWide ? 1 : 2) * kc * npad);  // FP64: kc x n, as fetched
+  A* amp2 = reinterpret_cast<A*>(raw + (kWide ? kc * n + (kc * n & 1) : 0));  // npad
   int* s_pos = reinterpret_cast<int*>(amp2 + npad);                   // win
-  __shared__ int s_tmp[33];
-  const int nb = npad / 4;
-  const int nblk = kFull ? nb * nb : nb * (nb + 1) / 2;
+  __shared__ int s_tmp[32];
+  const int nblk = nb * (nb + 1) / 2;
   const int64_t npairs = (int64_t)n * (n - 1) / 2;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  for (int e = tid; e < (kWide ? 1 : 2) * kc * npad; e += nt) zc[e] = cmake<C>(0, 0);  // padding images stay 0
+  // thread's staging walk over (row t, image c): nt elements ahead is (sdt, sdc)
+  const int t_first = tid / n, c_first = tid - t_first * n;
+  const int sdt = nt / n, sdc = nt - sdt * n;
+  const int rounds = (nblk + nt - 1) / nt;
+  __syncthreads();
 
   for (int64_t i = blockIdx.x; i < n_pc; i += gridDim.x) {
     int ra, rr;
@@ -94,86 +161,93 @@ __global__ void __launch_bounds__(kGramThreads) gram_kernel(
     if (ra < 0 || ra >= nlines || rr < 0 || rr >= width) {  // index outside the image: NaN row
       const float2 nan2 = make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
       if (kFull) {
-        for (int e = threadIdx.x; e < n * n; e += blockDim.x) { coh[i * n * n + e] = nan2; cov[i * n * n + e] = nan2; }
+        for (int e = tid; e < n * n; e += nt) { coh[i * n * n + e] = nan2; cov[i * n * n + e] = nan2; }
       } else {
-        for (int64_t e = threadIdx.x; e < npairs; e += blockDim.x) coh[i * npairs + e] = nan2;
+        for (int64_t e = tid; e < npairs; e += nt) coh[i * npairs + e] = nan2;
       }
       continue;
     }
     const uint8_t* m = mask + (mask_stride ? ((int64_t)ra * width + rr) : i) * win;
     const int S = collect_shps(m, az_win, r_win, ra, rr, nlines, width, s_pos, s_tmp);
-    // amplitude sums, window order
-    for (int c = threadIdx.x; c < npad; c += blockDim.x) {
-      A s = 0;
-      if (c < n)
-        for (int t = 0; t < S; ++t) {
-          float2 z = rslc[(int64_t)s_pos[t] * n + c];
-          s += (A)z.x * (A)z.x + (A)z.y * (A)z.y;
-        }
-      amp2[c] = s;
-    }
-    __syncthreads();
-    for (int round = 0; round * kGramThreads < nblk; ++round) {
-      const int blk = round * kGramThreads + threadIdx.x;
+    // fn(row t, image c) over this thread's elements of ns rows
+    auto each = [&](int ns, auto fn) {
+      int t = t_first, c = c_first;
+      while (t < ns) {
+        fn(t, c);
+        t += sdt;
+        c += sdc;
+        if (c >= n) { c -= n; ++t; }
+      }
+    };
+    auto place = [&](int t, int c) { return t * npad + (c & 3) / V * V * nb + (c >> 2) * V + (c & 3) % V; };
+    auto fetch = [&](int s0, int buf) {
+      each(min(kc, S - s0), [&](int t, int c) {
+        const float2* src = rslc + (int64_t)s_pos[s0 + t] * n + c;
+        if constexpr (kWide) copy8(raw + t * n + c, src);
+        else copy8(reinterpret_cast<float2*>(zc) + buf * kc * npad + place(t, c), src);
+      });
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int round = 0; round < rounds; ++round) {
+      const int blk = round * nt + tid;
       const bool active = blk < nblk;
       int bm = 0, bj = 0;
-      if (active) {
-        if (kFull) { bm = blk / nb; bj = blk - bm * nb; }
-        else {  // blk -> (bm <= bj), row-major over the upper triangle of blocks
-          int b = blk; bm = 0;
-          while (b >= nb - bm) { b -= nb - bm; ++bm; }
-          bj = bm + b;
+      if (active) {  // the diagonal blocks, then the rest row by row
+        if (blk < nb) { bm = bj = blk; }
+        else {
+          int q = blk - nb;
+          while (q >= nb - 1 - bm) { q -= nb - 1 - bm; ++bm; }
+          bj = bm + 1 + q;
         }
       }
-      C acc[4][4];
+      GramAcc<A> acc[4][4];
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) { acc[a][b].x = 0; acc[a][b].y = 0; }
-      const int sdt = (int)blockDim.x / npad, sdc = (int)blockDim.x - sdt * npad;
-      for (int s0 = 0; s0 < S; s0 += kChunk) {
-        const int ns = min(kChunk, S - s0);
-        __syncthreads();
-        // (row t, column c) of element e followed incrementally: no division per element
-        // (3 % faster)
-        for (int e = threadIdx.x, t = threadIdx.x / npad, c = threadIdx.x - (threadIdx.x / npad) * npad;
-             e < ns * npad; e += blockDim.x) {
-          float2 z = make_float2(0.f, 0.f);
-          if (c < n) z = rslc[(int64_t)s_pos[s0 + t] * n + c];
-          zc[t * npad + c] = z;
-          t += sdt;
-          c += sdc;
-          if (c >= npad) { c -= npad; ++t; }
+        for (int b = 0; b < 4; ++b) acc[a][b] = {};
+      if (S > 0) fetch(0, 0);
+      int buf = 0;
+      for (int s0 = 0; s0 < S; s0 += kc) {
+        const int ns = min(kc, S - s0);
+        const C* row = zc;
+        if constexpr (kWide) {
+          asm volatile("cp.async.wait_group 0;" ::: "memory");
+          each(ns, [&](int t, int c) {  // what this thread fetched
+            const float2 z = raw[t * n + c];
+            zc[place(t, c)] = cmake<C>((A)z.x, (A)z.y);
+          });
+          if (s0 + kc < S) fetch(s0 + kc, 0);
+        } else {
+          if (s0 + kc < S) {
+            fetch(s0 + kc, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+          } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+          }
+          row += buf * kc * npad;
+          buf ^= 1;
         }
         __syncthreads();
         if (active) {
-          for (int t = 0; t < ns; ++t) {
-            const float4* row = reinterpret_cast<const float4*>(zc + t * npad);
-            float4 ma = row[2 * bm], mb = row[2 * bm + 1];
-            float4 ja = row[2 * bj], jb = row[2 * bj + 1];
-            const A zm[4][2] = {{ma.x, ma.y}, {ma.z, ma.w}, {mb.x, mb.y}, {mb.z, mb.w}};
-            const A zj[4][2] = {{ja.x, ja.y}, {ja.z, ja.w}, {jb.x, jb.y}, {jb.z, jb.w}};
+#pragma unroll 2
+          for (int t = 0; t < ns; ++t, row += npad) {
+            C zm[4], zj[4];
+            load_block(row, nb, bm, zm);
+            load_block(row, nb, bj, zj);
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
-              for (int b = 0; b < 4; ++b) {
-                // z_m * conj(z_j). FP64: one FMA per product (the FP64 pipe bounds this loop,
-                // and the summed form costs a multiply and an add more per component, 13 %
-                // slower). FP32: the summed form, which rounds into the accumulator once per
-                // SHP instead of twice (with the FMA chain the error reached 2.5e-6 at 465
-                // SHPs, above the FP32 Gram's 2e-6 bound).
-                if constexpr (sizeof(A) == 8) {
-                  acc[a][b].x += zm[a][0] * zj[b][0];
-                  acc[a][b].x += zm[a][1] * zj[b][1];
-                  acc[a][b].y += zm[a][1] * zj[b][0];
-                  acc[a][b].y -= zm[a][0] * zj[b][1];
-                } else {
-                  acc[a][b].x += zm[a][0] * zj[b][0] + zm[a][1] * zj[b][1];
-                  acc[a][b].y += zm[a][1] * zj[b][0] - zm[a][0] * zj[b][1];
-                }
-              }
+              for (int b = 0; b < 4; ++b) acc[a][b].add(zm[a], zj[b]);
           }
         }
+        __syncthreads();  // the rows are overwritten by the next pass
+      }
+      if (round == 0) {  // FP64: 1 / sqrt of each sum, which saves two divisions per pair
+        if (blk < nb) {
+#pragma unroll
+          for (int a = 0; a < 4; ++a) amp2[4 * blk + a] = kWide ? (A)1 / sqrt(acc[a][a].re()) : acc[a][a].re();
+        }
+        __syncthreads();
       }
       if (active) {
 #pragma unroll
@@ -181,21 +255,261 @@ __global__ void __launch_bounds__(kGramThreads) gram_kernel(
 #pragma unroll
           for (int b = 0; b < 4; ++b) {
             const int mm = 4 * bm + a, jj = 4 * bj + b;
-            if (mm >= n || jj >= n) continue;
-            A den = sqrt(amp2[mm] * amp2[jj]);
+            if (mm >= n || jj >= n || mm > jj) continue;
+            const A re = acc[a][b].re(), im = acc[a][b].im();
+            float2 g;
+            if constexpr (kWide) {
+              const A r = amp2[mm] * amp2[jj];
+              g = make_float2((float)(re * r), (float)(im * r));
+            } else {
+              const A den = sqrt(amp2[mm] * amp2[jj]);
+              g = make_float2(re / den, im / den);
+            }
             if (kFull) {
-              const int64_t o = (i * n + mm) * n + jj;
-              coh[o] = make_float2((float)(acc[a][b].x / den), (float)(acc[a][b].y / den));
-              cov[o] = make_float2((float)(acc[a][b].x / (A)S), (float)(acc[a][b].y / (A)S));
+              const float2 v = make_float2((float)(re / (A)S), (float)(im / (A)S));
+              const int64_t o = (i * n + mm) * n + jj, ot = (i * n + jj) * n + mm;
+              coh[o] = g;
+              cov[o] = v;
+              if (mm != jj) {
+                coh[ot] = make_float2(g.x, -g.y);
+                cov[ot] = make_float2(v.x, -v.y);
+              }
             } else if (mm < jj) {
-              const int64_t o = i * npairs + triu_index(mm, jj, n);
-              coh[o] = make_float2((float)(acc[a][b].x / den), (float)(acc[a][b].y / den));
+              coh[i * npairs + triu_index(mm, jj, n)] = g;
             }
           }
       }
     }
-    __syncthreads();
+    __syncthreads();  // s_pos and amp2 are rewritten for the next point
   }
+}
+
+// FP64 up to kDmmaImages images on the FP64 tensor instruction (DMMA m16n8k8). It has the rate of
+// the FP64 pipe, 64 FMA per clock and SM, but reads each operand from shared memory once per
+// 16 x 8 block instead of once per 4 x 4. With k = 2 s + {re, im} as the contraction index,
+// A[m][k] = z_m's component k:
+//   Re = sum_k A[m][k] A[j][k],   Im = sum_k A[m][k] A'[j][k],  A' = (-im, re),
+// two products of real matrices with 2 S rows and no redundant sum. Every fragment is plain
+// 8-byte reads of the staged rows (image lane / 4, k = lane % 4).
+//
+// The upper triangle is cut into 16 x 8 blocks, and the blocks into runs of at most SLOTS that
+// span one or two block rows (plan_gram64); a run is one warp's accumulators, its A fragments are
+// read once or twice per step and its other addresses are a base and a constant (nothing issues
+// beside a DMMA, so every instruction counts: with a next-block rule per slot it took 5.9 ms
+// below, on m8n8k4 7.9 ms). Four warps of 13 blocks hold 104 images in one pass over the SHPs,
+// two such CTAs per SM; smaller runs leave room for more CTAs. Above that the accumulators
+// need several passes, which measured slower than gram_kernel<double> (6.4 against 5.2 ms at
+// N = 150).
+// N = 100, 11 x 21 window, 20,000 points: 4.6 ms against 6.4 (one CTA of 256 threads, samples
+// widened at each use); gram_kernel<double> 5.1. N = 50, 35,627 points: 2.3 against 4.6 ms; N = 17, 2,047 points: 42 against 126 us.
+constexpr int kGramWarps = 4;
+constexpr int kMaxRuns = 8;
+constexpr int kDmmaImages = 104;
+
+// Run r: blocks (br1, bc1 ...) c1 of them, then (br2, bc2 ...) up to cnt.
+struct GramRun {
+  uint8_t br1, bc1, c1, br2, bc2, cnt;
+};
+struct GramPlan {
+  int warps, runs, slots;  // slots: the longest run
+  GramRun run[kMaxRuns];
+};
+
+__device__ __forceinline__ void dmma(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+template <int SLOTS>
+__global__ void __launch_bounds__(32 * kGramWarps, SLOTS <= 4 ? 4 : SLOTS <= 7 ? 3 : 2) gram64_kernel(
+    const float2* __restrict__ rslc, int nlines, int width, int n, const int32_t* __restrict__ idx,
+    int64_t n_pc, const uint8_t* __restrict__ mask, int mask_stride, int az_win, int r_win,
+    float2* __restrict__ coh, const int64_t* __restrict__ dcount, int64_t doff, int kc,
+    const __grid_constant__ GramPlan plan) {
+  if (dcount) {
+    const int64_t c = *dcount - doff;
+    n_pc = c < 0 ? 0 : (c < n_pc ? c : n_pc);
+  }
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int win = az_win * r_win;
+  const int nr = (n + 15) >> 4;
+  const int npd = 16 * nr + 4;  // images of a staged row: = 4 mod 8, so that the two rows that a
+                                // fragment read spans lie on different banks
+  double2* zc = reinterpret_cast<double2*>(smem_raw);             // kc (a multiple of 4) x npd
+  double* rinv = reinterpret_cast<double*>(zc + kc * npd);         // 16 nr: 1 / sqrt(sum |z|^2)
+  float2* raw = reinterpret_cast<float2*>(rinv + 16 * nr);         // kc x n, as fetched
+  int* s_pos = reinterpret_cast<int*>(raw + kc * n);               // win
+  __shared__ int s_tmp[32];
+  const int64_t npairs = (int64_t)n * (n - 1) / 2;
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5;
+  for (int e = tid; e < kc * npd; e += nt) zc[e] = make_double2(0.0, 0.0);  // padding images stay 0
+  // thread's staging walk over (row t, image c): nt elements ahead is (sdt, sdc)
+  const int t_first = tid / n, c_first = tid - t_first * n;
+  const int sdt = nt / n, sdc = nt - sdt * n;
+  const int comp = lane & 1;
+  const double* zk = reinterpret_cast<const double*>(zc + ((lane >> 1) & 1) * npd + (lane >> 2));
+  const int k4 = 4 * npd;  // doubles from k to k + 4: two staged rows
+  const int row = lane >> 2, colp = 2 * (lane & 3);  // of accumulators 0 and 1; 2 and 3 are 8 rows on
+  __syncthreads();
+
+  for (int64_t i = blockIdx.x; i < n_pc; i += gridDim.x) {
+    const int ra = idx[2 * i], rr = idx[2 * i + 1];
+    if (ra < 0 || ra >= nlines || rr < 0 || rr >= width) {  // index outside the image: NaN row
+      const float2 nan2 = make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
+      for (int64_t e = tid; e < npairs; e += nt) coh[i * npairs + e] = nan2;
+      continue;
+    }
+    const uint8_t* m = mask + (mask_stride ? ((int64_t)ra * width + rr) : i) * win;
+    const int S = collect_shps(m, az_win, r_win, ra, rr, nlines, width, s_pos, s_tmp);
+    // rows s0 .. of the point's samples on their way to `raw`; a thread widens what it fetched
+    auto fetch = [&](int s0) {
+      const int ns = min(kc, S - s0);
+      int t = t_first, c = c_first;
+      while (t < ns) {
+        copy8(raw + t * n + c, rslc + (int64_t)s_pos[s0 + t] * n + c);
+        t += sdt;
+        c += sdc;
+        if (c >= n) { c -= n; ++t; }
+      }
+    };
+    int w = wid;
+    asm volatile("" : "+r"(w));  // the run is read for each point: kept over the loop it costs spills
+    const GramRun run = plan.run[w];
+    const int cnt = run.cnt, c1 = run.c1;
+    const int a1 = 32 * run.br1 + comp, a2 = 32 * run.br2 + comp;
+    const int b1 = 16 * run.bc1, b2 = 16 * ((int)run.bc2 - c1);
+    double re[SLOTS][4], im[SLOTS][4];
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q)
+#pragma unroll
+      for (int h = 0; h < 4; ++h) re[q][h] = im[q][h] = 0.0;
+    fetch(0);
+    for (int s0 = 0; s0 < S; s0 += kc) {
+      const int ns = min(kc, S - s0);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();  // the previous rows have been used
+      {
+        int t = t_first, c = c_first;
+        while (t < ns) {
+          const float2 z = raw[t * n + c];
+          zc[t * npd + c] = make_double2((double)z.x, (double)z.y);
+          t += sdt;
+          c += sdc;
+          if (c >= n) { c -= n; ++t; }
+        }
+      }
+      for (int r = ns; r & 3; ++r)  // a fragment takes four rows
+        for (int c2 = tid; c2 < n; c2 += nt) zc[r * npd + c2] = make_double2(0.0, 0.0);
+      fetch(s0 + kc);
+      __syncthreads();
+      const double* z = zk;
+      for (int t = 0; t < ns; t += 4, z += 2 * k4) {
+        double a[4];
+        auto load_a = [&](const double* p) {  // rows lane / 4 + 8 (h % 2), k = lane % 4 + 4 (h / 2)
+          a[0] = p[0];
+          a[1] = p[16];
+          a[2] = p[k4];
+          a[3] = p[k4 + 16];
+        };
+        load_a(z + a1);
+        const double* p = z + b1 + comp;
+        const double* o = z + b1 + (comp ^ 1);
+#pragma unroll
+        for (int q = 0; q < SLOTS; ++q) {
+          if (q < cnt) {
+            if (q == c1) {
+              load_a(z + a2);
+              p = z + b2 + comp;
+              o = z + b2 + (comp ^ 1);
+            }
+            const double b[2] = {p[16 * q], p[16 * q + k4]};
+            const double o0 = o[16 * q], o1 = o[16 * q + k4];
+            const double bx[2] = {comp ? o0 : -o0, comp ? o1 : -o1};
+            dmma(re[q], a, b);
+            dmma(im[q], a, bx);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q) {
+      if (q < cnt) {
+        const int br = q < c1 ? run.br1 : run.br2, bc = q < c1 ? run.bc1 + q : run.bc2 + q - c1;
+        const int h8 = bc - 2 * br;  // 0 or 1: the diagonal runs through this half of the rows
+        if (h8 < 2 && (row >> 1) == (lane & 3)) {
+          const double d0 = (row & 1) ? re[q][1] : re[q][0], d1 = (row & 1) ? re[q][3] : re[q][2];
+          rinv[8 * bc + row] = 1.0 / sqrt(h8 ? d1 : d0);
+        }
+      }
+    }
+    __syncthreads();
+    float2* out = coh + i * npairs;
+#pragma unroll
+    for (int q = 0; q < SLOTS; ++q) {
+      if (q < cnt) {
+        const int br = q < c1 ? run.br1 : run.br2, bc = q < c1 ? run.bc1 + q : run.bc2 + q - c1;
+        const int jj = 8 * bc + colp;
+        const double rj0 = rinv[jj], rj1 = rinv[jj + 1];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int mm = 16 * br + row + 8 * h;
+          const double rm = rinv[mm];
+          float2* o = out + (mm * n - ((mm * (mm + 1)) >> 1) - mm - 1 + jj);  // triu_index(mm, jj, n)
+          const double f0 = rm * rj0, f1 = rm * rj1;
+          if (mm < jj && jj < n) o[0] = make_float2((float)(re[q][2 * h] * f0), (float)(im[q][2 * h] * f0));
+          if (mm < jj + 1 && jj + 1 < n)
+            o[1] = make_float2((float)(re[q][2 * h + 1] * f1), (float)(im[q][2 * h + 1] * f1));
+        }
+      }
+    }
+    __syncthreads();  // s_pos and rinv are rewritten for the next point
+  }
+}
+
+// Runs of at most `cap` blocks for n images: each block row br has the blocks bc = 2 br .. nc - 1,
+// cut into pieces of cap; what is left of each row is paired with another rest, longest with the
+// longest that still fits.
+GramPlan cut_gram64(int n, int cap) {
+  struct Piece { int br, bc, len; };
+  const int nc = (n + 7) / 8, nr = (n + 15) / 16;
+  GramPlan plan{};
+  std::vector<Piece> rest;
+  auto add = [&](Piece a, Piece b) {
+    if (plan.runs < kMaxRuns)
+      plan.run[plan.runs] = {(uint8_t)a.br, (uint8_t)a.bc, (uint8_t)a.len, (uint8_t)b.br, (uint8_t)b.bc,
+                             (uint8_t)(a.len + b.len)};
+    ++plan.runs;
+    plan.slots = std::max(plan.slots, a.len + b.len);
+  };
+  for (int br = 0; br < nr; ++br) {
+    int bc = 2 * br;
+    for (; nc - bc >= cap; bc += cap) add({br, bc, cap}, {0, 0, 0});
+    if (bc < nc) rest.push_back({br, bc, nc - bc});
+  }
+  std::sort(rest.begin(), rest.end(), [](const Piece& a, const Piece& b) { return a.len > b.len; });
+  while (!rest.empty()) {
+    const Piece a = rest.front();
+    rest.erase(rest.begin());
+    auto b = std::find_if(rest.begin(), rest.end(), [&](const Piece& p) { return a.len + p.len <= cap; });
+    if (b == rest.end()) { add(a, {0, 0, 0}); continue; }
+    add(a, *b);
+    rest.erase(b);
+  }
+  plan.warps = plan.runs;
+  return plan;
+}
+
+// The cut into at most kGramWarps runs with the least warp time (warps times the longest run), short
+// runs where two are equal. n <= kDmmaImages always has one (runs of 13).
+GramPlan plan_gram64(int n) {
+  GramPlan best{};
+  for (int cap = 4; cap <= 13; ++cap) {
+    const GramPlan p = cut_gram64(n, cap);
+    if (p.runs <= kGramWarps && (!best.runs || p.warps * p.slots < best.warps * best.slots)) best = p;
+  }
+  return best;
 }
 
 // Arbitrary pair lists: one thread per (point, pair), serial over the window.
@@ -235,19 +549,55 @@ __global__ void gram_pairs_kernel(const float2* __restrict__ rslc, int nlines, i
   }
 }
 
+// Points of a launch: enough CTAs to fill the device several times over (their SHP counts, and
+// so their times, differ), each walking its share.
+template <class K>
+unsigned gram_grid(K kernel, int threads, size_t smem, int64_t n_pc) {
+  int occ = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess || occ < 1) occ = 1;
+  return (unsigned)std::min<int64_t>(n_pc, (int64_t)sm_count() * occ * 8);
+}
+
 template <typename A, bool kFull>
 int launch_gram(const float2* rslc, int nlines, int width, int n, const int32_t* idx, int64_t n_pc,
                 const uint8_t* mask, int mask_stride, int az_win, int r_win, float2* coh, float2* cov,
                 cudaStream_t s, const int64_t* dcount = nullptr, int64_t doff = 0) {
-  const int npad = (n + 3) & ~3;
-  const size_t smem = (size_t)kChunk * npad * sizeof(float2) + npad * sizeof(A) +
+  using C = typename cplx<A>::type;
+  constexpr bool kWide = sizeof(A) == 8;
+  const int nb = (n + 3) / 4, nblk = nb * (nb + 1) / 2;
+  // no more warps than the blocks fill; all but the last round run full
+  const int threads = std::min(kMaxGramThreads, (nblk + 31) / 32 * 32);
+  const size_t row = (size_t)(kWide ? 1 : 2) * 4 * nb * sizeof(C);
+  const int kc = chunk_rows(kWide ? 16 : 32, row);
+  const size_t smem = kc * row + (kWide ? ((size_t)kc * n + 1) / 2 * 2 * sizeof(float2) : 0) + 4 * nb * sizeof(A) +
                       (size_t)az_win * r_win * sizeof(int);
   if (int rc = allow_smem(reinterpret_cast<const void*>(gram_kernel<A, kFull>), smem)) return rc;
-  const int64_t grid = std::min<int64_t>(n_pc, (int64_t)sm_count() * 8);
-  KernelTimer kt(sizeof(A) == 8 ? "gram fp64" : "gram fp32", s);
-  gram_kernel<A, kFull><<<(unsigned)grid, kGramThreads, smem, s>>>(rslc, nlines, width, n, idx, n_pc, mask,
-                                                                   mask_stride, az_win, r_win, coh, cov, dcount, doff);
+  KernelTimer kt(kWide ? "gram fp64" : "gram fp32", s);
+  gram_kernel<A, kFull><<<gram_grid(gram_kernel<A, kFull>, threads, smem, n_pc), threads, smem, s>>>(
+      rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win, r_win, coh, cov, dcount, doff, kc);
   return check_launch("coherence gram");
+}
+
+int launch_gram64(const float2* rslc, int nlines, int width, int n, const int32_t* idx, int64_t n_pc,
+                  const uint8_t* mask, int mask_stride, int az_win, int r_win, float2* coh, cudaStream_t s,
+                  const int64_t* dcount = nullptr, int64_t doff = 0) {
+  if (n > kDmmaImages)
+    return launch_gram<double, false>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win, r_win, coh,
+                                      nullptr, s, dcount, doff);
+  const int nr = (n + 15) / 16;
+  const GramPlan plan = plan_gram64(n);
+  const int threads = 32 * plan.warps;
+  const int kc = plan.warps == 1 ? 8 : 16;  // one-warp CTAs stage fewer rows, so that more of them fit an SM
+  const size_t smem = (size_t)kc * ((16 * nr + 4) * sizeof(double2) + n * sizeof(float2)) + 16 * nr * sizeof(double) +
+                      (size_t)az_win * r_win * sizeof(int);
+  auto go = [&](auto kernel) {
+    if (int rc = allow_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
+    KernelTimer kt("gram fp64", s);
+    kernel<<<gram_grid(kernel, threads, smem, n_pc), threads, smem, s>>>(
+        rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win, r_win, coh, dcount, doff, kc, plan);
+    return check_launch("coherence gram");
+  };
+  return plan.slots <= 4 ? go(gram64_kernel<4>) : plan.slots <= 7 ? go(gram64_kernel<7>) : go(gram64_kernel<13>);
 }
 
 }  // namespace
@@ -291,8 +641,7 @@ extern "C" int mr_emperical_co_pc(const mr_complex64* rslc, int nlines, int widt
       return launch_gram<float, false>(z, nlines, width, nimages, idx, n_pc, mask, mask_stride, az_win, r_win,
                                        out, nullptr, s);
     case MR_PREC_FP64:
-      return launch_gram<double, false>(z, nlines, width, nimages, idx, n_pc, mask, mask_stride, az_win, r_win,
-                                        out, nullptr, s);
+      return launch_gram64(z, nlines, width, nimages, idx, n_pc, mask, mask_stride, az_win, r_win, out, s);
     case MR_PREC_BF16:
     case MR_PREC_BF16X3:
       return gram_tc(z, nlines, width, nimages, idx, n_pc, mask, mask_stride, az_win, r_win, out, precision, s);
@@ -348,8 +697,7 @@ int gram_counted(const float2* rslc, int nlines, int width, int n, const int32_t
     return launch_gram<float, false>(rslc, nlines, width, n, idx, n_max, mask, 1, az_win, r_win, coh, nullptr, s,
                                      dcount, doff);
   if (precision == MR_PREC_FP64)
-    return launch_gram<double, false>(rslc, nlines, width, n, idx, n_max, mask, 1, az_win, r_win, coh, nullptr, s,
-                                      dcount, doff);
+    return launch_gram64(rslc, nlines, width, n, idx, n_max, mask, 1, az_win, r_win, coh, s, dcount, doff);
   return fail(MR_ERR_UNSUPPORTED, "device-counted coherence runs in FP32 or FP64");
 }
 }  // namespace mr

@@ -92,3 +92,32 @@ def test_ks_selection_without_p(cuda, n, azh, rh):
         np.testing.assert_array_equal(got_num, num)
         assert got.max() <= 1
     np.testing.assert_array_equal(mb.ks_test(x, azh, rh), p)
+
+
+# ----------------------------------------------------------------------------- coherence
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 8, 9, 17, 31, 40, 57, 76, 77, 104, 105, 137, 200, 301, 409])
+def test_coherence_block_shapes(cuda, n):
+    """FP32 and FP64 Gram at the edges of their blocks, warps and rounds, SHP counts from one
+    to over two staged passes, points at the border and outside the image."""
+    rng = np.random.default_rng(n)
+    nl, w, azw, rw = 13, 17, 9, 11
+    z = (rng.normal(size=(nl, w, n)) + 1j * rng.normal(size=(nl, w, n))).astype(np.complex64)
+    idx = np.array([[6, 8], [0, 0], [12, 16], [5, 3], [7, 9], [6, 7], [2, 15]], np.int32)
+    mask = rng.random((len(idx), azw, rw)) < np.array([1, .7, .6, .35, .17, .02, .5])[:, None, None]
+    mask[:, azw // 2, rw // 2] = True
+    ref = O.emperical_co_pc(z, idx, mask)
+    for precision, tol in (("fp32", 2e-6), ("fp64", 1e-7)):
+        got = mb.emperical_co_pc(z, idx, mask, precision=precision)
+        np.testing.assert_allclose(got, ref, atol=tol, rtol=0)
+        out = mb.emperical_co_pc(z, np.array([[6, 8], [-1, 3], [6, 17]], np.int32), mask[:3], precision=precision)
+        np.testing.assert_array_equal(out[0], got[0])
+        assert np.isnan(out[1:].view(np.float32)).all()
+    if n <= 40:
+        is_shp = rng.random((nl, w, azw, rw)) < 0.4
+        is_shp[..., azw // 2, rw // 2] = True
+        cov_ref, coh_ref = O.emperical_co(z, is_shp)
+        cov, coh = mb.emperical_co(z, is_shp)
+        np.testing.assert_allclose(coh, coh_ref, atol=2e-6, rtol=0)
+        np.testing.assert_allclose(cov, cov_ref, atol=2e-6 * np.abs(cov_ref).max(), rtol=0)
+        np.testing.assert_array_equal(coh, np.conj(np.swapaxes(coh, -1, -2)))
