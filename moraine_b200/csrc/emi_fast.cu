@@ -214,68 +214,8 @@ __device__ bool gj_tile(T (&a)[NB][GjGrid<NB, CX>::NC], unsigned used, int n, in
 }
 
 // ----------------------------------------------------------------- packed reduction
-template <typename T>
-struct TriShared {
-  using C = typename C2<T>::type;
-  C* L;       // lower triangle by rows: (i, j <= i) at roff[i] + j
-  C* pv;      // [2][n] products of the last two steps
-  C* vec;     // [3][n]: u_k and u_{k-1} (by step parity), w_{k-1}
-  C* e;
-  T* d;
-  T* tau;
-  int* roff;  // row starts, n + 1 entries
-};
-
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 __host__ __device__ __forceinline__ int tri(int i) { return i * (i + 1) / 2; }
-
-// Row i of the FP32 triangle starts at roff_of(i) elements: row strides are the smallest
-// values >= i + 1 that are 4 mod 16, so that the row segments of mirrored pairs (phase 1) and
-// the column walks (phase 2) of a warp fall on distinct 8-byte bank pairs (the reduction
-// measured 5 % faster than with packed rows). The FP64 triangle stays packed (tri): there the
-// padding measured 3 % slower.
-__host__ __device__ __forceinline__ int roff_of(int i) {
-  const int a = (i + 12) >> 4, b = (i + 12) & 15;
-  return 4 * i + 128 * a * (a - 1) + 16 * a * b;
-}
-template <typename T> __host__ __device__ __forceinline__ int tri_elems(int n) {
-  return sizeof(T) == 4 ? roff_of(n) : n * (n + 1) / 2;
-}
-template <typename T> __device__ __forceinline__ int rstart(const TriShared<T>& s, int i) {
-  if constexpr (sizeof(T) == 4) return s.roff[i];
-  else return tri(i);
-}
-
-template <typename T>
-__host__ __device__ inline size_t tri_bytes(int n) {
-  using C = typename C2<T>::type;
-  size_t o = align16((size_t)tri_elems<T>(n) * sizeof(C));
-  o = align16(o + 2 * (size_t)n * sizeof(C));
-  o = align16(o + 3 * (size_t)n * sizeof(C));
-  o = align16(o + (size_t)n * sizeof(C));
-  o = align16(o + 2 * (size_t)n * sizeof(T));
-  return o + (size_t)(n + 1) * sizeof(int);
-}
-
-template <typename T>
-__device__ inline TriShared<T> tri_layout(unsigned char* base, int n) {
-  using C = typename C2<T>::type;
-  TriShared<T> s;
-  size_t o = 0;
-  s.L = reinterpret_cast<C*>(base + o);
-  o = align16(o + (size_t)tri_elems<T>(n) * sizeof(C));
-  s.pv = reinterpret_cast<C*>(base + o);
-  o = align16(o + 2 * (size_t)n * sizeof(C));
-  s.vec = reinterpret_cast<C*>(base + o);
-  o = align16(o + 3 * (size_t)n * sizeof(C));
-  s.e = reinterpret_cast<C*>(base + o);
-  o = align16(o + (size_t)n * sizeof(C));
-  s.d = reinterpret_cast<T*>(base + o);
-  s.tau = s.d + n;
-  o = align16(o + 2 * (size_t)n * sizeof(T));
-  s.roff = reinterpret_cast<int*>(base + o);
-  return s;
-}
 
 // a -= ui conj(wj) + wi conj(uj)
 template <typename C> __device__ __forceinline__ void rank2(C& a, C ui, C wj, C wi, C uj) {
@@ -283,173 +223,6 @@ template <typename C> __device__ __forceinline__ void rank2(C& a, C ui, C wj, C 
   a.x -= ui.x * wj.x; a.x -= ui.y * wj.y; a.x -= wi.x * uj.x; a.x -= wi.y * uj.y;
   a.y -= ui.y * wj.x; a.y += ui.x * wj.y; a.y -= wi.y * uj.x; a.y += wi.x * uj.y;
 }
-
-// Householder reduction of the Hermitian M (lower triangle, packed in s.L) to tridiagonal
-// (s.d, s.e); reflector k stored in column k (rows k+1..n-1) with scalar s.tau[k]. Whole
-// CTA, three barriers per step:
-//   1. warp 0 finishes step k-1 (w = p - K u, K = tau/2 u^H p) and forms reflector k from
-//      column k brought up to date, x_i = A_i + K B_i, with A_i and B_i computed in the same
-//      pass as the dot product (one load pass, two warp reductions);
-//   2. phase 1: step k-1's rank-2 update on the lower triangle of rows >= k+1 and the row
-//      part of (M u_k)_i = sum_{j<=i} M_ij u_j;
-//   3. phase 2: the column part sum_{j>i} conj(M_ji) u_j, then p_k = tau_k M u_k.
-// Rows are handled in mirrored pairs (i, n+k-i) by groups of 4 threads, which gives every
-// thread of a step the same number of elements in both phases. The packed triangle halves the
-// shared memory of full storage, so twice as many points are in flight per SM.
-template <typename T>
-__device__ void tridiag_packed(const TriShared<T>& s, int n) {
-  using C = typename C2<T>::type;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  C* L = s.L;
-  C* wp = s.vec + 2 * n;  // w_{k-1}
-  for (int k = 0; k + 2 < n; ++k) {
-    C* up = s.vec + ((k + 1) & 1) * n;  // u_{k-1}
-    C* uc = s.vec + (k & 1) * n;        // u_k
-    // ---- warp 0: finish step k-1 and form reflector k
-    if (wid == 0) {
-      const T tau_prev = k > 0 ? s.tau[k - 1] : T(0);
-      const bool pending = tau_prev != T(0);
-      const C* p = s.pv + ((k + 1) & 1) * n;
-      C A[4], B[4], pp[4], uu[4];
-      T dot = 0;
-      C pk = mk<T>(0, 0), ukk = mk<T>(0, 0);
-      if (pending) { pk = p[k]; ukk = up[k]; }
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int i = k + lane + 32 * t;
-        A[t] = B[t] = pp[t] = uu[t] = mk<T>(0, 0);
-        if (i < n) {
-          const int base = rstart(s, i);
-          A[t] = L[base + k];
-          if (pending) {
-            pp[t] = p[i];
-            uu[t] = up[i];
-            dot += uu[t].x * pp[t].x + uu[t].y * pp[t].y;
-            // x_i = a_ik - u_i conj(w_k) - w_i conj(u_k) = A_i + K B_i, w = p - K u
-            rank2(A[t], uu[t], pk, pp[t], ukk);
-            B[t] = mk<T>(2 * (uu[t].x * ukk.x + uu[t].y * ukk.y), 2 * (uu[t].y * ukk.x - uu[t].x * ukk.y));
-            L[base + k - 1] = uu[t];  // reflector k-1 (rows >= k) kept in column k-1
-          }
-        }
-      }
-      const T K = pending ? T(0.5) * tau_prev * warp_sum(dot) : T(0);
-      T xn2 = 0;
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int i = k + lane + 32 * t;
-        if (i < n) {
-          const C x = mk<T>(A[t].x + K * B[t].x, A[t].y + K * B[t].y);
-          if (pending) wp[i] = mk<T>(pp[t].x - K * uu[t].x, pp[t].y - K * uu[t].y);
-          uc[i] = x;
-          if (i >= k + 2) xn2 += x.x * x.x + x.y * x.y;
-        }
-      }
-      xn2 = warp_sum(xn2);
-      __syncwarp();
-      const C alpha = uc[k + 1];
-      T tau_k = 0;
-      C ek = alpha;
-      if (xn2 != T(0)) {
-        const T aa = sqrt(alpha.x * alpha.x + alpha.y * alpha.y);
-        const T nrm = sqrt(aa * aa + xn2);
-        const C ph1 = aa > T(0) ? mk<T>(alpha.x / aa, alpha.y / aa) : mk<T>(1, 0);
-        tau_k = T(2) / ((aa + nrm) * (aa + nrm) + xn2);
-        ek = mk<T>(-ph1.x * nrm, -ph1.y * nrm);
-        if (lane == 0) uc[k + 1] = mk<T>(ph1.x * (aa + nrm), ph1.y * (aa + nrm));
-      }
-      if (lane == 0) { s.d[k] = uc[k].x; s.e[k] = ek; s.tau[k] = tau_k; }
-    }
-    __syncthreads();
-    const bool pending = k > 0 && s.tau[k - 1] != T(0);
-    const T tau_k = s.tau[k];
-    const int m = n - k - 1;         // rows k+1..n-1
-    const int npair = (m + 1) >> 1;  // mirrored pairs (the middle row of an odd m alone)
-    // G = 4 threads per pair. Widening the groups to keep every thread busy as the trailing
-    // matrix shrinks measured 3 % slower: the short rows of late steps then cost more loop
-    // set-up than they save, while idle warps leave the issue slots to the other CTAs.
-    const int G = 4;
-    const int pq = tid / G, sub = tid & (G - 1);
-    const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << G) - 1u) << (lane & ~(G - 1));
-    const bool active = (pending || tau_k != T(0)) && pq < npair;
-    const int i1 = k + 1 + pq, i2 = n - 1 - pq;
-    const bool two = i2 != i1;
-    // ---- phase 1: update the lower rows, row part of M u
-    C rs1 = mk<T>(0, 0), rs2 = mk<T>(0, 0);
-    if (active) {
-#pragma unroll 1
-      for (int r = 0; r < 2; ++r) {
-        if (r && !two) break;
-        const int i = r ? i2 : i1;
-        C* row = L + rstart(s, i);
-        C upi = mk<T>(0, 0), wpi = mk<T>(0, 0);
-        if (pending) { upi = up[i]; wpi = wp[i]; }
-        C acc = mk<T>(0, 0);
-#pragma unroll 2  // measured: 5 % faster than the compiler's default, 4 gave less
-        for (int j = k + 1 + sub; j <= i; j += G) {
-          C a = row[j];
-          if (pending) { rank2(a, upi, wp[j], wpi, up[j]); row[j] = a; }
-          const C u = uc[j];
-          acc.x += a.x * u.x; acc.x -= a.y * u.y;
-          acc.y += a.x * u.y; acc.y += a.y * u.x;
-        }
-        if (r) rs2 = acc; else rs1 = acc;
-      }
-    }
-    __syncthreads();
-    // ---- phase 2: column part, then p_k
-    if (active && tau_k != T(0)) {
-#pragma unroll 1
-      for (int r = 0; r < 2; ++r) {
-        if (r && !two) break;
-        const int i = r ? i2 : i1;
-        C acc = r ? rs2 : rs1;
-#pragma unroll 2
-        for (int j = i + 1 + sub; j < n; j += G) {
-          const C a = L[rstart(s, j) + i];  // M_ji, lower triangle
-          const C u = uc[j];
-          acc.x += a.x * u.x; acc.x += a.y * u.y;  // conj(M_ji) u_j
-          acc.y += a.x * u.y; acc.y -= a.y * u.x;
-        }
-        for (int o = 1; o < G; o <<= 1) {
-          acc.x += __shfl_xor_sync(gmask, acc.x, o);
-          acc.y += __shfl_xor_sync(gmask, acc.y, o);
-        }
-        if (sub == 0) s.pv[(k & 1) * n + i] = mk<T>(tau_k * acc.x, tau_k * acc.y);
-      }
-    }
-    __syncthreads();
-  }
-  // last pending update (step n-3) on the trailing 2 x 2 block; reflector n-3 stored
-  if (wid == 0) {
-    if (n >= 3 && s.tau[n - 3] != T(0)) {
-      const T tau_prev = s.tau[n - 3];
-      const C* up = s.vec + ((n - 3) & 1) * n;
-      const C* p = s.pv + ((n - 3) & 1) * n;
-      T dot = 0;
-      for (int i = n - 2 + lane; i < n; i += 32) {
-        const C pi = p[i], ui = up[i];
-        wp[i] = pi;
-        dot += ui.x * pi.x + ui.y * pi.y;
-      }
-      const T K = T(0.5) * tau_prev * warp_sum(dot);
-      for (int i = n - 2 + lane; i < n; i += 32) { wp[i].x -= K * up[i].x; wp[i].y -= K * up[i].y; }
-      __syncwarp();
-      if (lane < 3) {
-        const int i = (lane == 0) ? n - 2 : n - 1, j = (lane == 2) ? n - 1 : n - 2;
-        rank2(L[rstart(s, i) + j], up[i], wp[j], wp[i], up[j]);
-      }
-      for (int i = n - 2 + lane; i < n; i += 32) L[rstart(s, i) + n - 3] = up[i];
-      __syncwarp();
-    }
-    if (lane == 0) {
-      s.d[n - 2] = L[rstart(s, n - 2) + n - 2].x;
-      s.d[n - 1] = L[rstart(s, n - 1) + n - 1].x;
-      s.e[n - 2] = L[rstart(s, n - 1) + n - 2];
-    }
-  }
-  __syncthreads();
-}
-
 
 // acc += a b (one FMA per product)
 template <typename C> __device__ __forceinline__ void cmac(C& acc, C a, C b) {
@@ -486,6 +259,28 @@ template <typename C> __device__ __forceinline__ C warp_sum4(const C (&r)[4]) {
   k = cadd(k, shfl_xor_c(k, 2));
   k = cadd(k, shfl_xor_c(k, 1));
   return k;
+}
+
+// Sums over the 16 lanes of each half-warp: lane l holds the total of value (l % 16) / 4 of four, or
+// (l % 16) / 8 of two.
+template <typename C> __device__ __forceinline__ C half_warp_sum(const C (&r)[2]) {
+  const bool hi3 = threadIdx.x & 8;
+  C k = hi3 ? r[1] : r[0];
+  k = cadd(k, shfl_xor_c(hi3 ? r[0] : r[1], 8));
+  k = cadd(k, shfl_xor_c(k, 4));
+  k = cadd(k, shfl_xor_c(k, 2));
+  return cadd(k, shfl_xor_c(k, 1));
+}
+template <typename C> __device__ __forceinline__ C half_warp_sum(const C (&r)[4]) {
+  const bool hi3 = threadIdx.x & 8, hi2 = threadIdx.x & 4;
+  C k0 = hi3 ? r[2] : r[0], k1 = hi3 ? r[3] : r[1];
+  const C s0 = hi3 ? r[0] : r[2], s1 = hi3 ? r[1] : r[3];
+  k0 = cadd(k0, shfl_xor_c(s0, 8));
+  k1 = cadd(k1, shfl_xor_c(s1, 8));
+  C k = hi2 ? k1 : k0;
+  k = cadd(k, shfl_xor_c(hi2 ? k0 : k1, 4));
+  k = cadd(k, shfl_xor_c(k, 2));
+  return cadd(k, shfl_xor_c(k, 1));
 }
 
 // ----------------------------------------------------------------- workspace layout
@@ -789,48 +584,233 @@ __global__ void __launch_bounds__(256, 2) sweep_kernel(const float2* __restrict_
 }
 
 // ----------------------------------------------------------------- kernel 2: reduction
-template <typename T, typename TA>
-__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 4 : 2) reduce_kernel(const float2* __restrict__ coh, PointSet pts, int n,
-                                                         unsigned char* __restrict__ ws) {
+// Householder reduction of M = inv(|Gamma|) o Gamma to a Hermitian tridiagonal (d, e), M in
+// shared memory as a packed lower triangle ((i, j <= i) at tri(i) + j). One CTA per point, two
+// barriers per step k:
+//   A. warp 0 (lane l owns rows l + 32 t): p = tau M u of step k-1 from its partial sums, K = tau/2
+//      u^H p, w = p - K u; column k brought up to date; reflector u_k, tau_k from it.
+//   B. every warp, over strips of R rows per half-warp (longest first): step k-1's rank-2 update of
+//      the rows > k and, on the updated values, both parts of M u_k: the rows' sums over the 16
+//      lanes, and the columns' sums of conj(M_ij) u_i, which stay in the lane that owns column j
+//      (lanes run along columns k + 1 + lane % 16 + 16 q) until the warp is through its strips.
+// Every element is read and written once per step and a row's vectors are read once per strip;
+// partial sums are added in a fixed order, so results do not depend on timing. Blocks of 16 columns
+// that meet the diagonal run unmasked over the next rows' entries, keep what is theirs and count half
+// of the diagonal in either part. Bound by latency: the chain of A (two warp sums, roots and
+// divisions) and the short strips of B, hidden only by the other CTAs of the SM. The previous form
+// (256 threads, three barriers, groups of four threads on mirrored row pairs, row and column parts in
+// separate passes over M): FP32, N = 17, 2,047 points 146 us, now 37; N = 50, 35,627 points 8.4 ms,
+// now 3.4; N = 100, 286,294 points 199 ms, now 178; FP64, N = 17, 1,003 points 157 us, now 38; N = 100,
+// 4,001 points 6.2 ms, now 5.8.
+// Shared memory: the triangle, 16 entries that reads past the end of its last row may touch, (u, w)
+// of step k-1 and u_k with kRowPad entries in front (rows above the first of a strip), and each
+// warp's part of M u.
+constexpr int kRowPad = 8, kColPad = 16;
+template <typename T>
+__host__ __device__ inline size_t reduce_smem(int n, int warps) {
+  return ((size_t)n * (n + 1) / 2 + kColPad + 3 * (size_t)(n + kRowPad + kColPad) + (size_t)warps * n) *
+         sizeof(typename C2<T>::type);
+}
+
+template <typename C> struct alignas(2 * sizeof(C)) Pair {
+  C u, w;
+};
+
+template <typename T, typename TA, int QC, int R, int W>
+__global__ void __launch_bounds__(32 * W, W >= 4 ? 16 / W : 1) reduce_kernel(const float2* __restrict__ coh, PointSet pts,
+                                                                          int n, unsigned char* __restrict__ ws) {
+  using C = typename C2<T>::type;
+  constexpr int Q = (QC + 1) / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const TriShared<T> s = tri_layout<T>(smem_raw, n);
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int i = tid; i <= n; i += nt) s.roff[i] = roff_of(i);
-  __syncthreads();
+  const int tid = threadIdx.x, lane = tid & 31, lc = lane & 15, wid = tid >> 5;
+  constexpr int nw = W;
+  Pair<C>* uw = reinterpret_cast<Pair<C>*>(smem_raw) + kRowPad;  // u_{k-1}, w_{k-1}
+  C* uc = reinterpret_cast<C*>(uw + n + kColPad) + kRowPad;      // u_k
+  C* part = uc + n + kColPad;                                    // [warps][n]: each warp's part of M u
+  C* L = part + nw * n;
   const int64_t npairs = (int64_t)n * (n - 1) / 2;
-  const int np = n * (n + 1) / 2;
   const int64_t npt = pts.size();
+  for (int e = tid; e < kRowPad; e += blockDim.x) {
+    uw[-1 - e] = {mk<T>(0, 0), mk<T>(0, 0)};
+    uc[-1 - e] = mk<T>(0, 0);
+  }
+  for (int e = tid; e < kColPad; e += blockDim.x) {
+    uw[n + e] = {mk<T>(0, 0), mk<T>(0, 0)};
+    uc[n + e] = mk<T>(0, 0);
+    L[tri(n) + e] = mk<T>(0, 0);
+  }
   for (int64_t pt = blockIdx.x; pt < npt; pt += gridDim.x) {
     const float2* c = coh + pts[pt] * npairs;
     PointPtr<T, TA> w(ws, pt, n);
-    // M = inv(|Gamma|) o Gamma: read along the upper triangle (inverse and coherence both
-    // contiguous), written to the packed lower triangle as M_jm = conj(M_mj)
-    // row m of element q: rows start at tri_up(m, m, n), which grows only up to m = n, so the
-    // walk stops at the last row
-    int m = 0;
-    while (m + 1 < n && tri_up(m + 1, m + 1, n) <= tid) ++m;
-    for (int q = tid; q < np; q += nt) {
-      while (m + 1 < n && tri_up(m + 1, m + 1, n) <= q) ++m;
-      const int j = m + (q - (int)tri_up(m, m, n));
-      const TA sc = w.ainv[q];
-      T gx = 1, gy = 0;
-      if (j != m) {
-        const float2 g = c[(int64_t)q - (m + 1)];  // pair (m, j): triu_index(m, j) = tri_up(m, j) - m - 1
-        gx = g.x;
-        gy = -g.y;
+    // M along the upper triangle (inverse and coherence both contiguous there), a warp per row;
+    // M_jm = conj(M_mj)
+    for (int m = wid; m < n; m += nw) {
+      const TA* ai = w.ainv + (tri_up(m, m, n) - m);
+      const float2* ci = c + (triu_index(m, m + 1, n) - (m + 1));
+      for (int j = m + lane; j < n; j += 32) {
+        const TA sc = ai[j];
+        const float2 g = j == m ? make_float2(1.f, 0.f) : ci[j];
+        L[tri(j) + m] = mk<T>((T)(sc * g.x), (T)(sc * -g.y));
       }
-      s.L[rstart(s, j) + m] = mk<T>((T)(sc * gx), (T)(sc * gy));
     }
+    C u[Q];  // warp 0: u_{k-1}, rows lane + 32 t
+#pragma unroll
+    for (int t = 0; t < Q; ++t) u[t] = mk<T>(0, 0);
+    T tau_prev = 0;
     __syncthreads();
-    tridiag_packed<T>(s, n);
-    for (int k = tid; k < n; k += nt) {
-      w.d[k] = s.d[k];
-      w.tau[k] = (k + 2 < n) ? s.tau[k] : T(0);
-      if (k + 1 < n) w.e[k] = s.e[k];
+    for (int k = 0; k + 1 < n; ++k) {
+      if (wid == 0) {
+        C wr[Q];
+        T dot = 0;
+#pragma unroll
+        for (int t = 0; t < Q; ++t) {
+          const int i = lane + 32 * t;
+          wr[t] = mk<T>(0, 0);
+          if (tau_prev != T(0) && i >= k && i < n) {
+            C p = part[i];
+            for (int q = 1; q < nw; ++q) p = cadd(p, part[q * n + i]);
+            wr[t] = mk<T>(tau_prev * p.x, tau_prev * p.y);
+            dot += u[t].x * wr[t].x + u[t].y * wr[t].y;
+          }
+        }
+        const T K = T(0.5) * tau_prev * warp_sum(dot);
+#pragma unroll
+        for (int t = 0; t < Q; ++t) {
+          const int i = lane + 32 * t;
+          wr[t].x -= K * u[t].x;
+          wr[t].y -= K * u[t].y;
+          if (i < n) uw[i] = {u[t], wr[t]};
+        }
+        __syncwarp();
+        const Pair<C> at_k = uw[k];
+        C x[Q];
+        T xn2 = 0;
+#pragma unroll
+        for (int t = 0; t < Q; ++t) {
+          const int i = lane + 32 * t;
+          x[t] = mk<T>(0, 0);
+          if (i >= k && i < n) {
+            x[t] = L[tri(i) + k];
+            rank2(x[t], u[t], at_k.w, wr[t], at_k.u);
+          }
+          if (i >= k + 2) xn2 += x[t].x * x[t].x + x[t].y * x[t].y;
+        }
+        xn2 = warp_sum(xn2);
+        C alpha = x[0];
+#pragma unroll
+        for (int t = 1; t < Q; ++t)
+          if ((k + 1) >> 5 == t) alpha = x[t];
+        alpha.x = __shfl_sync(0xffffffffu, alpha.x, (k + 1) & 31);
+        alpha.y = __shfl_sync(0xffffffffu, alpha.y, (k + 1) & 31);
+        T tau = 0;
+        C ek = alpha, v1 = alpha;
+        if (xn2 != T(0)) {
+          // e_k = -alpha nrm / |alpha|, v_1 = alpha (1 + nrm / |alpha|), tau = 1 / (nrm (nrm + |alpha|)): the
+          // two roots and the two divisions side by side
+          const T a2 = alpha.x * alpha.x + alpha.y * alpha.y;
+          const T aa = sqrt(a2), nrm = sqrt(a2 + xn2);
+          tau = T(1) / (nrm * (nrm + aa));
+          const T f = nrm / aa;
+          if (aa > T(0)) {
+            ek = mk<T>(-alpha.x * f, -alpha.y * f);
+            v1 = mk<T>(alpha.x - ek.x, alpha.y - ek.y);
+          } else {
+            ek = mk<T>(-nrm, 0);
+            v1 = mk<T>(nrm, 0);
+          }
+        }
+        C* refl = w.refl + refl_off(k, n) - (k + 1);
+#pragma unroll
+        for (int t = 0; t < Q; ++t) {
+          const int i = lane + 32 * t;
+          if (i == k) w.d[k] = x[t].x;
+          if (k + 2 == n && i == n - 1) {  // the last step: what is left of the diagonal
+            C a = L[tri(i) + i];
+            rank2(a, u[t], wr[t], wr[t], u[t]);
+            w.d[i] = a.x;
+            w.tau[i] = T(0);
+          }
+          u[t] = i == k + 1 ? v1 : x[t];
+          if (i <= k || tau == T(0)) u[t] = mk<T>(0, 0);
+          if (i < n) uc[i] = u[t];
+          if (i > k && i < n && k + 2 < n) refl[i] = u[t];
+        }
+        if (lane == 0) {
+          w.e[k] = ek;
+          w.tau[k] = tau;
+        }
+        tau_prev = tau;
+      }
+      if (k + 2 == n) break;
+      __syncthreads();
+      // ---- B
+      C* mine = part + wid * n;
+      C acc[QC];  // column sums, of columns k + 1 + lc + 16 q
+#pragma unroll
+      for (int q = 0; q < QC; ++q) acc[q] = mk<T>(0, 0);
+      const Pair<C>* cuw = uw + (k + 1 + lc);
+      const C* cuc = uc + (k + 1 + lc);
+      for (int top = n - 1 - 2 * R * wid; top > k; top -= 2 * R * nw) {
+        const int hi = top - R * (lane >> 4);  // this half-warp's strip: rows hi - R + 1 .. hi
+        Pair<C> rv[R];
+        C rc[R], sum[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          rv[r] = uw[hi - r];
+          rc[r] = uc[hi - r];
+          sum[r] = mk<T>(0, 0);
+        }
+        C* row0 = L + tri(hi) + (k + 1 + lc);
+        // row hi - r starts r hi - r (r - 1) / 2 entries earlier
+#pragma unroll
+        for (int q = 0; q < QC; ++q) {
+          const int j0 = k + 1 + 16 * q;
+          if (j0 > top) break;
+          const Pair<C> cv = cuw[16 * q];
+          const C cc = cuc[16 * q];
+          if (j0 + 15 < top - (2 * R - 1)) {  // all lanes left of every diagonal of the two strips
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              C* e = row0 - (r * hi - r * (r - 1) / 2) + 16 * q;
+              C a = *e;
+              rank2(a, rv[r].u, cv.w, rv[r].w, cv.u);
+              *e = a;
+              cmac(sum[r], a, cc);
+              cmacc(acc[q], a, rc[r]);
+            }
+          } else {
+            const int left = hi - (j0 + lc);  // of row hi's diagonal
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+              C* e = row0 - (r * hi - r * (r - 1) / 2) + 16 * q;
+              C a = *e;  // past the diagonal: the next row's, not kept
+              rank2(a, rv[r].u, cv.w, rv[r].w, cv.u);
+              if (left >= r) *e = a;
+              // half of the diagonal in either part, nothing beyond it
+              a.x = left > r ? a.x : left == r ? T(0.5) * a.x : T(0);
+              a.y = left > r ? a.y : T(0);
+              cmac(sum[r], a, cc);
+              cmacc(acc[q], a, rc[r]);
+            }
+          }
+        }
+        const C tot = half_warp_sum(sum);
+        const int i = hi - (lane & 15) / (16 / R);
+        if (lane % (16 / R) == 0 && i > k) mine[i] = tot;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < QC; ++q) {
+        const int j = k + 1 + lc + 16 * q;
+        acc[q] = cadd(acc[q], shfl_xor_c(acc[q], 16));
+        if (lane < 16 && j < n) {
+          if (((n - 1 - j) / (2 * R)) % nw == wid) acc[q] = cadd(acc[q], mine[j]);  // a row of this warp's strips
+          mine[j] = acc[q];
+        }
+      }
+      __syncthreads();
     }
-    for (int k = 0; k + 2 < n; ++k)  // reflector k: column k, rows k+1..n-1
-      for (int r = tid; r < n - k - 1; r += nt) w.refl[refl_off(k, n) + r] = s.L[rstart(s, k + 1 + r) + k];
-    __syncthreads();
+    __syncthreads();  // L and the vectors are rewritten for the next point
   }
 }
 
@@ -1542,16 +1522,37 @@ int run_inverse(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t
   }
 }
 
-template <typename T, typename TA>
-int run_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
-  const size_t rsmem = tri_bytes<T>(n);
-  if (int rc_ = allow_smem(reinterpret_cast<const void*>(reduce_kernel<T, TA>), (size_t)(rsmem))) return rc_;
-  const int rocc = occupancy(reduce_kernel<T, TA>, kThreads, rsmem);
+template <typename T, typename TA, int QC, int R, int W>
+int launch_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
+  const size_t rsmem = reduce_smem<T>(n, W);
+  auto kernel = reduce_kernel<T, TA, QC, R, W>;
+  if (int rc_ = allow_smem(reinterpret_cast<const void*>(kernel), rsmem)) return rc_;
+  const int rocc = occupancy(kernel, 32 * W, rsmem);
   if (rocc < 1) return fail(MR_ERR_UNSUPPORTED, "emi: %zu bytes of shared memory per CTA do not fit", rsmem);
   KernelTimer kt(pts.list ? "emi reduce rerun" : sizeof(T) == 8 ? "emi reduce fp64" : "emi reduce fp32", s);
-  reduce_kernel<T, TA><<<(unsigned)std::min<int64_t>(pts.n_pc, (int64_t)sm_count() * rocc), kThreads, rsmem, s>>>(
-      c, pts, n, ws);
+  kernel<<<(unsigned)std::min<int64_t>(pts.n_pc, (int64_t)sm_count() * rocc), 32 * W, rsmem, s>>>(c, pts, n, ws);
   return check_launch("emi reduce");
+}
+
+template <typename T, typename TA>
+int run_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
+  // Warps per point and rows per half-warp strip. Up to 64 images one warp (FP64: two above 32)
+  // needs no or little waiting on other warps and an SM holds many points; above, shared memory
+  // holds two to four points per SM, and more warps each hide their latencies: N = 100, FP32, 1, 2, 4,
+  // 8 warps of 4 rows: 243, 222, 178, 285 ms for 286,294 points; FP64, 4 and 8 warps of 4 rows 6.5 and
+  // 6.2, of 2 rows (128 registers, two CTAs of 8 warps) 6.4 and 5.8 ms for 4,001 points.
+  constexpr bool f64 = sizeof(T) == 8;
+  constexpr int W4 = f64 ? 2 : 1, W8 = f64 ? 8 : 4, R8 = f64 ? 2 : 4;
+  switch ((n + 15) / 16) {
+    case 1: return launch_reduce<T, TA, 1, 4, 1>(c, pts, n, ws, s);
+    case 2: return launch_reduce<T, TA, 2, 4, 1>(c, pts, n, ws, s);
+    case 3: return launch_reduce<T, TA, 3, 4, W4>(c, pts, n, ws, s);
+    case 4: return launch_reduce<T, TA, 4, 4, W4>(c, pts, n, ws, s);
+    case 5: return launch_reduce<T, TA, 5, R8, W8>(c, pts, n, ws, s);
+    case 6: return launch_reduce<T, TA, 6, R8, W8>(c, pts, n, ws, s);
+    case 7: return launch_reduce<T, TA, 7, R8, W8>(c, pts, n, ws, s);
+    default: return launch_reduce<T, TA, 8, R8, W8>(c, pts, n, ws, s);
+  }
 }
 
 // One pass of the three kernels over a sub-batch (pts.list == nullptr: all pts.n_pc points;
