@@ -61,6 +61,24 @@ __device__ int collect_shps(const uint8_t* __restrict__ mask, int az_win, int r_
   return total;
 }
 
+// Out of line: called for a few values in 10^7, from a hundred places of an unrolled epilogue.
+__device__ __noinline__ double quotient(double num, const double* am, const double* aj) {
+  return num / sqrt(*am * *aj);
+}
+
+// (re, im) / sqrt(am aj) rounded to FP32, from f ~ 1 / sqrt(am aj): products in place of an FP64 root
+// and two divisions, which are computed only where a product is within 16 FP64 ulps of the middle
+// between two floats (its error is a few). The same floats as the quotients'.
+__device__ __forceinline__ float2 normalised(double re, double im, double f, const double* am, const double* aj) {
+  double x = re * f, y = im * f;
+  const unsigned lx = (unsigned)__double2loint(x) & 0x1fffffffu, ly = (unsigned)__double2loint(y) & 0x1fffffffu;
+  if (lx - 0x0ffffff0u < 32u || ly - 0x0ffffff0u < 32u) {
+    x = quotient(re, am, aj);
+    y = quotient(im, am, aj);
+  }
+  return make_float2((float)x, (float)y);
+}
+
 __device__ __forceinline__ void copy8(float2* dst, const float2* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
@@ -80,11 +98,12 @@ __device__ __forceinline__ void copy8(float2* dst, const float2* src) {
 // products rounded into one accumulator took six instructions and was less exact). FP64: fetched
 // by cp.async as stored, widened once when staged (at 16 conversions per clock and SM, widening at
 // each use cost as much time as the products themselves), one FMA chain per component. The sums
-// |z|^2 are the Gram's own diagonal: blocks (b, b) come first, in round 0.
+// |z|^2 are the Gram's own diagonal in FP32 (blocks (b, b) come first, in round 0), and
+// summed from the staged rows in FP64.
 // FP32 is bound by its issue slots, FP64 by shared memory (eight 16-byte reads, four wavefronts
 // each, take as long as their 64 FP64 FMAs). FP32, N = 50, 15 x 31 window, 30,011 points: 1.65 ms
 // against 2.9 with a separate pass for |z|^2 and 256-thread CTAs; N = 20 raster of 123 x 131: 0.16
-// against 0.38 ms. FP64 at N = 150, 5,224 points of 166 SHPs: 5.2 against 5.4 ms.
+// against 0.38 ms. FP64 at N = 150, 8,000 points of 95 SHPs: 4.7 against 5.0 ms.
 constexpr int kMaxGramThreads = 192;
 
 template <typename A> struct GramAcc;
@@ -110,6 +129,20 @@ template <> struct GramAcc<double> {
   __device__ __forceinline__ double re() const { return x; }
   __device__ __forceinline__ double im() const { return y; }
 };
+
+// amp2[c] (+)= sum of |z|^2 of each image over ns staged rows (image c at at(c)), each |z|^2 rounded
+// once (its two products are exact in FP64) and added in row order.
+template <class At>
+__device__ __forceinline__ void sum_squares(const double2* rows, int stride, int n, int ns, bool first, double* amp2,
+                                            At at) {
+  for (int c = threadIdx.x; c < n; c += blockDim.x) {
+    const double2* z = rows + at(c);
+    double s = first ? 0.0 : amp2[c];
+#pragma unroll 4
+    for (int t = 0; t < ns; ++t) s += fma(z[t * stride].x, z[t * stride].x, z[t * stride].y * z[t * stride].y);
+    amp2[c] = s;
+  }
+}
 
 // Images 4 b .. 4 b + 3 of a staged row.
 __device__ __forceinline__ void load_block(const float2* row, int nb, int b, float2 (&z)[4]) {
@@ -142,7 +175,8 @@ __global__ void __launch_bounds__(kMaxGramThreads, sizeof(A) == 8 ? 2 : 3) gram_
   C* zc = reinterpret_cast<C*>(smem_raw);                             // FP32: 2 x kc x npad; FP64: kc x npad
   float2* raw = reinterpret_cast<float2*>(zc + (kWide ? 1 : 2) * kc * npad);  // FP64: kc x n, as fetched
   A* amp2 = reinterpret_cast<A*>(raw + (kWide ? kc * n + (kc * n & 1) : 0));  // npad
-  int* s_pos = reinterpret_cast<int*>(amp2 + npad);                   // win
+  A* rinv = amp2 + npad;                                              // FP64: npad
+  int* s_pos = reinterpret_cast<int*>(amp2 + (kWide ? 2 : 1) * npad);  // win
   __shared__ int s_tmp[32];
   const int nblk = nb * (nb + 1) / 2;
   const int64_t npairs = (int64_t)n * (n - 1) / 2;
@@ -188,6 +222,10 @@ __global__ void __launch_bounds__(kMaxGramThreads, sizeof(A) == 8 ? 2 : 3) gram_
       });
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    if constexpr (kWide) {
+      if (S == 0)
+        for (int c = tid; c < n; c += nt) amp2[c] = 0;
+    }
     for (int round = 0; round < rounds; ++round) {
       const int blk = round * nt + tid;
       const bool active = blk < nblk;
@@ -228,6 +266,9 @@ __global__ void __launch_bounds__(kMaxGramThreads, sizeof(A) == 8 ? 2 : 3) gram_
           buf ^= 1;
         }
         __syncthreads();
+        if constexpr (kWide) {
+          if (round == 0) sum_squares(zc, npad, n, ns, s0 == 0, amp2, [&](int c) { return place(0, c); });
+        }
         if (active) {
 #pragma unroll 2
           for (int t = 0; t < ns; ++t, row += npad) {
@@ -242,10 +283,12 @@ __global__ void __launch_bounds__(kMaxGramThreads, sizeof(A) == 8 ? 2 : 3) gram_
         }
         __syncthreads();  // the rows are overwritten by the next pass
       }
-      if (round == 0) {  // FP64: 1 / sqrt of each sum, which saves two divisions per pair
-        if (blk < nb) {
+      if (round == 0) {
+        if constexpr (kWide) {
+          for (int c = tid; c < n; c += nt) rinv[c] = (A)1 / sqrt(amp2[c]);
+        } else if (blk < nb) {
 #pragma unroll
-          for (int a = 0; a < 4; ++a) amp2[4 * blk + a] = kWide ? (A)1 / sqrt(acc[a][a].re()) : acc[a][a].re();
+          for (int a = 0; a < 4; ++a) amp2[4 * blk + a] = acc[a][a].re();
         }
         __syncthreads();
       }
@@ -259,8 +302,8 @@ __global__ void __launch_bounds__(kMaxGramThreads, sizeof(A) == 8 ? 2 : 3) gram_
             const A re = acc[a][b].re(), im = acc[a][b].im();
             float2 g;
             if constexpr (kWide) {
-              const A r = amp2[mm] * amp2[jj];
-              g = make_float2((float)(re * r), (float)(im * r));
+              const A f = rinv[mm] * rinv[jj];
+              g = normalised(re, im, f, amp2 + mm, amp2 + jj);
             } else {
               const A den = sqrt(amp2[mm] * amp2[jj]);
               g = make_float2(re / den, im / den);
@@ -288,9 +331,10 @@ __global__ void __launch_bounds__(kMaxGramThreads, sizeof(A) == 8 ? 2 : 3) gram_
 // the FP64 pipe, 64 FMA per clock and SM, but reads each operand from shared memory once per
 // 16 x 8 block instead of once per 4 x 4. With k = 2 s + {re, im} as the contraction index,
 // A[m][k] = z_m's component k:
-//   Re = sum_k A[m][k] A[j][k],   Im = sum_k A[m][k] A'[j][k],  A' = (-im, re),
-// two products of real matrices with 2 S rows and no redundant sum. Every fragment is plain
-// 8-byte reads of the staged rows (image lane / 4, k = lane % 4).
+//   Re = sum_k A[m][k] A[j][k],   Im = sum_k X[m][k] Y[j][k],  X = (im, re), Y = (re, -im),
+// two products of real matrices with 2 S rows and no redundant sum, each added up in the order of
+// gram_kernel's FMA chain. Every fragment is plain 8-byte reads of the staged rows (image
+// lane / 4, k = lane % 4); Y is a sign on A's.
 //
 // The upper triangle is cut into 16 x 8 blocks, and the blocks into runs of at most SLOTS that
 // span one or two block rows (plan_gram64); a run is one warp's accumulators, its A fragments are
@@ -298,10 +342,13 @@ __global__ void __launch_bounds__(kMaxGramThreads, sizeof(A) == 8 ? 2 : 3) gram_
 // beside a DMMA, so every instruction counts: with a next-block rule per slot it took 5.9 ms
 // below, on m8n8k4 7.9 ms). Four warps of 13 blocks hold 104 images in one pass over the SHPs,
 // two such CTAs per SM; smaller runs leave room for more CTAs. Above that the accumulators
-// need several passes, which measured slower than gram_kernel<double> (6.4 against 5.2 ms at
-// N = 150).
-// N = 100, 11 x 21 window, 20,000 points: 4.6 ms against 6.4 (one CTA of 256 threads, samples
-// widened at each use); gram_kernel<double> 5.1. N = 50, 35,627 points: 2.3 against 4.6 ms; N = 17, 2,047 points: 42 against 126 us.
+// need several passes, which measured slower than gram_kernel<double> (6.4 against 5.2 ms for 5,224
+// points of 166 SHPs at N = 150).
+// N = 100, 11 x 21 window, 20,000 points: 5.2 ms against 6.4 (one CTA of 256 threads, samples
+// widened at each use) and 5.5 with gram_kernel<double>; N = 64 1.9 against 3.3 and 2.8; N = 50,
+// 35,627 points: 2.5 against 4.6; N = 17, 2,047 points: 47 against 126 us. The exact sums |z|^2 and the
+// rounding test of `normalised` are 0.4 ms of the 5.2: without them a few coherences in 10^8 round
+// to the other float, which the EMI of a nearly singular point magnifies to milliradians.
 constexpr int kGramWarps = 4;
 constexpr int kMaxRuns = 8;
 constexpr int kDmmaImages = 104;
@@ -339,7 +386,8 @@ __global__ void __launch_bounds__(32 * kGramWarps, SLOTS <= 4 ? 4 : SLOTS <= 7 ?
                                 // fragment read spans lie on different banks
   double2* zc = reinterpret_cast<double2*>(smem_raw);             // kc (a multiple of 4) x npd
   double* rinv = reinterpret_cast<double*>(zc + kc * npd);         // 16 nr: 1 / sqrt(sum |z|^2)
-  float2* raw = reinterpret_cast<float2*>(rinv + 16 * nr);         // kc x n, as fetched
+  double* amp2 = rinv + 16 * nr;                                   // 16 nr: sum |z|^2
+  float2* raw = reinterpret_cast<float2*>(amp2 + 16 * nr);         // kc x n, as fetched
   int* s_pos = reinterpret_cast<int*>(raw + kc * n);               // win
   __shared__ int s_tmp[32];
   const int64_t npairs = (int64_t)n * (n - 1) / 2;
@@ -378,7 +426,7 @@ __global__ void __launch_bounds__(32 * kGramWarps, SLOTS <= 4 ? 4 : SLOTS <= 7 ?
     asm volatile("" : "+r"(w));  // the run is read for each point: kept over the loop it costs spills
     const GramRun run = plan.run[w];
     const int cnt = run.cnt, c1 = run.c1;
-    const int a1 = 32 * run.br1 + comp, a2 = 32 * run.br2 + comp;
+    const int a1 = 32 * run.br1, a2 = 32 * run.br2;
     const int b1 = 16 * run.bc1, b2 = 16 * ((int)run.bc2 - c1);
     double re[SLOTS][4], im[SLOTS][4];
 #pragma unroll
@@ -404,46 +452,41 @@ __global__ void __launch_bounds__(32 * kGramWarps, SLOTS <= 4 ? 4 : SLOTS <= 7 ?
         for (int c2 = tid; c2 < n; c2 += nt) zc[r * npd + c2] = make_double2(0.0, 0.0);
       fetch(s0 + kc);
       __syncthreads();
+      sum_squares(zc, npd, n, ns, s0 == 0, amp2, [](int c) { return c; });
       const double* z = zk;
       for (int t = 0; t < ns; t += 4, z += 2 * k4) {
-        double a[4];
-        auto load_a = [&](const double* p) {  // rows lane / 4 + 8 (h % 2), k = lane % 4 + 4 (h / 2)
+        double a[4], x[4];  // rows lane / 4 + 8 (h % 2), k = lane % 4 + 4 (h / 2)
+        auto load_a = [&](const double* p, const double* o) {
           a[0] = p[0];
           a[1] = p[16];
           a[2] = p[k4];
           a[3] = p[k4 + 16];
+          x[0] = o[0];
+          x[1] = o[16];
+          x[2] = o[k4];
+          x[3] = o[k4 + 16];
         };
-        load_a(z + a1);
+        load_a(z + a1 + comp, z + a1 + (comp ^ 1));
         const double* p = z + b1 + comp;
-        const double* o = z + b1 + (comp ^ 1);
 #pragma unroll
         for (int q = 0; q < SLOTS; ++q) {
           if (q < cnt) {
             if (q == c1) {
-              load_a(z + a2);
+              load_a(z + a2 + comp, z + a2 + (comp ^ 1));
               p = z + b2 + comp;
-              o = z + b2 + (comp ^ 1);
             }
-            const double b[2] = {p[16 * q], p[16 * q + k4]};
-            const double o0 = o[16 * q], o1 = o[16 * q + k4];
-            const double bx[2] = {comp ? o0 : -o0, comp ? o1 : -o1};
+            double b[2] = {p[16 * q], p[16 * q + k4]};
             dmma(re[q], a, b);
-            dmma(im[q], a, bx);
+            b[0] = comp ? -b[0] : b[0];
+            b[1] = comp ? -b[1] : b[1];
+            dmma(im[q], x, b);
           }
         }
       }
     }
-#pragma unroll
-    for (int q = 0; q < SLOTS; ++q) {
-      if (q < cnt) {
-        const int br = q < c1 ? run.br1 : run.br2, bc = q < c1 ? run.bc1 + q : run.bc2 + q - c1;
-        const int h8 = bc - 2 * br;  // 0 or 1: the diagonal runs through this half of the rows
-        if (h8 < 2 && (row >> 1) == (lane & 3)) {
-          const double d0 = (row & 1) ? re[q][1] : re[q][0], d1 = (row & 1) ? re[q][3] : re[q][2];
-          rinv[8 * bc + row] = 1.0 / sqrt(h8 ? d1 : d0);
-        }
-      }
-    }
+    for (int c = tid; c < n; c += nt) rinv[c] = 1.0 / sqrt(S > 0 ? amp2[c] : 0.0);
+    if (S == 0)
+      for (int c = tid; c < n; c += nt) amp2[c] = 0.0;
     __syncthreads();
     float2* out = coh + i * npairs;
 #pragma unroll
@@ -451,16 +494,13 @@ __global__ void __launch_bounds__(32 * kGramWarps, SLOTS <= 4 ? 4 : SLOTS <= 7 ?
       if (q < cnt) {
         const int br = q < c1 ? run.br1 : run.br2, bc = q < c1 ? run.bc1 + q : run.bc2 + q - c1;
         const int jj = 8 * bc + colp;
-        const double rj0 = rinv[jj], rj1 = rinv[jj + 1];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int mm = 16 * br + row + 8 * h;
-          const double rm = rinv[mm];
-          float2* o = out + (mm * n - ((mm * (mm + 1)) >> 1) - mm - 1 + jj);  // triu_index(mm, jj, n)
-          const double f0 = rm * rj0, f1 = rm * rj1;
-          if (mm < jj && jj < n) o[0] = make_float2((float)(re[q][2 * h] * f0), (float)(im[q][2 * h] * f0));
-          if (mm < jj + 1 && jj + 1 < n)
-            o[1] = make_float2((float)(re[q][2 * h + 1] * f1), (float)(im[q][2 * h + 1] * f1));
+        for (int h = 0; h < 4; ++h) {
+          const int mm = 16 * br + row + 8 * (h >> 1), j = jj + (h & 1);
+          if (mm < j && j < n) {
+            out[mm * n - ((mm * (mm + 1)) >> 1) - mm - 1 + j] =  // triu_index(mm, j, n)
+                normalised(re[q][h], im[q][h], rinv[mm] * rinv[j], amp2 + mm, amp2 + j);
+          }
         }
       }
     }
@@ -569,7 +609,7 @@ int launch_gram(const float2* rslc, int nlines, int width, int n, const int32_t*
   const int threads = std::min(kMaxGramThreads, (nblk + 31) / 32 * 32);
   const size_t row = (size_t)(kWide ? 1 : 2) * 4 * nb * sizeof(C);
   const int kc = chunk_rows(kWide ? 16 : 32, row);
-  const size_t smem = kc * row + (kWide ? ((size_t)kc * n + 1) / 2 * 2 * sizeof(float2) : 0) + 4 * nb * sizeof(A) +
+  const size_t smem = kc * row + (kWide ? ((size_t)kc * n + 1) / 2 * 2 * sizeof(float2) : 0) + (kWide ? 2 : 1) * 4 * nb * sizeof(A) +
                       (size_t)az_win * r_win * sizeof(int);
   if (int rc = allow_smem(reinterpret_cast<const void*>(gram_kernel<A, kFull>), smem)) return rc;
   KernelTimer kt(kWide ? "gram fp64" : "gram fp32", s);
@@ -588,7 +628,7 @@ int launch_gram64(const float2* rslc, int nlines, int width, int n, const int32_
   const GramPlan plan = plan_gram64(n);
   const int threads = 32 * plan.warps;
   const int kc = plan.warps == 1 ? 8 : 16;  // one-warp CTAs stage fewer rows, so that more of them fit an SM
-  const size_t smem = (size_t)kc * ((16 * nr + 4) * sizeof(double2) + n * sizeof(float2)) + 16 * nr * sizeof(double) +
+  const size_t smem = (size_t)kc * ((16 * nr + 4) * sizeof(double2) + n * sizeof(float2)) + 32 * nr * sizeof(double) +
                       (size_t)az_win * r_win * sizeof(int);
   auto go = [&](auto kernel) {
     if (int rc = allow_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
