@@ -26,42 +26,88 @@ __global__ void rslc2amp_kernel(const float2* __restrict__ z, int64_t n, float* 
     amp[i] = abs_c64(z[i]);
 }
 
-// One warp per pixel: the pixel's dates are contiguous (image axis innermost), lanes stride
-// over them; mean, then the population standard deviation about it.
-constexpr int kMaxPerLane = MR_MAX_NIMAGES / 32;
+// |z| to within a fraction of a float32 ulp in FP32: x^2 + y^2 as a sum with its rounding errors, the
+// approximate root corrected by its residual. Squares near the ends of the FP32 range, NaN and
+// infinities take the FP64 path.
+__device__ __forceinline__ float abs_c64_fast(float2 z) {
+  const float p = z.x * z.x, h = z.y * z.y;
+  const float s = p + h;
+  if (!(s > 1e-28f && s < 1e37f)) return abs_c64(z);
+  const float big = fmaxf(p, h), small = fminf(p, h);
+  const float lo = (small - (s - big)) + (fmaf(z.x, z.x, -p) + fmaf(z.y, z.y, -h));
+  const float y = rsqrtf(s), r = s * y;
+  return fmaf(fmaf(-r, r, s) + lo, 0.5f * y, r);
+}
 
-__global__ void amp_disp_kernel(const float2* __restrict__ z, int64_t npix, int n, float* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t p = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < npix; p += warps) {
-    const float2* zp = z + p * n;
-    float a[kMaxPerLane];
-    double s = 0;
+// kPx pixels per group of G lanes and step, lanes over a pixel's dates (contiguous, image axis
+// innermost; NPL per lane). Sums of a - a_0 and (a - a_0)^2 in FP64, a_0 the pixel's first
+// amplitude: the variance about the mean in one pass without cancellation on near-constant (PS)
+// pixels, both sums of all kPx pixels reduced together. Bound by HBM and, below 32 dates a
+// pixel, by the lane sums: 700 x 701 x 30 takes 70 us (with FP64 roots and two sums per
+// pixel one after the other over 16 slots a lane: 383 us).
+constexpr int kPx = 4;
+
+template <int G, int NPL>
+__global__ void __launch_bounds__(256) amp_disp_kernel(const float2* __restrict__ z, int64_t npix, int n,
+                                                       float* __restrict__ out) {
+  const int lane = threadIdx.x & (G - 1);
+  const int64_t groups = (int64_t)gridDim.x * (256 / G);
+  for (int64_t p0 = ((int64_t)blockIdx.x * (256 / G) + threadIdx.x / G) * kPx; p0 - kPx * (threadIdx.x % 32 / G) < npix;
+       p0 += groups * kPx) {  // the test is the same for a whole warp
+    float a[kPx][NPL], a0[kPx];
 #pragma unroll
-    for (int t = 0; t < kMaxPerLane; ++t) {
-      const int k = lane + 32 * t;
-      a[t] = 0.f;
-      if (k < n) {
-        a[t] = abs_c64(zp[k]);
-        s += a[t];
+    for (int q = 0; q < kPx; ++q)
+#pragma unroll
+      for (int t = 0; t < NPL; ++t) {
+        const int k = lane + G * t;
+        a[q][t] = (k < n && p0 + q < npix) ? abs_c64_fast(z[(p0 + q) * n + k]) : 0.f;
+      }
+    double v[2 * kPx];
+#pragma unroll
+    for (int q = 0; q < kPx; ++q) {
+      a0[q] = __shfl_sync(0xffffffffu, a[q][0], 0, G);
+      v[2 * q] = v[2 * q + 1] = 0.0;
+#pragma unroll
+      for (int t = 0; t < NPL; ++t) {
+        const double d = lane + G * t < n ? (double)a[q][t] - (double)a0[q] : 0.0;
+        v[2 * q] += d;
+        v[2 * q + 1] += d * d;
       }
     }
+    // eight sums over G >= 8 lanes: each halving hands half of them to the other half of the lanes,
+    // so that lane l ends with sum l / (G / 8) of the group
+    int live = 2 * kPx;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const double mean = s / n;
-    double v = 0;
+    for (int o = G / 2; o > 0; o >>= 1) {
+      if (live > 1) {
+        live >>= 1;
+        const bool hi = lane & o;
 #pragma unroll
-    for (int t = 0; t < kMaxPerLane; ++t) {
-      const int k = lane + 32 * t;
-      if (k < n) {
-        const double d = (double)a[t] - mean;
-        v += d * d;
+        for (int e = 0; e < kPx; ++e)
+          if (e < live) {
+            const double keep = hi ? v[e + live] : v[e], give = hi ? v[e] : v[e + live];
+            v[e] = keep + __shfl_xor_sync(0xffffffffu, give, o, G);
+          }
+      } else {
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], o, G);
       }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) out[p] = (float)(sqrt(v / n) / mean);  // one rounding: near-constant PS pixels keep their digits
+    const int q = lane / (G / kPx);  // pixel of the sum that this lane holds
+    const double sq = __shfl_xor_sync(0xffffffffu, v[0], G / 8, G);
+    const float first = q == 0 ? a0[0] : q == 1 ? a0[1] : q == 2 ? a0[2] : a0[3];
+    if (lane % (G / kPx) == 0 && p0 + q < npix) {
+      const double m1 = v[0] / n, var = sq / n - m1 * m1;
+      // one rounding: near-constant PS pixels keep their digits
+      out[p0 + q] = (float)(sqrt(var < 0.0 ? 0.0 : var) / ((double)first + m1));
+    }
   }
+}
+
+template <int G, int NPL>
+void launch_amp_disp(const float2* z, int64_t npix, int n, float* out, cudaStream_t s) {
+  const int64_t blocks = (npix + (256 / G) * kPx - 1) / ((256 / G) * kPx);
+  amp_disp_kernel<G, NPL><<<(unsigned)std::min<int64_t>(blocks, (int64_t)sm_count() * 64), 256, 0, s>>>(z, npix, n,
+                                                                                                      out);
 }
 
 // calamp: per-block (sum, count) of the non-NaN amplitudes in double, then one block adds
@@ -125,8 +171,16 @@ extern "C" int mr_amp_disp(const mr_complex64* rslc, int64_t npix, int nimages, 
   if (nimages > MR_MAX_NIMAGES) return fail(MR_ERR_UNSUPPORTED, "amp_disp: nimages %d > %d", nimages, MR_MAX_NIMAGES);
   if (npix == 0) return MR_OK;
   MR_REQUIRE(rslc && amp_disp, "amp_disp: NULL pointer");
-  amp_disp_kernel<<<grid_of(npix, 8), 256, 0, as_stream(stream)>>>(reinterpret_cast<const float2*>(rslc), npix,
-                                                                   nimages, amp_disp);
+  const auto* z = reinterpret_cast<const float2*>(rslc);
+  cudaStream_t s = as_stream(stream);
+  // as many lanes per pixel as it has dates, up to a warp
+  if (nimages <= 8) launch_amp_disp<8, 1>(z, npix, nimages, amp_disp, s);
+  else if (nimages <= 16) launch_amp_disp<16, 1>(z, npix, nimages, amp_disp, s);
+  else if (nimages <= 32) launch_amp_disp<32, 1>(z, npix, nimages, amp_disp, s);
+  else if (nimages <= 64) launch_amp_disp<32, 2>(z, npix, nimages, amp_disp, s);
+  else if (nimages <= 128) launch_amp_disp<32, 4>(z, npix, nimages, amp_disp, s);
+  else if (nimages <= 256) launch_amp_disp<32, 8>(z, npix, nimages, amp_disp, s);
+  else launch_amp_disp<32, 16>(z, npix, nimages, amp_disp, s);
   return check_launch("amp_disp");
 }
 

@@ -121,3 +121,46 @@ def test_coherence_block_shapes(cuda, n):
         np.testing.assert_allclose(coh, coh_ref, atol=2e-6, rtol=0)
         np.testing.assert_allclose(cov, cov_ref, atol=2e-6 * np.abs(cov_ref).max(), rtol=0)
         np.testing.assert_array_equal(coh, np.conj(np.swapaxes(coh, -1, -2)))
+
+
+# ----------------------------------------------------------------------------- streaming statistics
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 16, 17, 32, 33, 64, 65, 129, 300])
+def test_amp_disp_group_shapes(cuda, n):
+    """Amplitude dispersion at the edges of the lane groups; near-constant, tiny, huge, zero,
+    NaN and infinite amplitudes."""
+    rng = np.random.default_rng(n)
+    z = (rng.normal(size=(5, 23, n)) + 1j * rng.normal(size=(5, 23, n))).astype(np.complex64)
+    z[0, 0] = 3 - 4j                       # constant: exactly 0
+    z[0, 1] = (7 + 1e-4 * rng.normal(size=n)).astype(np.complex64)
+    z[0, 2] *= 1e-20
+    z[0, 3] *= 1e25
+    z[0, 4] = 0
+    z[0, 5, -1] = np.nan
+    z[0, 6, 0] = np.inf
+    got = mb.amp_disp(z)
+    amp = np.abs(z.astype(np.complex128))
+    with np.errstate(all="ignore"):
+        ref = amp.std(-1) / amp.mean(-1)
+    # one float32 rounding of the result, and half a float32 ulp per amplitude (5e-8 / dispersion)
+    tol = 1.2e-7 * np.abs(ref) + 6e-8
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(ref))
+    ok = ~np.isnan(ref)
+    assert np.all(np.abs(got - ref)[ok] <= tol[ok])
+    assert got[0, 0] == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 3, 8, 9, 17, 33, 100, 128, 129])
+def test_temp_coh_all_pairs_shapes(cuda, n):
+    """Both temporal coherences over all pairs, at the edges of the unrolled walk and of the pair
+    table, zero and tiny coherence included."""
+    rng = np.random.default_rng(n)
+    q = n * (n - 1) // 2
+    coh = (rng.normal(size=(37, q)) + 1j * rng.normal(size=(37, q))).astype(np.complex64)
+    ph = np.exp(1j * rng.uniform(0, 7, (37, n))).astype(np.complex64)
+    coh[1, 0] = 0                          # 0 / 0
+    coh[2] *= 1e-15
+    np.testing.assert_allclose(mb.ds_temp_coh(coh, ph), O.ds_temp_coh(coh, ph), atol=1e-6)
+    np.testing.assert_allclose(mb.temp_coh(coh, ph), O.temp_coh(coh, ph), atol=1e-6)
+    assert np.isnan(mb.ds_temp_coh(coh, ph)[1])
