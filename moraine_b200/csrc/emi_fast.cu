@@ -394,6 +394,106 @@ __global__ void __launch_bounds__(16 * CX, 1) inverse_kernel(const float2* __res
   }
 }
 
+// ----------------------------------------------------------------- kernel 1c: inverse, N > 128
+// The same Gauss-Jordan (partial pivoting, rows never swapped) with the matrix in shared memory
+// (kIn: up to kBigIn images) or in the CTA's slice of the workspace, one CTA of 32 warps per point.
+// Every warp finds the pivot of column k for itself from the column's values, which the update of
+// step k-1 has put aside, and takes the scaled pivot row into registers; after a barrier the warps
+// update their rows, lanes along the columns. Two barriers per step. Bound by shared-memory (or L2)
+// bandwidth, 16 bytes per element and step.
+constexpr int kBigThreads = 1024;
+constexpr int kBigIn = 160;
+
+template <int Q, bool kIn>
+__global__ void __launch_bounds__(kBigThreads, 1) big_inverse_kernel(const float2* __restrict__ coh, PointSet pts, int n,
+                                                                     unsigned char* __restrict__ ws,
+                                                                     uint8_t* __restrict__ sing,
+                                                                     double* __restrict__ slices) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double col[2][32 * Q];
+  __shared__ int piv_of_step[32 * Q], step_of_row[32 * Q];
+  constexpr int W = kBigThreads / 32;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int ld = kIn ? n | 1 : n;  // odd: a column's values on different banks
+  double* A = kIn ? reinterpret_cast<double*>(smem_raw) : slices + (size_t)blockIdx.x * n * n;
+  const int64_t npairs = (int64_t)n * (n - 1) / 2;
+  const int64_t npt = pts.size();
+  for (int64_t pt = blockIdx.x; pt < npt; pt += gridDim.x) {
+    const float2* c = coh + pts[pt] * npairs;
+    for (int i = wid; i < n; i += W) {
+      const float2* ci = c + (triu_index(i, i + 1, n) - (i + 1));
+      for (int j = i + lane; j < n; j += 32) {
+        const float2 g = j == i ? make_float2(1.f, 0.f) : ci[j];
+        const double v = sqrt((double)g.x * g.x + (double)g.y * g.y);
+        A[i * ld + j] = v;
+        A[j * ld + i] = v;
+        if (i == 0) col[0][j] = v;
+      }
+    }
+    for (int i = tid; i < n; i += kBigThreads) step_of_row[i] = -1;
+    bool singular = false;
+    __syncthreads();
+    for (int k = 0; k < n; ++k) {
+      const double* ck = col[k & 1];
+      double best = -1.0;
+      int p = -1;
+#pragma unroll
+      for (int t = 0; t < Q; ++t) {
+        const int i = lane + 32 * t;
+        if (i < n && step_of_row[i] < 0) {
+          const double av = fabs(ck[i]) == fabs(ck[i]) ? fabs(ck[i]) : -0.5;  // NaN ranks last but is taken
+          if (av > best) { best = av; p = i; }
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, p, o);
+        if (ob > best || (ob == best && oi >= 0 && (p < 0 || oi < p))) { best = ob; p = oi; }
+      }
+      double pv = ck[p];
+      if (pv == 0.0) { singular = true; pv = 1.0; }
+      const double rp = recip(pv);
+      double r[Q];  // the pivot row, scaled
+#pragma unroll
+      for (int t = 0; t < Q; ++t) {
+        const int j = lane + 32 * t;
+        r[t] = j < n ? A[p * ld + j] * rp : 0.0;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        step_of_row[p] = k;
+        piv_of_step[k] = p;
+      }
+      for (int i = wid; i < n; i += W) {
+        double* row = A + i * ld;
+        const double f = ck[i];
+#pragma unroll
+        for (int t = 0; t < Q; ++t) {
+          const int j = lane + 32 * t;
+          if (j < n) {
+            double a = i == p ? r[t] : row[j] - f * r[t];
+            if (j == k) a = i == p ? rp : -f * rp;
+            row[j] = a;
+            if (j == k + 1) col[(k + 1) & 1][i] = a;
+          }
+        }
+      }
+      __syncthreads();
+    }
+    double* out = PointPtr<double, double>(ws, pt, n).ainv;
+    for (int i = wid; i < n; i += W) {
+      const int kr = step_of_row[i];
+      for (int j = lane; j < n; j += 32) {
+        const int pc = piv_of_step[j];
+        if (kr >= pc) out[tri_up(pc, kr, n)] = A[i * ld + j];  // inv[kr][pc], kept once
+      }
+    }
+    if (tid == 0) sing[pt] = singular ? kRouteSingular : 0;
+    __syncthreads();
+  }
+}
+
 // ----------------------------------------------------------------- kernel 1b: symmetric sweep
 // inv(|Gamma|) for the refined mixed precision, FP64: Gauss-Jordan on the symmetric matrix
 // with diagonal pivots in natural order (the sweep operator), which keeps the matrix
@@ -606,9 +706,10 @@ __global__ void __launch_bounds__(256, 2) sweep_kernel(const float2* __restrict_
 // of step k-1 and u_k with kRowPad entries in front (rows above the first of a strip), and each
 // warp's part of M u.
 constexpr int kRowPad = 8, kColPad = 16;
+__host__ __device__ inline size_t reduce_tri(int n) { return (size_t)n * (n + 1) / 2 + kColPad; }
 template <typename T>
-__host__ __device__ inline size_t reduce_smem(int n, int warps) {
-  return ((size_t)n * (n + 1) / 2 + kColPad + 3 * (size_t)(n + kRowPad + kColPad) + (size_t)warps * n) *
+__host__ __device__ inline size_t reduce_smem(int n, int warps, bool tri_in) {
+  return ((tri_in ? reduce_tri(n) : 0) + 3 * (size_t)(n + kRowPad + kColPad) + (size_t)warps * n) *
          sizeof(typename C2<T>::type);
 }
 
@@ -616,9 +717,10 @@ template <typename C> struct alignas(2 * sizeof(C)) Pair {
   C u, w;
 };
 
-template <typename T, typename TA, int QC, int R, int W>
-__global__ void __launch_bounds__(32 * W, W >= 4 ? 16 / W : 1) reduce_kernel(const float2* __restrict__ coh, PointSet pts,
-                                                                          int n, unsigned char* __restrict__ ws) {
+template <typename T, typename TA, int QC, int R, int W, bool kTriIn = true>
+__global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
+    reduce_kernel(const float2* __restrict__ coh, PointSet pts, int n, unsigned char* __restrict__ ws,
+                  typename C2<T>::type* __restrict__ slices) {
   using C = typename C2<T>::type;
   constexpr int Q = (QC + 1) / 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -627,7 +729,7 @@ __global__ void __launch_bounds__(32 * W, W >= 4 ? 16 / W : 1) reduce_kernel(con
   Pair<C>* uw = reinterpret_cast<Pair<C>*>(smem_raw) + kRowPad;  // u_{k-1}, w_{k-1}
   C* uc = reinterpret_cast<C*>(uw + n + kColPad) + kRowPad;      // u_k
   C* part = uc + n + kColPad;                                    // [warps][n]: each warp's part of M u
-  C* L = part + nw * n;
+  C* L = kTriIn ? part + nw * n : slices + blockIdx.x * reduce_tri(n);
   const int64_t npairs = (int64_t)n * (n - 1) / 2;
   const int64_t npt = pts.size();
   for (int e = tid; e < kRowPad; e += blockDim.x) {
@@ -816,14 +918,14 @@ __global__ void __launch_bounds__(32 * W, W >= 4 ? 16 / W : 1) reduce_kernel(con
 
 // Reflector k of a point (its scalar and the lane's four entries, zero past its end) into
 // registers.
-template <typename T, typename TA>
+template <typename T, typename TA, int NR>
 __device__ __forceinline__ void load_refl(const PointPtr<T, TA>& w, int n, int k, int lane,
-                                          typename C2<T>::type (&u)[4], T& tau) {
+                                          typename C2<T>::type (&u)[NR], T& tau) {
   tau = w.tau[k];
   const typename C2<T>::type* src = w.refl + refl_off(k, n);
   const int m = n - k - 1;
 #pragma unroll
-  for (int t = 0; t < 4; ++t) {
+  for (int t = 0; t < NR; ++t) {
     const int i = lane + 32 * t;
     u[t] = i < m ? src[i] : mk<T>(0, 0);
   }
@@ -838,8 +940,9 @@ __host__ __device__ inline size_t tail_warp_bytes(int n) {
   return align16(6 * (size_t)n * sizeof(T)) + align16((size_t)n * sizeof(C)) + align16((size_t)n * sizeof(double2));
 }
 
-template <typename T, typename TA>
-__global__ void __launch_bounds__(32 * kTailWarps, 3) tail_kernel(const float2* __restrict__ coh, PointSet pts, int n,
+// NR: rows per lane (32 NR >= n); W warps per CTA.
+template <typename T, typename TA, int NR, int W>
+__global__ void __launch_bounds__(32 * W, NR <= 4 ? 3 : 1) tail_kernel(const float2* __restrict__ coh, PointSet pts, int n,
                                                               int ref, const unsigned char* __restrict__ ws,
                                                               const uint8_t* __restrict__ sing,
                                                               float2* __restrict__ ph, float* __restrict__ quality,
@@ -859,7 +962,7 @@ __global__ void __launch_bounds__(32 * kTailWarps, 3) tail_kernel(const float2* 
   const int64_t npairs = (int64_t)n * (n - 1) / 2;
   const float fnan = __int_as_float(0x7fffffff);
   const int64_t npt = pts.size();
-  for (int64_t pt = (int64_t)blockIdx.x * kTailWarps + wid; pt < npt; pt += (int64_t)gridDim.x * kTailWarps) {
+  for (int64_t pt = (int64_t)blockIdx.x * W + wid; pt < npt; pt += (int64_t)gridDim.x * W) {
     const int64_t gp = pts[pt];
     const PointPtr<T, TA> w(const_cast<unsigned char*>(ws), pt, n);
     // real tridiagonal: b = |e|, phases delta_{k+1} = delta_k e_k/|e_k| (warp prefix product)
@@ -940,7 +1043,7 @@ __global__ void __launch_bounds__(32 * kTailWarps, 3) tail_kernel(const float2* 
     // reflectors applied from the last; the next one's values are loaded while the current
     // one is applied, so the serial chain does not wait on memory
     {
-      C uu[4], nu[4];
+      C uu[NR], nu[NR];
       T tau = 0, ntau = 0;
       if (n >= 3) load_refl(w, n, n - 3, lane, uu, tau);
       for (int k = n - 3; k >= 0; --k) {
@@ -949,7 +1052,7 @@ __global__ void __launch_bounds__(32 * kTailWarps, 3) tail_kernel(const float2* 
           const int m = n - k - 1;
           C sacc = mk<T>(0, 0);
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
+          for (int t = 0; t < NR; ++t) {
             const int i = lane + 32 * t;
             if (i < m) {
               const C zi = z[k + 1 + i];
@@ -960,7 +1063,7 @@ __global__ void __launch_bounds__(32 * kTailWarps, 3) tail_kernel(const float2* 
           sacc.x = warp_sum(sacc.x);
           sacc.y = warp_sum(sacc.y);
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
+          for (int t = 0; t < NR; ++t) {
             const int i = lane + 32 * t;
             if (i < m) {
               const C tt = cmul_t(uu[t], sacc);
@@ -971,7 +1074,7 @@ __global__ void __launch_bounds__(32 * kTailWarps, 3) tail_kernel(const float2* 
           __syncwarp();
         }
 #pragma unroll
-        for (int t = 0; t < 4; ++t) uu[t] = nu[t];
+        for (int t = 0; t < NR; ++t) uu[t] = nu[t];
         tau = ntau;
       }
     }
@@ -1453,6 +1556,7 @@ struct SubWs {
   uint8_t* sing2;
   int32_t* list;
   int32_t* count;
+  unsigned char* slices;  // above kReduceIn images: per-CTA matrices
   static size_t bytes(int64_t sub, size_t point_bytes, int64_t n_list) {
     return align16((size_t)sub * point_bytes) + 2 * align16((size_t)sub) + align16(4 * (size_t)n_list) + 16;
   }
@@ -1467,6 +1571,7 @@ struct SubWs {
     list = reinterpret_cast<int32_t*>(b);
     b += align16(4 * (size_t)n_list);
     count = reinterpret_cast<int32_t*>(b);
+    slices = b + 16;
   }
 };
 
@@ -1507,6 +1612,36 @@ int launch_inverse(const float2* coh, PointSet pts, int64_t grid_cap, int n, uns
 }
 
 // inv(|Gamma|) in arithmetic TA into a workspace laid out for a reduction in T.
+// Most images with the reduction's FP64 triangle in shared memory.
+constexpr int kReduceIn = 158;
+
+template <int Q, bool kIn>
+int launch_big_inverse(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t* sing, void* slices,
+                       cudaStream_t s) {
+  const size_t smem = kIn ? (size_t)n * (n | 1) * sizeof(double) : 0;
+  auto kernel = big_inverse_kernel<Q, kIn>;
+  if (int rc = allow_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
+  KernelTimer kt("emi inverse fp64", s);
+  kernel<<<(unsigned)std::min<int64_t>(pts.n_pc, sm_count()), kBigThreads, smem, s>>>(c, pts, n, ws, sing,
+                                                                                     static_cast<double*>(slices));
+  return check_launch("emi inverse");
+}
+
+int run_big_inverse(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t* sing, void* slices,
+                    cudaStream_t s) {
+  if (n <= kBigIn) return launch_big_inverse<5, true>(c, pts, n, ws, sing, slices, s);
+  if (n <= 192) return launch_big_inverse<6, false>(c, pts, n, ws, sing, slices, s);
+  if (n <= 256) return launch_big_inverse<8, false>(c, pts, n, ws, sing, slices, s);
+  return launch_big_inverse<16, false>(c, pts, n, ws, sing, slices, s);
+}
+
+// Bytes of one CTA's slice (inverse: n x n; reduction: its triangle), one per SM; none where both
+// kernels have their matrix in shared memory.
+size_t slice_bytes(int n) {
+  if (n <= kReduceIn) return 0;
+  return align16(std::max((size_t)n * n * sizeof(double), reduce_tri(n) * sizeof(double2)));
+}
+
 template <typename TA, typename T>
 int run_inverse(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t* sing, float cond_max,
                 cudaStream_t s) {
@@ -1522,15 +1657,18 @@ int run_inverse(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t
   }
 }
 
-template <typename T, typename TA, int QC, int R, int W>
-int launch_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
-  const size_t rsmem = reduce_smem<T>(n, W);
-  auto kernel = reduce_kernel<T, TA, QC, R, W>;
+template <typename T, typename TA, int QC, int R, int W, bool kTriIn = true>
+int launch_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, cudaStream_t s,
+                  typename C2<T>::type* slices = nullptr) {
+  const size_t rsmem = reduce_smem<T>(n, W, kTriIn);
+  auto kernel = reduce_kernel<T, TA, QC, R, W, kTriIn>;
   if (int rc_ = allow_smem(reinterpret_cast<const void*>(kernel), rsmem)) return rc_;
   const int rocc = occupancy(kernel, 32 * W, rsmem);
   if (rocc < 1) return fail(MR_ERR_UNSUPPORTED, "emi: %zu bytes of shared memory per CTA do not fit", rsmem);
   KernelTimer kt(pts.list ? "emi reduce rerun" : sizeof(T) == 8 ? "emi reduce fp64" : "emi reduce fp32", s);
-  kernel<<<(unsigned)std::min<int64_t>(pts.n_pc, (int64_t)sm_count() * rocc), 32 * W, rsmem, s>>>(c, pts, n, ws);
+  // one slice of the workspace per SM where the triangle is not in shared memory
+  const int64_t most = (int64_t)sm_count() * (kTriIn ? rocc : 1);
+  kernel<<<(unsigned)std::min<int64_t>(pts.n_pc, most), 32 * W, rsmem, s>>>(c, pts, n, ws, slices);
   return check_launch("emi reduce");
 }
 
@@ -1555,21 +1693,48 @@ int run_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, cudaStre
   }
 }
 
+// The reduction above kMaxFastN images, FP64: the triangle in shared memory up to kReduceIn images.
+int run_big_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, void* slices, cudaStream_t s) {
+  auto* sl = static_cast<double2*>(slices);
+  if (n <= 144) return launch_reduce<double, double, 9, 4, 8>(c, pts, n, ws, s);
+  if (n <= kReduceIn) return launch_reduce<double, double, 10, 4, 8>(c, pts, n, ws, s);
+  if (n <= 160) return launch_reduce<double, double, 10, 4, 8, false>(c, pts, n, ws, s, sl);
+  if (n <= 192) return launch_reduce<double, double, 12, 4, 8, false>(c, pts, n, ws, s, sl);
+  if (n <= 256) return launch_reduce<double, double, 16, 4, 8, false>(c, pts, n, ws, s, sl);
+  return launch_reduce<double, double, 32, 2, 8, false>(c, pts, n, ws, s, sl);
+}
+
 // One pass of the three kernels over a sub-batch (pts.list == nullptr: all pts.n_pc points;
 // else the listed ones, whose count is read on the device), inverse and reduction both in
 // T. cond_max > 0 flags the points whose condition estimate exceeds it.
+template <typename T, int NR, int W>
+int launch_tail(const float2* c, PointSet pts, int n, int ref, float2* ph, float* quality, float* tcoh,
+                const unsigned char* ws, const uint8_t* sing, cudaStream_t s) {
+  const size_t tsmem = W * tail_warp_bytes<T>(n);
+  auto kernel = tail_kernel<T, T, NR, W>;
+  if (int rc_ = allow_smem(reinterpret_cast<const void*>(kernel), tsmem)) return rc_;
+  const int tocc = std::max(1, occupancy(kernel, 32 * W, tsmem));
+  const int64_t tgrid = std::min<int64_t>((pts.n_pc + W - 1) / W, (int64_t)sm_count() * tocc);
+  KernelTimer kt(pts.list ? "emi tail rerun" : sizeof(T) == 8 ? "emi tail fp64" : "emi tail fp32", s);
+  kernel<<<(unsigned)tgrid, 32 * W, tsmem, s>>>(c, pts, n, ref, ws, sing, ph, quality, tcoh);
+  return check_launch("emi tail");
+}
+
 template <typename T>
 int run_pass(const float2* c, PointSet pts, int n, int ref, float2* ph, float* quality, float* tcoh,
-             unsigned char* ws, uint8_t* sing, float cond_max, cudaStream_t s) {
+             unsigned char* ws, uint8_t* sing, float cond_max, void* slices, cudaStream_t s) {
+  if constexpr (sizeof(T) == 8) {
+    if (n > kMaxFastN) {
+      if (int rc = run_big_inverse(c, pts, n, ws, sing, slices, s)) return rc;
+      if (int rc = run_big_reduce(c, pts, n, ws, slices, s)) return rc;
+      return n <= 160   ? launch_tail<T, 5, 4>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s)
+             : n <= 256 ? launch_tail<T, 8, 4>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s)
+                        : launch_tail<T, 16, 4>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s);
+    }
+  }
   if (int rc = run_inverse<T, T>(c, pts, n, ws, sing, cond_max, s)) return rc;
   if (int rc = run_reduce<T, T>(c, pts, n, ws, s)) return rc;
-  const size_t tsmem = kTailWarps * tail_warp_bytes<T>(n);
-  if (int rc_ = allow_smem(reinterpret_cast<const void*>(tail_kernel<T, T>), (size_t)(tsmem))) return rc_;
-  const int tocc = std::max(1, occupancy(tail_kernel<T, T>, 32 * kTailWarps, tsmem));
-  const int64_t tgrid = std::min<int64_t>((pts.n_pc + kTailWarps - 1) / kTailWarps, (int64_t)sm_count() * tocc);
-  KernelTimer kt(pts.list ? "emi tail rerun" : sizeof(T) == 8 ? "emi tail fp64" : "emi tail fp32", s);
-  tail_kernel<T, T><<<(unsigned)tgrid, 32 * kTailWarps, tsmem, s>>>(c, pts, n, ref, ws, sing, ph, quality, tcoh);
-  return check_launch("emi tail");
+  return launch_tail<T, 4, kTailWarps>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s);
 }
 
 template <int NB>
@@ -1616,9 +1781,10 @@ size_t point_bytes_max(int n) {
 
 }  // namespace
 
-int fast_supported(int n) { return n >= 2 && n <= kMaxFastN; }
-
 size_t fast_workspace_bytes(int64_t n_pc, int n) {
+  if (n > kMaxFastN)
+    return SubWs::bytes(std::min<int64_t>(n_pc, sub_batch<double>(n)), PointWs<double>(n).bytes, n_pc) +
+           std::min<int64_t>(n_pc, sm_count()) * slice_bytes(n);
   const int64_t s32 = std::min<int64_t>(n_pc, sub_batch<float>(n));
   const int64_t s64 = std::min<int64_t>(n_pc, sub_batch<double>(n));
   return std::max(SubWs::bytes(s32, PointWs<float>(n).bytes, n_pc), SubWs::bytes(s64, point_bytes_max(n), n_pc));
@@ -1651,11 +1817,11 @@ int fast_run(const float2* coh, int64_t n_pc, int n, int ref, int precision, flo
     const PointSet all{nullptr, nullptr, nb, dcount, doff + b0};
     int rc;
     if (f64) {
-      rc = run_pass<double>(c, all, n, ref, p, q, t, w.pts, w.sing, 0.f, s);
+      rc = run_pass<double>(c, all, n, ref, p, q, t, w.pts, w.sing, 0.f, w.slices, s);
       if (!rc && route) MR_CUDA_TRY(cudaMemsetAsync(route + b0, 1, (size_t)nb, s));
     } else {
       rc = refine ? run_refine_pass(c, all, n, ref, p, q, t, w.pts, w.sing, (double)cond_max, s)
-                  : run_pass<float>(c, all, n, ref, p, q, t, w.pts, w.sing, mixed ? cond_max : 0.f, s);
+                  : run_pass<float>(c, all, n, ref, p, q, t, w.pts, w.sing, mixed ? cond_max : 0.f, nullptr, s);
       if (!rc && routed) {
         const int grid = (int)std::min<int64_t>((nb + 255) / 256, (int64_t)sm_count() * 8);
         route_kernel<<<grid, 256, 0, s>>>(w.sing, nb, b0, w.list, w.count, route ? route + b0 : nullptr, refine,
@@ -1672,7 +1838,7 @@ int fast_run(const float2* coh, int64_t n_pc, int n, int ref, int precision, flo
   if (routed) {
     for (int64_t l0 = 0; l0 < n_pc; l0 += sub) {
       const int rc = run_pass<double>(coh, PointSet{w.list, w.count, sub, nullptr, l0}, n, ref, ph, quality, tcoh,
-                                      w.pts, w.sing2, 0.f, s);
+                                      w.pts, w.sing2, 0.f, nullptr, s);
       if (rc) return rc;
     }
   }

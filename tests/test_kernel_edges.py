@@ -164,3 +164,38 @@ def test_temp_coh_all_pairs_shapes(cuda, n):
     np.testing.assert_allclose(mb.ds_temp_coh(coh, ph), O.ds_temp_coh(coh, ph), atol=1e-6)
     np.testing.assert_allclose(mb.temp_coh(coh, ph), O.temp_coh(coh, ph), atol=1e-6)
     assert np.isnan(mb.ds_temp_coh(coh, ph)[1])
+
+
+# ----------------------------------------------------------------------------- EMI
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 3, 15, 16, 17, 32, 33, 48, 49, 64, 65, 80, 97, 113, 128, 129, 144, 145, 158, 159,
+                               160, 161, 192, 193, 257])
+def test_emi_block_shapes(cuda, n):
+    """EMI at the edges of its kernels' tiles, warps and matrix placements against LAPACK FP64; a
+    point whose |Gamma| is singular gives NaN and leaves its neighbours alone."""
+    rng = np.random.default_rng(n)
+    npts, looks = (40, 2 * n + 8) if n <= 128 else (7, n + 40)
+    z = rng.normal(size=(npts, looks, n)) + 1j * rng.normal(size=(npts, looks, n))
+    z += 0.8 * rng.normal(size=(npts, looks, 1)) * np.exp(1j * rng.uniform(0, 6, (npts, 1, n)))
+    c = np.einsum("pli,plj->pij", z, z.conj())
+    d = np.sqrt(np.einsum("pii->pi", c).real)
+    r, s = np.triu_indices(n, 1)
+    coh = (c / (d[:, :, None] * d[:, None, :]))[:, r, s].astype(np.complex64)
+    ref = n // 2
+    ph_r, q_r, gap, cond = O.emi(coh, ref=ref)
+    singular = coh.copy()
+    singular[3] = 1.0  # |Gamma| = ones
+    for precision in ("fp64",) if n > 128 else ("fp64", "fp32"):
+        ph, q = mb.emi(coh, ref=ref, precision=precision)
+        eps, floor = (1e3 * 1.2e-16, 3e-7) if precision == "fp64" else (4 * 6e-8, 2e-6)
+        err = np.abs(np.angle(ph * np.conj(ph_r))).max(-1)
+        assert np.all(err <= O.phase_tolerance(cond, gap, eps=eps, floor=floor))
+        qtol = np.maximum(1e-5, eps * cond if precision == "fp64" else 1e-5 * cond) * np.maximum(1, np.abs(q_r))
+        assert np.all(np.abs(q - q_r) <= qtol)
+        ph2, q2 = mb.emi(singular, ref=ref, precision=precision)
+        keep = np.arange(npts) != 3
+        np.testing.assert_array_equal(ph2[keep], ph[keep])
+        assert n == 2 or (np.isnan(ph2[3]).all() and np.isnan(q2[3]))
+    if n > 128:
+        _, _, route = mb.emi(coh, ref=ref, precision="refine", return_route=True)
+        assert (route == 1).all()
