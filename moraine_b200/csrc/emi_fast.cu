@@ -397,10 +397,10 @@ __global__ void __launch_bounds__(16 * CX, 1) inverse_kernel(const float2* __res
 // ----------------------------------------------------------------- kernel 1c: inverse, N > 128
 // The same Gauss-Jordan (partial pivoting, rows never swapped) with the matrix in shared memory
 // (kIn: up to kBigIn images) or in the CTA's slice of the workspace, one CTA of 32 warps per point.
-// Every warp finds the pivot of column k for itself from the column's values, which the update of
-// step k-1 has put aside, and takes the scaled pivot row into registers; after a barrier the warps
-// update their rows, lanes along the columns. Two barriers per step. Bound by shared-memory (or L2)
-// bandwidth, 16 bytes per element and step.
+// Every warp takes the pivot of column k from the 32 warps' candidates, which they left with the
+// column's values while they updated it in step k-1, and the scaled pivot row into registers; after
+// a barrier the warps update their rows, lanes along the columns. Two barriers per step. Bound by
+// shared-memory (or L2) bandwidth, 16 bytes per element and step.
 constexpr int kBigThreads = 1024;
 constexpr int kBigIn = 160;
 
@@ -413,6 +413,9 @@ __global__ void __launch_bounds__(kBigThreads, 1) big_inverse_kernel(const float
   __shared__ double col[2][32 * Q];
   __shared__ int piv_of_step[32 * Q], step_of_row[32 * Q];
   constexpr int W = kBigThreads / 32;
+  static_assert(W == 32, "one candidate per lane");
+  __shared__ double cand[W];
+  __shared__ int cand_row[W];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int ld = kIn ? n | 1 : n;  // odd: a column's values on different banks
   double* A = kIn ? reinterpret_cast<double*>(smem_raw) : slices + (size_t)blockIdx.x * n * n;
@@ -430,21 +433,24 @@ __global__ void __launch_bounds__(kBigThreads, 1) big_inverse_kernel(const float
         if (i == 0) col[0][j] = v;
       }
     }
-    for (int i = tid; i < n; i += kBigThreads) step_of_row[i] = -1;
+    if (lane == 0) {  // the first column's candidates
+      double best = -1.0;
+      int at = -1;
+      for (int i = wid; i < n; i += W) {
+        const float2 g = i ? c[i - 1] : make_float2(1.f, 0.f);
+        const double v = sqrt((double)g.x * g.x + (double)g.y * g.y), av = v == v ? v : -0.5;
+        if (av > best) { best = av; at = i; }
+      }
+      cand[wid] = best;
+      cand_row[wid] = at;
+    }
+    unsigned used = 0;  // bit r: this warp's row wid + W r has been a pivot row
     bool singular = false;
     __syncthreads();
     for (int k = 0; k < n; ++k) {
       const double* ck = col[k & 1];
-      double best = -1.0;
-      int p = -1;
-#pragma unroll
-      for (int t = 0; t < Q; ++t) {
-        const int i = lane + 32 * t;
-        if (i < n && step_of_row[i] < 0) {
-          const double av = fabs(ck[i]) == fabs(ck[i]) ? fabs(ck[i]) : -0.5;  // NaN ranks last but is taken
-          if (av > best) { best = av; p = i; }
-        }
-      }
+      double best = cand[lane];  // W = 32 candidates, -1 and no row from a warp with none left
+      int p = cand_row[lane];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         const double ob = __shfl_xor_sync(0xffffffffu, best, o);
@@ -465,19 +471,37 @@ __global__ void __launch_bounds__(kBigThreads, 1) big_inverse_kernel(const float
         step_of_row[p] = k;
         piv_of_step[k] = p;
       }
-      for (int i = wid; i < n; i += W) {
+      if (wid == (p & (W - 1))) used |= 1u << (p / W);
+      double* cn = col[(k + 1) & 1];
+      double top = -1.0;
+      int at = -1;
+      for (int i = wid, b = 0; i < n; i += W, ++b) {
         double* row = A + i * ld;
-        const double f = ck[i];
+        if (i == p) {
 #pragma unroll
-        for (int t = 0; t < Q; ++t) {
-          const int j = lane + 32 * t;
-          if (j < n) {
-            double a = i == p ? r[t] : row[j] - f * r[t];
-            if (j == k) a = i == p ? rp : -f * rp;
-            row[j] = a;
-            if (j == k + 1) col[(k + 1) & 1][i] = a;
+          for (int t = 0; t < Q; ++t)
+            if (lane + 32 * t < n) row[lane + 32 * t] = r[t];
+        } else {
+          const double f = ck[i];
+#pragma unroll
+          for (int t = 0; t < Q; ++t) {
+            const int j = lane + 32 * t;
+            if (32 * t + 31 < n || j < n) row[j] -= f * r[t];
           }
         }
+        __syncwarp();
+        if (lane == 0) {  // column k, and column k + 1 with this warp's best unused row for the next step
+          row[k] = i == p ? rp : -ck[i] * rp;
+          if (k + 1 < n) {
+            const double v = row[k + 1], av = fabs(v) == fabs(v) ? fabs(v) : -0.5;  // NaN ranks last but is taken
+            cn[i] = v;
+            if (!(used >> b & 1) && av > top) { top = av; at = i; }
+          }
+        }
+      }
+      if (lane == 0) {
+        cand[wid] = top;
+        cand_row[wid] = at;
       }
       __syncthreads();
     }
