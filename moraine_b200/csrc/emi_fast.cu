@@ -1,23 +1,26 @@
-// EMI for N <= 128 (moraine/pl.py:46-77: M = inv(|Gamma|) o Gamma, its smallest eigenpair,
-// phases referred to image `ref`, fused temporal coherence), in sub-batches of points.
+// EMI (moraine/pl.py:46-77: M = inv(|Gamma|) o Gamma, its smallest eigenpair, phases referred to
+// image `ref`, fused temporal coherence), in sub-batches of points: in FP32, FP64 or refined up
+// to 128 images, in FP64 above.
 //
 // Kernels, each at its own occupancy (the register-bound inverse is not held back by the
-// shared memory of the reduction, and the serial O(N) tails of many points overlap on an SM):
-//   inverse_kernel<T, NB>  inv(|Gamma|) by Gauss-Jordan with partial pivoting in registers
+// shared memory of the reduction, and serial recurrences of many points share a warp):
+//   inverse_kernel         inv(|Gamma|) by Gauss-Jordan with partial pivoting in registers
 //                          (gj_tile): the padded 16NB x 16NB matrix on a 16 x 16 thread grid,
 //                          rows never swapped, one barrier per step; the result stored
 //                          upper-packed in the workspace. FP32 and FP64 EMI, and the FP64
 //                          recomputation of routed points.
-//   sweep_kernel<NB>       inv(|Gamma|) in FP64 for the refined EMI: the symmetric sweep, two
+//   sweep_kernel           inv(|Gamma|) in FP64 for the refined EMI: the symmetric sweep, two
 //                          pivots per barrier, only the lower triangle held.
-//   reduce_kernel<T, TA>   M in shared memory as a packed lower triangle, Householder
-//                          reduction to a real tridiagonal (tridiag_packed) -> workspace (d, e,
-//                          tau, reflectors).
-//   tail_kernel<T, TA>     one warp per point: smallest eigenvalue by Sturm multisection,
-//                          inverse iteration, back-transformation, normalisation, temporal
+//   big_inverse_kernel     the pivoted inverse above 128 images, in shared memory or L2.
+//   reduce_kernel          M in shared memory as a packed lower triangle, Householder
+//                          reduction to a Hermitian tridiagonal -> workspace (d, e, tau,
+//                          reflectors).
+//   tri_eig_kernel         smallest eigenpair of the real tridiagonal: Sturm counts and inverse
+//                          iteration, several points per warp.
+//   tail_kernel            one warp per point: back-transformation, normalisation, temporal
 //                          coherence.
-//   tail_refine_kernel     the refined EMI's tail: FP32 eigenpair of the tridiagonal, one FP64
-//                          Newton correction and an FP64 error bound that routes the points
+//   refine_*_kernel        the refined EMI's tail: one FP64 Newton correction of the FP32
+//                          eigenvector and an FP64 error bound that routes the points
 //                          it does not certify to FP64.
 //   route_kernel           collects the points to recompute in FP64 over all sub-batches.
 #include <algorithm>
@@ -300,8 +303,10 @@ struct PointWs {
     np = (size_t)n * (n + 1) / 2;
     nq = (size_t)n * (n - 1) / 2;
     bytes = align16(np * sizeof(TA)) + align16(nq * sizeof(C)) + align16(2 * (size_t)n * sizeof(T)) +
-            align16((size_t)n * sizeof(C));
+            align16((size_t)n * sizeof(C)) + align16(((size_t)n + 2) * sizeof(T)) +
+            (kRefined ? (2 * (size_t)n + 1) * sizeof(double2) : 0);
   }
+  static constexpr bool kRefined = sizeof(T) == 4 && sizeof(TA) == 8;
 };
 
 template <typename T, typename TA = T>
@@ -312,6 +317,11 @@ struct PointPtr {
   T* d;
   T* tau;
   C* e;
+  T* y;        // eigenvector of the real tridiagonal
+  T* scal;     // its eigenvalue; the tridiagonal's largest row sum
+  double2* v;  // refined EMI: eigenvector of M,
+  double2* x;  // right-hand side and solution of the projected solve,
+  double* lam; // Rayleigh quotient
   __device__ PointPtr(unsigned char* ws, int64_t pt, int n) {
     const PointWs<T, TA> w(n);
     unsigned char* b = ws + (size_t)pt * w.bytes;
@@ -323,6 +333,13 @@ struct PointPtr {
     tau = d + n;
     b += align16(2 * (size_t)n * sizeof(T));
     e = reinterpret_cast<C*>(b);
+    b += align16((size_t)n * sizeof(C));
+    y = reinterpret_cast<T*>(b);
+    scal = y + n;
+    b += align16(((size_t)n + 2) * sizeof(T));
+    v = reinterpret_cast<double2*>(b);
+    x = v + n;
+    lam = reinterpret_cast<double*>(x + n);
   }
 };
 
@@ -940,227 +957,89 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
   }
 }
 
-// Reflector k of a point (its scalar and the lane's four entries, zero past its end) into
-// registers.
+// Reflector k of a point (its scalar and the lane's entries, of rows lane + 32 t) into registers.
 template <typename T, typename TA, int NR>
 __device__ __forceinline__ void load_refl(const PointPtr<T, TA>& w, int n, int k, int lane,
                                           typename C2<T>::type (&u)[NR], T& tau) {
   tau = w.tau[k];
-  const typename C2<T>::type* src = w.refl + refl_off(k, n);
-  const int m = n - k - 1;
+  const typename C2<T>::type* src = w.refl + refl_off(k, n) - (k + 1);
 #pragma unroll
   for (int t = 0; t < NR; ++t) {
     const int i = lane + 32 * t;
-    u[t] = i < m ? src[i] : mk<T>(0, 0);
+    u[t] = i > k && i < n ? src[i] : mk<T>(0, 0);
   }
 }
 
-// ----------------------------------------------------------------- kernel 3: tail, one warp per point
-constexpr int kTailWarps = 8;
-
-template <typename T>
-__host__ __device__ inline size_t tail_warp_bytes(int n) {
+// z <- H_k z for the reflectors of the workspace, k ascending (forward, Q^H z) or descending (back,
+// Q z), z in registers (row lane + 32 t). A ring of D reflectors is on its way while one is applied,
+// so that the serial chain does not wait on memory. One warp.
+template <typename T, typename TA, int NR>
+__device__ __forceinline__ void apply_q(const PointPtr<T, TA>& w, int n, typename C2<T>::type (&z)[NR], bool forward) {
   using C = typename C2<T>::type;
-  return align16(6 * (size_t)n * sizeof(T)) + align16((size_t)n * sizeof(C)) + align16((size_t)n * sizeof(double2));
-}
-
-// NR: rows per lane (32 NR >= n); W warps per CTA.
-template <typename T, typename TA, int NR, int W>
-__global__ void __launch_bounds__(32 * W, NR <= 4 ? 3 : 1) tail_kernel(const float2* __restrict__ coh, PointSet pts, int n,
-                                                              int ref, const unsigned char* __restrict__ ws,
-                                                              const uint8_t* __restrict__ sing,
-                                                              float2* __restrict__ ph, float* __restrict__ quality,
-                                                              float* __restrict__ tcoh) {
-  using C = typename C2<T>::type;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  unsigned char* mine = smem_raw + (size_t)wid * tail_warp_bytes<T>(n);
-  T* d = reinterpret_cast<T*>(mine);
-  T* b = d + n;
-  T* b2 = b + n;
-  T* y = b2 + n;
-  T* w1 = y + n;
-  T* w2 = w1 + n;
-  C* z = reinterpret_cast<C*>(mine + align16(6 * (size_t)n * sizeof(T)));
-  double2* phs = reinterpret_cast<double2*>(mine + align16(6 * (size_t)n * sizeof(T)) + align16((size_t)n * sizeof(C)));
-  const int64_t npairs = (int64_t)n * (n - 1) / 2;
-  const float fnan = __int_as_float(0x7fffffff);
-  const int64_t npt = pts.size();
-  for (int64_t pt = (int64_t)blockIdx.x * W + wid; pt < npt; pt += (int64_t)gridDim.x * W) {
-    const int64_t gp = pts[pt];
-    const PointPtr<T, TA> w(const_cast<unsigned char*>(ws), pt, n);
-    // real tridiagonal: b = |e|, phases delta_{k+1} = delta_k e_k/|e_k| (warp prefix product)
-    C carry = mk<T>(1, 0);
-    for (int k0 = 0; k0 < n; k0 += 32) {
-      const int k = k0 + lane;
-      if (k < n) d[k] = w.d[k];
-      C f = mk<T>(1, 0);
-      if (k + 1 < n) {
-        const C ek = w.e[k];
-        const T a = sqrt(ek.x * ek.x + ek.y * ek.y);
-        b[k] = a;
-        b2[k] = a * a;
-        if (a > T(0)) f = mk<T>(ek.x / a, ek.y / a);
-      }
-      // inclusive scan of the factors f over the lanes
+  constexpr int D = NR * sizeof(C) <= 16 ? 4 : NR * sizeof(C) <= 64 ? 2 : 1;
+  const int lane = threadIdx.x & 31, steps = n - 2;
+  C u[D][NR];
+  T tau[D];
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const T ox = __shfl_up_sync(0xffffffffu, f.x, o), oy = __shfl_up_sync(0xffffffffu, f.y, o);
-        if (lane >= o) f = cmul_t(mk<T>(ox, oy), f);
-      }
-      const C dl = cmul_t(carry, f);  // delta_{k+1}
-      if (k0 == 0 && lane == 0) z[0] = mk<T>(1, 0);
-      if (k + 1 < n) z[k + 1] = dl;
-      carry = mk<T>(__shfl_sync(0xffffffffu, dl.x, 31), __shfl_sync(0xffffffffu, dl.y, 31));
-    }
-    __syncwarp();
-    // lambda_min by multisection
-    T lo = Lim<T>::huge(), hi = -Lim<T>::huge(), tnorm = 0;
-    for (int i = lane; i < n; i += 32) {
-      const T r = (i > 0 ? b[i - 1] : T(0)) + (i + 1 < n ? b[i] : T(0));
-      lo = fmin(lo, d[i] - r);
-      hi = fmax(hi, d[i] + r);
-      tnorm = fmax(tnorm, fabs(d[i]) + r);
-    }
+  for (int r = 0; r < D; ++r) {
+    tau[r] = T(0);
+    if (r < steps) load_refl(w, n, forward ? r : n - 3 - r, lane, u[r], tau[r]);
+  }
+  for (int s0 = 0; s0 < steps; s0 += D) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-      tnorm = fmax(tnorm, __shfl_xor_sync(0xffffffffu, tnorm, o));
-    }
-    const T eps = Lim<T>::eps();
-    const T pivmin = fmax(Lim<T>::tiny(), eps * eps * tnorm * tnorm) + Lim<T>::tiny();
-    const T pad = T(2) * eps * fmax(tnorm, Lim<T>::tiny()) + T(2) * pivmin;
-    lo -= pad;
-    hi += pad;
-    for (int it = 0; it < 64; ++it) {
-      const T width = hi - lo;
-      if (!(width > T(2) * eps * fmax(fabs(lo), fabs(hi)) + T(4) * pivmin)) break;
-      const T sg = lo + width * (T)(lane + 1) / T(33);
-      const int cnt = sturm_count(d, b2, n, sg, pivmin);
-      const unsigned ball = __ballot_sync(0xffffffffu, cnt >= 1);
-      const int first = ball ? __ffs(ball) - 1 : 32;
-      const T nlo = (first == 0) ? lo : lo + width * (T)first / T(33);
-      const T nhi = (first == 32) ? hi : lo + width * (T)(first + 1) / T(33);
-      lo = nlo;
-      hi = nhi;
-    }
-    const T lam = T(0.5) * (lo + hi);
-    // eigenvector of the real tridiagonal by inverse iteration (lane 0)
-    for (int i = lane; i < n; i += 32) y[i] = T(1) + T(0.25) * (T)((i * 37) % 11) / T(11);
-    __syncwarp();
-    if (lane == 0) {
-      const T tiny = eps * fmax(tnorm, Lim<T>::tiny());
-      for (int it = 0; it < 2; ++it) {
-        tridiag_solve(d, b, n, lam, tiny, y, w1, w2, b2);  // b2 is free after the bisection
-        T sc = 0;
-        for (int i = 0; i < n; ++i) sc = fmax(sc, fabs(y[i]));
-        if (!(sc > T(0)) || !isfinite(sc)) break;
-        const T r = T(1) / sc;
-        for (int i = 0; i < n; ++i) y[i] *= r;
-      }
-    }
-    __syncwarp();
-    // v = Q D y
-    for (int i = lane; i < n; i += 32) { const C dl = z[i]; z[i] = mk<T>(dl.x * y[i], dl.y * y[i]); }
-    __syncwarp();
-    // reflectors applied from the last; the next one's values are loaded while the current
-    // one is applied, so the serial chain does not wait on memory
-    {
-      C uu[NR], nu[NR];
-      T tau = 0, ntau = 0;
-      if (n >= 3) load_refl(w, n, n - 3, lane, uu, tau);
-      for (int k = n - 3; k >= 0; --k) {
-        if (k > 0) load_refl(w, n, k - 1, lane, nu, ntau);
-        if (tau != T(0)) {
-          const int m = n - k - 1;
-          C sacc = mk<T>(0, 0);
+    for (int r = 0; r < D; ++r) {
+      const int s = s0 + r;
+      if (s >= steps) break;
+      C acc = mk<T>(0, 0);
 #pragma unroll
-          for (int t = 0; t < NR; ++t) {
-            const int i = lane + 32 * t;
-            if (i < m) {
-              const C zi = z[k + 1 + i];
-              sacc.x += uu[t].x * zi.x + uu[t].y * zi.y;
-              sacc.y += uu[t].x * zi.y - uu[t].y * zi.x;
-            }
-          }
-          sacc.x = warp_sum(sacc.x);
-          sacc.y = warp_sum(sacc.y);
+      for (int t = 0; t < NR; ++t) cmacc(acc, u[r][t], z[t]);  // u^H z
+      acc.x = tau[r] * warp_sum(acc.x);
+      acc.y = tau[r] * warp_sum(acc.y);
 #pragma unroll
-          for (int t = 0; t < NR; ++t) {
-            const int i = lane + 32 * t;
-            if (i < m) {
-              const C tt = cmul_t(uu[t], sacc);
-              z[k + 1 + i].x -= tau * tt.x;
-              z[k + 1 + i].y -= tau * tt.y;
-            }
-          }
-          __syncwarp();
-        }
-#pragma unroll
-        for (int t = 0; t < NR; ++t) uu[t] = nu[t];
-        tau = ntau;
+      for (int t = 0; t < NR; ++t) {
+        z[t].x -= u[r][t].x * acc.x;
+        z[t].x += u[r][t].y * acc.y;
+        z[t].y -= u[r][t].x * acc.y;
+        z[t].y -= u[r][t].y * acc.x;
       }
+      if (s + D < steps) load_refl(w, n, forward ? s + D : n - 3 - s - D, lane, u[r], tau[r]);
     }
-    // normalise to the reference image
-    const bool singular = (sing[pt] & kRouteSingular) != 0;
-    const C zr = z[ref];
-    for (int i = lane; i < n; i += 32) {
-      const C v = cmulc_t(z[i], zr);
-      const double vx = v.x, vy = v.y, a = sqrt(vx * vx + vy * vy);
-      float2 o = make_float2((float)(vx / a), (float)(vy / a));
-      if (singular) o = make_float2(fnan, fnan);
-      ph[gp * n + i] = o;
-      phs[i] = make_double2(o.x, o.y);
-    }
-    if (lane == 0) quality[gp] = singular ? fnan : (float)lam;
-    __syncwarp();
-    if (tcoh) {  // |sum_q coh_q/|coh_q| conj(ph_m) ph_j| / n_pairs
-      const float2* c = coh + gp * npairs;
-      double tx = 0, ty = 0;
-      int mm = 0, jj = 1 + lane;
-      while (jj >= n && mm < n - 1) { mm += 1; jj = jj - n + mm + 1; }
-      for (int64_t q = lane; q < npairs; q += 32) {
-        const int m0 = mm, j0 = jj;
-        jj += 32;
-        while (jj >= n && mm < n - 1) { mm += 1; jj = jj - n + mm + 1; }
-        const float2 g = c[q];
-        const double ga = sqrt((double)g.x * g.x + (double)g.y * g.y);
-        const double2 v = cmul(make_double2(g.x / ga, g.y / ga), cmulc(phs[j0], phs[m0]));
-        tx += v.x;
-        ty += v.y;
-      }
-      tx = warp_sum(tx);
-      ty = warp_sum(ty);
-      if (lane == 0) tcoh[gp] = (float)(sqrt(tx * tx + ty * ty) / (double)npairs);
-    }
-    __syncwarp();
   }
 }
 
-
-// ----------------------------------------------------------------- kernel 3b: refined tail
-// For the refined mixed precision (FP64 inverse, FP32 reduction): the FP32 eigenvector is
-// improved by one step of a Newton (Jacobi-Davidson) correction in FP64,
-//   r = M v - lambda v (lambda = v^H M v, M = inv(|Gamma|) o Gamma from the FP64 inverse),
-//   (M - lambda I) dv = r solved approximately through the FP32 factors M ~ Q D R D^H Q^H,
-//   dv = Q D P (R - lambda I)^-1 P D^H Q^H r, P the projector orthogonal to R's eigenvector,
-// which divides the error by about eps32 ||M|| / gap. Then the refined pair is checked in
-// FP64: with residual r', gap g = lambda_2(R) - lambda and smallest component |v_i|, the
-// phase error of every date is at most |r'| / (g min|v_i|); points above `tol` are flagged
-// for an FP64 recomputation. One warp per point.
-constexpr int kRefineWarps = 4;
-
-__host__ __device__ inline size_t refine_warp_bytes(int n) {
-  return align16(6 * (size_t)n * sizeof(float)) + align16(6 * (size_t)n * sizeof(double)) +
-         3 * align16((size_t)n * sizeof(double2));
+// Phases of the real tridiagonal R = D^H T D: delta_0 = 1, delta_{k+1} = delta_k e_k / |e_k|, as a warp
+// prefix product; lane l gets delta of rows l + 32 t. One warp.
+template <typename V, typename T, typename TA, int NR>
+__device__ __forceinline__ void row_phases(const PointPtr<T, TA>& w, int n, typename C2<V>::type (&dl)[NR]) {
+  using C = typename C2<V>::type;
+  const int lane = threadIdx.x & 31;
+  C carry = mk<V>(1, 0);
+#pragma unroll
+  for (int t = 0; t < NR; ++t) {
+    const int i = lane + 32 * t;
+    C f = mk<V>(1, 0);
+    if (i > 0 && i < n) {
+      const V x = w.e[i - 1].x, y = w.e[i - 1].y, a = sqrt(x * x + y * y);
+      if (a > V(0)) f = mk<V>(x / a, y / a);
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const V ox = __shfl_up_sync(0xffffffffu, f.x, o), oy = __shfl_up_sync(0xffffffffu, f.y, o);
+      if (lane >= o) f = cmul_t(mk<V>(ox, oy), f);
+    }
+    dl[t] = cmul_t(carry, f);
+    carry = mk<V>(__shfl_sync(0xffffffffu, dl[t].x, 31), __shfl_sync(0xffffffffu, dl[t].y, 31));
+  }
 }
 
-// Solve (R - lambda I) x = y in place, R real symmetric tridiagonal (d, b), by elimination
-// with row interchanges, for a real (V = T) or complex (V = C2<T>) right-hand side. Each
-// row's final pivot is inverted once and kept in dd, so the back substitution multiplies:
-// one reciprocal per row on the serial chain instead of a division per row and component.
-// dd, du, dl: work arrays of length n; dl ends as the second super-diagonal of each row.
+// ----------------------------------------------------------------- kernel 3: tridiagonal eigenpair
+// Elements of many points' vectors in shared memory: entry i of point p at [i * stride + p].
+template <typename V> struct Strided {
+  V* p;
+  int stride;
+  __device__ __forceinline__ V& operator[](int i) const { return p[i * stride]; }
+};
+
 template <typename T> __device__ __forceinline__ void axpy_r(T& y, T f, const T& x) { y -= f * x; }
 template <typename T> __device__ __forceinline__ void axpy_r(typename C2<T>::type& y, T f,
                                                               const typename C2<T>::type& x) {
@@ -1173,379 +1052,574 @@ template <typename T> __device__ __forceinline__ void scale_r(typename C2<T>::ty
   y.y *= f;
 }
 
-template <typename T, typename V>
-__device__ inline void tridiag_solve_rcp(const T* d, const T* b, int n, T lambda, T tiny, V* y, T* dd, T* du,
-                                         T* dl) {
-  for (int i = 0; i < n; ++i) {
-    dd[i] = d[i] - lambda;
-    if (i < n - 1) { du[i] = b[i]; dl[i] = b[i]; }
-  }
+// Solve (R - lambda I) x = scale y in place, R real symmetric tridiagonal with diagonal d(i) and
+// off-diagonal b(i), by elimination with row interchanges, for a real (V = T) or complex (V = C2<T>)
+// right-hand side. Each row's final pivot is inverted once and kept in dd, so the back substitution
+// multiplies: one reciprocal per row on the serial chain; the row under elimination stays in
+// registers. dd, du, dl: work arrays of length n (dl: the second super-diagonal). One thread.
+template <typename T, typename V, class D, class B>
+__device__ __forceinline__ void tridiag_solve(D d, B b, int n, T lambda, T tiny, T scale, Strided<V> y, Strided<T> dd,
+                                              Strided<T> du, Strided<T> dl) {
+  T di = d(0) - lambda, dui = b(0);
+  V yi = y[0];
+  scale_r<T>(yi, scale);
   for (int i = 0; i < n - 1; ++i) {
-    const T sub = dl[i];
-    if (fabs(dd[i]) >= fabs(sub)) {
-      if (dd[i] == T(0)) dd[i] = tiny;
-      const T r = recip(dd[i]);
-      const T f = sub * r;
-      dd[i + 1] -= f * du[i];
-      axpy_r<T>(y[i + 1], f, y[i]);
+    const T sub = b(i), dn = d(i + 1) - lambda, dun = i < n - 2 ? b(i + 1) : T(0);
+    V yn = y[i + 1];
+    scale_r<T>(yn, scale);
+    if (fabs(di) >= fabs(sub)) {
+      if (di == T(0)) di = tiny;
+      const T r = recip(di), f = sub * r;
+      dd[i] = r;
+      du[i] = dui;
       dl[i] = T(0);
-      dd[i] = r;
+      y[i] = yi;
+      di = dn - f * dui;
+      dui = dun;
+      axpy_r<T>(yn, f, yi);
+      yi = yn;
     } else {
-      const T r = recip(sub);
-      const T f = dd[i] * r;
-      const T t = dd[i + 1];
-      dd[i + 1] = du[i] - f * t;
-      if (i < n - 2) {
-        dl[i] = du[i + 1];
-        du[i + 1] = -f * dl[i];
-      } else {
-        dl[i] = T(0);
-      }
-      du[i] = t;
-      const V ty = y[i];
-      y[i] = y[i + 1];
-      y[i + 1] = ty;
-      axpy_r<T>(y[i + 1], f, y[i]);
+      const T r = recip(sub), f = di * r;
       dd[i] = r;
+      du[i] = dn;
+      dl[i] = dun;
+      y[i] = yn;
+      di = dui - f * dn;
+      dui = -f * dun;
+      axpy_r<T>(yi, f, yn);
     }
   }
-  if (dd[n - 1] == T(0)) dd[n - 1] = tiny;
-  scale_r<T>(y[n - 1], recip(dd[n - 1]));
-  if (n > 1) {
-    axpy_r<T>(y[n - 2], du[n - 2], y[n - 1]);
-    scale_r<T>(y[n - 2], dd[n - 2]);
-  }
-  for (int i = n - 3; i >= 0; --i) {
-    axpy_r<T>(y[i], du[i], y[i + 1]);
-    axpy_r<T>(y[i], dl[i], y[i + 2]);
-    scale_r<T>(y[i], dd[i]);
-  }
-}
-
-// out = M v for M = inv(|Gamma|) o Gamma (Hermitian), read along the upper triangle: the
-// element (m, j > m) adds M_mj v_j to row m and conj(M_mj) v_m to row j. Lanes own columns
-// j = lane + 32 c; rows go four at a time through warp_sum4. One warp.
-__device__ void herm_matvec(const double* __restrict__ ainv, const float2* __restrict__ c, int n,
-                            const double2* v, double2* out) {
-  constexpr int NC = (kMaxFastN + 31) / 32;
-  const int lane = threadIdx.x & 31;
-  double2 vj[NC], cacc[NC];
-#pragma unroll
-  for (int t = 0; t < NC; ++t) {
-    const int j = lane + 32 * t;
-    vj[t] = j < n ? v[j] : make_double2(0, 0);
-    cacc[t] = make_double2(0, 0);
-  }
-  for (int m0 = 0; m0 < n; m0 += 4) {
-    double2 racc[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      racc[r] = make_double2(0, 0);
-      const int m = m0 + r;
-      if (m >= n) continue;  // warp-uniform
-      const double2 vm = v[m];
-      const int64_t um = tri_up(m, m, n), qm = um - (m + 1);
-#pragma unroll
-      for (int t = 0; t < NC; ++t) {
-        const int j = lane + 32 * t;
-        if (j < m || j >= n) continue;
-        const double s = ainv[um + (j - m)];
-        if (j == m) {
-          racc[r].x += s * vm.x;
-          racc[r].y += s * vm.y;
-        } else {
-          const float2 g = c[qm + (j - m)];
-          const double2 a = make_double2(s * (double)g.x, s * (double)g.y);  // M_mj
-          cmac(racc[r], a, vj[t]);
-          cmacc(cacc[t], a, vm);
-        }
-      }
-    }
-    const double2 tot = warp_sum4(racc);
-    const int r = lane >> 3;
-    if ((lane & 7) == 0 && m0 + r < n) out[m0 + r] = tot;
-  }
-  __syncwarp();
-#pragma unroll
-  for (int t = 0; t < NC; ++t) {
-    const int j = lane + 32 * t;
-    if (j < n) out[j] = cadd(out[j], cacc[t]);
-  }
-  __syncwarp();
-}
-
-// z <- H_k z for the reflectors of the workspace, k ascending (forward, Q^H z) or
-// descending (back, Q z), in the arithmetic V of z (float2 or double2); the reflectors'
-// stored values are used exactly. One warp.
-template <typename V, typename T, typename TA>
-__device__ void apply_q(const PointPtr<T, TA>& w, int n, typename C2<V>::type* z, bool forward) {
-  using C = typename C2<T>::type;
-  using CV = typename C2<V>::type;
-  const int lane = threadIdx.x & 31;
-  if (n < 3) return;
-  C cu[4], nu[4];
-  T ct = 0, nt = 0;
-  load_refl(w, n, forward ? 0 : n - 3, lane, cu, ct);
-  for (int s = 0; s + 2 < n; ++s) {
-    const int k = forward ? s : n - 3 - s;
-    if (s + 3 < n) load_refl(w, n, forward ? s + 1 : n - 4 - s, lane, nu, nt);  // the next one, early
-    const V tau = (V)ct;
-    if (tau != V(0)) {
-      const int m = n - k - 1;
-      CV acc = mk<V>(0, 0), uu[4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int i = lane + 32 * t;
-        uu[t] = mk<V>((V)cu[t].x, (V)cu[t].y);
-        if (i < m) cmacc(acc, uu[t], z[k + 1 + i]);  // u^H z
-      }
-      acc.x = warp_sum(acc.x);
-      acc.y = warp_sum(acc.y);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int i = lane + 32 * t;
-        if (i < m) {
-          const CV tt = cmul(uu[t], acc);
-          z[k + 1 + i].x -= tau * tt.x;
-          z[k + 1 + i].y -= tau * tt.y;
-        }
-      }
-      __syncwarp();
-    }
-#pragma unroll
-    for (int t = 0; t < 4; ++t) cu[t] = nu[t];
-    ct = nt;
+  if (di == T(0)) di = tiny;
+  V y1 = yi, y2 = yi;
+  scale_r<T>(y1, recip(di));
+  y[n - 1] = y1;
+  for (int i = n - 2; i >= 0; --i) {
+    V v = y[i];
+    axpy_r<T>(v, du[i], y1);
+    if (i < n - 2) axpy_r<T>(v, dl[i], y2);
+    scale_r<T>(v, dd[i]);
+    y[i] = v;
+    y2 = y1;
+    y1 = v;
   }
 }
 
-// Smallest sigma (to the bisection's resolution) with at least `target` eigenvalues of the
-// real tridiagonal (d, b2) at or below it, by multisection over the warp from [lo, hi].
-template <typename T>
-__device__ T multisect(const T* d, const T* b2, int n, T lo, T hi, int target, T pivmin, int rounds) {
-  const int lane = threadIdx.x & 31;
-  const T eps = Lim<T>::eps();
-  for (int it = 0; it < rounds; ++it) {
-    const T width = hi - lo;
-    if (!(width > T(2) * eps * fmax(fabs(lo), fabs(hi)) + T(4) * pivmin)) break;
-    const T sg = lo + width * (T)(lane + 1) / T(33);
-    const int cnt = sturm_count(d, b2, n, sg, pivmin);
-    const unsigned ball = __ballot_sync(0xffffffffu, cnt >= target);
-    const int first = ball ? __ffs(ball) - 1 : 32;
-    const T nlo = (first == 0) ? lo : lo + width * (T)first / T(33);
-    const T nhi = (first == 32) ? hi : lo + width * (T)(first + 1) / T(33);
-    lo = nlo;
-    hi = nhi;
-  }
-  return T(0.5) * (lo + hi);
-}
+// Smallest eigenvalue of the real tridiagonal (by sections of a bracket, G Sturm counts at a time) and
+// its eigenvector y (two inverse iterations, one lane), G lanes per point and kEigThreads / G points
+// per CTA, everything in shared memory. A warp per point left its other lanes idle in the solves,
+// and 33 sections a round cost 5 times the operations of 5: the serial recurrences of a point
+// take as long either way, but here a warp runs those of 32 / G points at once (286,294 points,
+// N = 100: 2.9 ms). Results (lambda, max row sum, y) go to the workspace.
+constexpr int kEigThreads = 128;
 
-template <typename T>
-__global__ void __launch_bounds__(32 * kRefineWarps, 4) tail_refine_kernel(
-    const float2* __restrict__ coh, PointSet pts, int n, int ref, const unsigned char* __restrict__ ws,
-    uint8_t* __restrict__ sing, float2* __restrict__ ph, float* __restrict__ quality, float* __restrict__ tcoh,
-    double tol) {
+template <typename T> inline size_t eig_smem(int n, int g) { return 6 * (size_t)n * (kEigThreads / g + 1) * sizeof(T); }
+
+template <typename T, typename TA, int G>
+__global__ void __launch_bounds__(kEigThreads) tri_eig_kernel(PointSet pts, int n, unsigned char* __restrict__ ws) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  unsigned char* mine = smem_raw + (size_t)wid * refine_warp_bytes(n);
-  T* d = reinterpret_cast<T*>(mine);
-  T* b = d + n;
-  T* b2 = b + n;
-  T* y = b2 + n;
-  T* w1 = y + n;
-  T* w2 = w1 + n;
-  double* dd = reinterpret_cast<double*>(mine + align16(6 * (size_t)n * sizeof(float)));
-  double* bd = dd + n;
-  double* yd = bd + n;
-  double* s1 = yd + n;
-  double* s2 = s1 + n;
-  double* s3 = s2 + n;
-  float2* z32 = reinterpret_cast<float2*>(s1);  // FP32 work vector; s1 is scratch only inside the solve
-  double2* dph = reinterpret_cast<double2*>(reinterpret_cast<unsigned char*>(dd) + align16(6 * (size_t)n * sizeof(double)));
-  double2* v = dph + n;
-  double2* t1 = v + n;
-  const int64_t npairs = (int64_t)n * (n - 1) / 2;
-  const float fnan = __int_as_float(0x7fffffff);
+  constexpr int P = kEigThreads / G, S = P + 1;
+  const int tid = threadIdx.x, lane = tid & 31, p = tid / G, g = tid % G;
+  T* d0 = reinterpret_cast<T*>(smem_raw);
+  T* b0 = d0 + n * S;
   const int64_t npt = pts.size();
-  for (int64_t pt = (int64_t)blockIdx.x * kRefineWarps + wid; pt < npt; pt += (int64_t)gridDim.x * kRefineWarps) {
-    const int64_t gp = pts[pt];
-    const PointPtr<T, double> w(const_cast<unsigned char*>(ws), pt, n);
-    const float2* c = coh + gp * npairs;
-    // real tridiagonal R: b = |e|, phases delta_{k+1} = delta_k e_k/|e_k| (warp prefix product, FP64)
-    double2 carry = make_double2(1, 0);
-    for (int k0 = 0; k0 < n; k0 += 32) {
-      const int k = k0 + lane;
-      if (k < n) { d[k] = w.d[k]; dd[k] = (double)w.d[k]; }
-      double2 f = make_double2(1, 0);
-      if (k + 1 < n) {
-        const typename C2<T>::type ek = w.e[k];
-        const double ex = ek.x, ey = ek.y, a = sqrt(ex * ex + ey * ey);
-        b[k] = (T)a;
-        b2[k] = (T)a * (T)a;
-        bd[k] = a;
-        if (a > 0.0) f = make_double2(ex / a, ey / a);
-      }
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const double ox = __shfl_up_sync(0xffffffffu, f.x, o), oy = __shfl_up_sync(0xffffffffu, f.y, o);
-        if (lane >= o) f = cmul(make_double2(ox, oy), f);
-      }
-      const double2 dl = cmul(carry, f);
-      if (k0 == 0 && lane == 0) dph[0] = make_double2(1, 0);
-      if (k + 1 < n) dph[k + 1] = dl;
-      carry = make_double2(__shfl_sync(0xffffffffu, dl.x, 31), __shfl_sync(0xffffffffu, dl.y, 31));
+  for (int64_t base = (int64_t)blockIdx.x * P; base < npt; base += (int64_t)gridDim.x * P) {
+    const int here = (int)(npt - base < P ? npt - base : P);
+#pragma unroll 4
+    for (int f = tid; f < here * n; f += kEigThreads) {
+      const int q = f / n, i = f - q * n;
+      const PointPtr<T, TA> w(ws, base + q, n);
+      d0[i * S + q] = w.d[i];
+      const typename C2<T>::type e = w.e[min(i, n - 2)];
+      b0[i * S + q] = sqrt(e.x * e.x + e.y * e.y);  // entry n - 1 is not used
     }
-    __syncwarp();
-    // lambda_1 and lambda_2 of R (FP32 Sturm counts)
+    __syncthreads();
+    const bool live = base + p < npt;
+    const Strided<T> d{d0 + p, S}, b{b0 + p, S}, y{b0 + n * S + p, S}, dd{b0 + 2 * n * S + p, S},
+        du{b0 + 3 * n * S + p, S}, dl{b0 + 4 * n * S + p, S};
     T lo = Lim<T>::huge(), hi = -Lim<T>::huge(), tnorm = 0;
-    for (int i = lane; i < n; i += 32) {
-      const T r = (i > 0 ? b[i - 1] : T(0)) + (i + 1 < n ? b[i] : T(0));
-      lo = fmin(lo, d[i] - r);
-      hi = fmax(hi, d[i] + r);
-      tnorm = fmax(tnorm, fabs(d[i]) + r);
-    }
+    if (live)
+      for (int i = g; i < n; i += G) {
+        const T r = (i > 0 ? b[i - 1] : T(0)) + (i + 1 < n ? b[i] : T(0));
+        lo = fmin(lo, d[i] - r);
+        hi = fmax(hi, d[i] + r);
+        tnorm = fmax(tnorm, fabs(d[i]) + r);
+        if (i + 1 < n) dd[i] = b[i] * b[i];
+        y[i] = T(1) + T(0.25) * (T)((i * 37) % 11) / T(11);
+      }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = G / 2; o > 0; o >>= 1) {
       lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
       hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
       tnorm = fmax(tnorm, __shfl_xor_sync(0xffffffffu, tnorm, o));
     }
+    __syncwarp();
     const T eps = Lim<T>::eps();
     const T pivmin = fmax(Lim<T>::tiny(), eps * eps * tnorm * tnorm) + Lim<T>::tiny();
     const T pad = T(2) * eps * fmax(tnorm, Lim<T>::tiny()) + T(2) * pivmin;
     lo -= pad;
     hi += pad;
-    const T lam1 = multisect(d, b2, n, lo, hi, 1, pivmin, 64);
-    // eigenvector y of R by inverse iteration (FP32, lane 0)
-    for (int i = lane; i < n; i += 32) y[i] = T(1) + T(0.25) * (T)((i * 37) % 11) / T(11);
+    for (int it = 0; it < 64; ++it) {
+      const T width = hi - lo;
+      const bool open = live && width > T(2) * eps * fmax(fabs(lo), fabs(hi)) + T(4) * pivmin;
+      if (!__any_sync(0xffffffffu, open)) break;
+      int cnt = 0;
+      if (open) cnt = sturm_count(d, dd, n, lo + width * (T)(g + 1) / T(G + 1), pivmin);
+      const unsigned ball = __ballot_sync(0xffffffffu, cnt >= 1) >> (lane & ~(G - 1));
+      const unsigned mine = G == 32 ? ball : ball & ((1u << (G & 31)) - 1u);
+      if (open) {
+        const int first = mine ? __ffs(mine) - 1 : G;
+        const T nlo = first == 0 ? lo : lo + width * (T)first / T(G + 1);
+        hi = first == G ? hi : lo + width * (T)(first + 1) / T(G + 1);
+        lo = nlo;
+      }
+    }
+    const T lam = T(0.5) * (lo + hi);
     __syncwarp();
-    if (lane == 0) {
+    if (g == 0 && live) {
       const T tiny = eps * fmax(tnorm, Lim<T>::tiny());
+      T scale = 1;
       for (int it = 0; it < 2; ++it) {
-        tridiag_solve_rcp(d, b, n, lam1, tiny, y, w1, w2, b2);  // b2 is free after the bisections
+        tridiag_solve<T>([&](int i) { return d[i]; }, [&](int i) { return b[i]; }, n, lam, tiny, scale, y, dd, du, dl);
         T sc = 0;
         for (int i = 0; i < n; ++i) sc = fmax(sc, fabs(y[i]));
-        if (!(sc > T(0)) || !isfinite(sc)) break;
-        const T r = T(1) / sc;
-        for (int i = 0; i < n; ++i) y[i] *= r;
+        scale = T(1) / sc;
+        if (!(sc > T(0)) || !isfinite(sc)) { scale = T(1); break; }
       }
+      du[0] = scale;  // for the group's other lanes
     }
     __syncwarp();
-    // y to unit length in FP64; v = Q D y
-    double yn = 0;
-    for (int i = lane; i < n; i += 32) { yd[i] = (double)y[i]; yn += yd[i] * yd[i]; }
-    yn = 1.0 / sqrt(warp_sum(yn));
-    for (int i = lane; i < n; i += 32) {
-      yd[i] *= yn;
-      z32[i] = make_float2((float)(dph[i].x * yd[i]), (float)(dph[i].y * yd[i]));
+    if (live) {
+      const PointPtr<T, TA> w(ws, base + p, n);
+      const T scale = du[0];
+      for (int i = g; i < n; i += G) w.y[i] = y[i] * scale;
+      if (g == 0) {
+        w.scal[0] = lam;
+        w.scal[1] = tnorm;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// ----------------------------------------------------------------- kernel 4: phases from the eigenvector
+constexpr int kTailWarps = 8;
+
+// 1 / sqrt(x) in FP64 from the FP32 root: two Newton steps, to about an FP64 ulp. x within FP32's
+// normal range, else the quotient.
+__device__ __forceinline__ double inv_sqrt(double x) {
+  if (!(x > 1.2e-38 && x < 3.0e38)) return 1.0 / sqrt(x);
+  double y = (double)rsqrtf((float)x);
+  const double h = 0.5 * x;
+  y = y * fma(-h * y, y, 1.5);
+  return y * fma(-h * y, y, 1.5);
+}
+
+// |sum_q coh_q / |coh_q| conj(ph_m) ph_j| / n_pairs of one point, phs its phases. One warp; lane 0's value.
+__device__ __forceinline__ float temp_coh_of(const float2* __restrict__ c, const double2* phs, int n) {
+  const int lane = threadIdx.x & 31;
+  const int npairs = n * (n - 1) / 2;
+  double tx = 0, ty = 0;
+  int mm = 0, jj = 1 + lane;
+  while (jj >= n && mm < n - 1) { mm += 1; jj = jj - n + mm + 1; }
+  auto add = [&](float2 g) {
+    const int m0 = mm, j0 = jj;
+    jj += 32;
+    while (jj >= n && mm < n - 1) { mm += 1; jj = jj - n + mm + 1; }
+    const double gx = g.x, gy = g.y;
+    const double r = inv_sqrt(gx * gx + gy * gy);
+    const double2 v = cmul(make_double2(gx, gy), cmulc(phs[j0], phs[m0]));
+    tx = fma(v.x, r, tx);
+    ty = fma(v.y, r, ty);
+  };
+  int q = lane;
+  for (; q + 96 < npairs; q += 128) {  // four coherences on their way at a time
+    const float2 g0 = c[q], g1 = c[q + 32], g2 = c[q + 64], g3 = c[q + 96];
+    add(g0);
+    add(g1);
+    add(g2);
+    add(g3);
+  }
+  for (; q < npairs; q += 32) add(c[q]);
+  tx = warp_sum(tx);
+  ty = warp_sum(ty);
+  return (float)(sqrt(tx * tx + ty * ty) / (double)npairs);
+}
+
+// Value of row `ref` of a vector held by rows lane + 32 t.
+template <typename C, int NR> __device__ __forceinline__ C row_value(const C (&v)[NR], int ref) {
+  C r = v[0];
+#pragma unroll
+  for (int t = 1; t < NR; ++t)
+    if (ref >> 5 == t) r = v[t];
+  r.x = __shfl_sync(0xffffffffu, r.x, ref & 31);
+  r.y = __shfl_sync(0xffffffffu, r.y, ref & 31);
+  return r;
+}
+
+// ph = v conj(v[ref]) / |.| of one point (NaN where singular) to global memory and to phs.
+template <typename C, int NR>
+__device__ __forceinline__ void write_phases(const C (&v)[NR], int n, int ref, bool singular, float2* __restrict__ ph,
+                                             double2* phs) {
+  const int lane = threadIdx.x & 31;
+  const float fnan = __int_as_float(0x7fffffff);
+  const C zr = row_value(v, ref);
+#pragma unroll
+  for (int t = 0; t < NR; ++t) {
+    const int i = lane + 32 * t;
+    const C q = cmulc_t(v[t], zr);
+    const double vx = q.x, vy = q.y, a = sqrt(vx * vx + vy * vy);
+    float2 o = make_float2((float)(vx / a), (float)(vy / a));
+    if (singular) o = make_float2(fnan, fnan);
+    if (i < n) {
+      ph[i] = o;
+      phs[i] = make_double2(o.x, o.y);
+    }
+  }
+  __syncwarp();
+}
+
+// One warp per point: v = Q D y, normalisation, temporal coherence. NR: rows per lane (32 NR >= n).
+template <typename T, typename TA, int NR>
+__global__ void __launch_bounds__(32 * kTailWarps) tail_kernel(const float2* __restrict__ coh, PointSet pts, int n,
+                                                               int ref, unsigned char* __restrict__ ws,
+                                                               const uint8_t* __restrict__ sing,
+                                                               float2* __restrict__ ph, float* __restrict__ quality,
+                                                               float* __restrict__ tcoh) {
+  using C = typename C2<T>::type;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double2* phs = reinterpret_cast<double2*>(smem_raw) + wid * n;
+  const int64_t npairs = (int64_t)n * (n - 1) / 2;
+  const int64_t npt = pts.size();
+  for (int64_t pt = (int64_t)blockIdx.x * kTailWarps + wid; pt < npt; pt += (int64_t)gridDim.x * kTailWarps) {
+    const int64_t gp = pts[pt];
+    const PointPtr<T, TA> w(ws, pt, n);
+    C z[NR];
+    row_phases<T>(w, n, z);
+#pragma unroll
+    for (int t = 0; t < NR; ++t) {
+      const int i = lane + 32 * t;
+      const T yi = i < n ? w.y[i] : T(0);
+      z[t] = mk<T>(z[t].x * yi, z[t].y * yi);
+    }
+    apply_q(w, n, z, false);
+    const bool singular = (sing[pt] & kRouteSingular) != 0;
+    write_phases(z, n, ref, singular, ph + gp * n, phs);
+    if (lane == 0) quality[gp] = singular ? __int_as_float(0x7fffffff) : (float)w.scal[0];
+    if (tcoh) {
+      const float t = temp_coh_of(coh + gp * npairs, phs, n);
+      if (lane == 0) tcoh[gp] = t;
     }
     __syncwarp();
-    apply_q<float>(w, n, z32, false);
-    for (int i = lane; i < n; i += 32) v[i] = make_double2(z32[i].x, z32[i].y);
-    __syncwarp();
-    // one correction step, then the check
-    double lam = 0, rn = 0;
-    for (int pass = 0; pass < 2; ++pass) {
-      herm_matvec(w.ainv, c, n, v, t1);
-      double vmv = 0, vv = 0;
-      for (int i = lane; i < n; i += 32) {
-        vmv += v[i].x * t1[i].x + v[i].y * t1[i].y;
-        vv += v[i].x * v[i].x + v[i].y * v[i].y;
+  }
+}
+
+// ----------------------------------------------------------------- kernels 4a-c: refined tail
+// For the refined mixed precision (FP64 inverse, FP32 reduction): the FP32 eigenvector is
+// improved by one step of a Newton (Jacobi-Davidson) correction in FP64,
+//   r = M v - lambda v (lambda = v^H M v, M = inv(|Gamma|) o Gamma from the FP64 inverse),
+//   (M - lambda I) dv = r solved approximately through the FP32 factors M ~ Q D R D^H Q^H,
+//   dv = Q D P (R - lambda I)^-1 P D^H Q^H r, P the projector orthogonal to R's eigenvector,
+// which divides the error by about eps32 ||M|| / gap. Then the refined pair is checked in
+// FP64: with residual r', gap g = lambda_2(R) - lambda and smallest component |v_i|, the
+// phase error of every date is at most |r'| / (g min|v_i|); points above `tol` are flagged
+// for an FP64 recomputation. Two kernels of one warp per point (residual; correction and check),
+// the projected solve between them with one thread per point. The reflectors are applied in FP32
+// (the factors hold M only to FP32 accuracy anyway), the projected solve runs in FP64. Bound by the
+// latency of the reads of M and the reflectors at 16 to 20 warps per SM; a group of four matvec rows
+// fetches its values together, without a branch in between (fetched value by value, or two rows at a
+// time behind their bounds tests: 33 and 35 against 22 ms for the residual). 286,294 points, N = 100:
+// 54 ms in all, against 89 for one kernel of a warp per point with the eigenpair and the solves on one
+// lane; 35,627 points, N = 50: 2.0 against 4.8 ms.
+constexpr int kRefineWarps = 4;
+
+// out = M v for M = inv(|Gamma|) o Gamma (Hermitian), read along the upper triangle: the
+// element (m, j > m) adds M_mj v_j to row m and conj(M_mj) v_m to row j. Lanes own columns
+// j = lane + 32 t (vj: v's values there); rows go four at a time through warp_sum4, row values of v
+// and the sums through shared memory. One warp.
+template <int NR>
+__device__ __forceinline__ void herm_matvec(const double* __restrict__ ainv, const float2* __restrict__ c, int n,
+                                            const double2 (&vj)[NR], double2* v, double2* sums, double2 (&out)[NR]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int t = 0; t < NR; ++t) {
+    if (lane + 32 * t < n) v[lane + 32 * t] = vj[t];
+    out[t] = make_double2(0, 0);
+  }
+  __syncwarp();
+  for (int m0 = 0; m0 < n; m0 += 4) {
+    double2 racc[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) racc[r] = make_double2(0, 0);
+#pragma unroll
+    for (int t = 0; t < NR; ++t) {
+      if (32 * t + 31 < m0) continue;  // warp-uniform
+      const int j = lane + 32 * t;
+      double sc[4];
+      float2 g[4];
+      // the four rows' values are fetched together, without a branch: what is outside the triangle
+      // reads an element of its row and counts nothing
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int m = min(m0 + r, n - 1), um = (int)tri_up(m, m, n) - m;
+        sc[r] = ainv[um + max(min(j, n - 1), m)];
+        g[r] = c[max(um - (m + 1) + max(min(j, n - 1), min(m + 1, n - 1)), 0)];
       }
-      vv = warp_sum(vv);
-      lam = warp_sum(vmv) / vv;
-      double r2 = 0;
-      for (int i = lane; i < n; i += 32) {
-        t1[i] = make_double2(t1[i].x - lam * v[i].x, t1[i].y - lam * v[i].y);
-        r2 += t1[i].x * t1[i].x + t1[i].y * t1[i].y;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int m = m0 + r;
+        const double s = j >= m && j < n && m < n ? sc[r] : 0.0;
+        if (j == m) g[r] = make_float2(1.f, 0.f);
+        const double2 a = make_double2(s * (double)g[r].x, s * (double)g[r].y);  // M_mj
+        cmac(racc[r], a, vj[t]);
+        const double2 vm = v[min(m, n - 1)];
+        if (j > m) cmacc(out[t], a, vm);
       }
-      rn = sqrt(warp_sum(r2) / vv);
-      __syncwarp();
-      if (pass == 1) break;
-      // dv = Q D P (R - lam I)^-1 P D^H Q^H r; the reflectors are applied in FP32 (the factors
-      // hold M only to FP32 accuracy anyway), the projected solve runs in FP64
-      for (int i = lane; i < n; i += 32) z32[i] = make_float2((float)t1[i].x, (float)t1[i].y);
-      __syncwarp();
-      apply_q<float>(w, n, z32, true);
-      double2 pr = make_double2(0, 0);
-      for (int i = lane; i < n; i += 32) {
-        t1[i] = cmulc(make_double2(z32[i].x, z32[i].y), dph[i]);  // D^H: times conj(delta_i)
-        pr.x += yd[i] * t1[i].x;
-        pr.y += yd[i] * t1[i].y;
-      }
-      pr.x = warp_sum(pr.x);
-      pr.y = warp_sum(pr.y);
-      for (int i = lane; i < n; i += 32) { t1[i].x -= yd[i] * pr.x; t1[i].y -= yd[i] * pr.y; }
-      __syncwarp();
-      if (lane == 0) tridiag_solve_rcp(dd, bd, n, lam, DBL_EPSILON * (double)tnorm + DBL_MIN, t1, s1, s2, s3);
-      __syncwarp();
-      pr = make_double2(0, 0);
-      for (int i = lane; i < n; i += 32) { pr.x += yd[i] * t1[i].x; pr.y += yd[i] * t1[i].y; }
-      pr.x = warp_sum(pr.x);
-      pr.y = warp_sum(pr.y);
-      for (int i = lane; i < n; i += 32) {
-        const double2 x = cmul(make_double2(t1[i].x - yd[i] * pr.x, t1[i].y - yd[i] * pr.y), dph[i]);
-        z32[i] = make_float2((float)x.x, (float)x.y);
-      }
-      __syncwarp();
-      apply_q<float>(w, n, z32, false);
-      double vn = 0;
-      for (int i = lane; i < n; i += 32) {
-        v[i] = make_double2(v[i].x - (double)z32[i].x, v[i].y - (double)z32[i].y);
-        vn += v[i].x * v[i].x + v[i].y * v[i].y;
-      }
-      vn = 1.0 / sqrt(warp_sum(vn));
-      for (int i = lane; i < n; i += 32) v[i] = make_double2(v[i].x * vn, v[i].y * vn);
-      __syncwarp();
     }
+    const double2 tot = warp_sum4(racc);
+    const int r = lane >> 3;
+    if ((lane & 7) == 0 && m0 + r < n) sums[m0 + r] = tot;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < NR; ++t)
+    if (lane + 32 * t < n) out[t] = cadd(out[t], sums[lane + 32 * t]);
+  __syncwarp();
+}
+
+// v^H M v / v^H v into lam; mv becomes the residual M v - lam v; its norm relative to |v| returned.
+template <int NR>
+__device__ __forceinline__ double residual(const double2 (&v)[NR], double2 (&mv)[NR], double& lam) {
+  double vmv = 0, vv = 0, r2 = 0;
+#pragma unroll
+  for (int t = 0; t < NR; ++t) {
+    vmv += v[t].x * mv[t].x + v[t].y * mv[t].y;
+    vv += v[t].x * v[t].x + v[t].y * v[t].y;
+  }
+  vv = warp_sum(vv);
+  lam = warp_sum(vmv) / vv;
+#pragma unroll
+  for (int t = 0; t < NR; ++t) {
+    mv[t] = make_double2(mv[t].x - lam * v[t].x, mv[t].y - lam * v[t].y);
+    r2 += mv[t].x * mv[t].x + mv[t].y * mv[t].y;
+  }
+  return sqrt(warp_sum(r2) / vv);
+}
+
+// y of unit length in FP64, rows lane + 32 t.
+template <int NR>
+__device__ __forceinline__ void unit_y(const float* y, int n, double (&yd)[NR]) {
+  const int lane = threadIdx.x & 31;
+  double yn = 0;
+#pragma unroll
+  for (int t = 0; t < NR; ++t) {
+    yd[t] = lane + 32 * t < n ? (double)y[lane + 32 * t] : 0.0;
+    yn += yd[t] * yd[t];
+  }
+  yn = 1.0 / sqrt(warp_sum(yn));
+#pragma unroll
+  for (int t = 0; t < NR; ++t) yd[t] *= yn;
+}
+
+// x - yd (yd . x): the projector P.
+template <int NR> __device__ __forceinline__ void project(const double (&yd)[NR], double2 (&x)[NR]) {
+  double2 pr = make_double2(0, 0);
+#pragma unroll
+  for (int t = 0; t < NR; ++t) {
+    pr.x += yd[t] * x[t].x;
+    pr.y += yd[t] * x[t].y;
+  }
+  pr.x = warp_sum(pr.x);
+  pr.y = warp_sum(pr.y);
+#pragma unroll
+  for (int t = 0; t < NR; ++t) {
+    x[t].x -= yd[t] * pr.x;
+    x[t].y -= yd[t] * pr.y;
+  }
+}
+
+template <int NR>
+__global__ void __launch_bounds__(32 * kRefineWarps, NR <= 2 ? 5 : 4) refine_residual_kernel(
+    const float2* __restrict__ coh, PointSet pts, int n, unsigned char* __restrict__ ws) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double2* sv = reinterpret_cast<double2*>(smem_raw) + 3 * n * wid;
+  double2* sd = sv + 2 * n;  // the rows' phases, out of the registers' way
+  const int64_t npairs = (int64_t)n * (n - 1) / 2;
+  const int64_t npt = pts.size();
+  for (int64_t pt = (int64_t)blockIdx.x * kRefineWarps + wid; pt < npt; pt += (int64_t)gridDim.x * kRefineWarps) {
+    const PointPtr<float, double> w(ws, pt, n);
+    float2 z[NR];  // v = Q D y
+    {
+      double2 dph[NR];
+      double yd[NR];
+      row_phases<double>(w, n, dph);
+      unit_y(w.y, n, yd);
+#pragma unroll
+      for (int t = 0; t < NR; ++t) {
+        if (lane + 32 * t < n) sd[lane + 32 * t] = dph[t];
+        z[t] = make_float2((float)(dph[t].x * yd[t]), (float)(dph[t].y * yd[t]));
+      }
+    }
+    double2 v[NR], mv[NR];
+    apply_q(w, n, z, false);
+#pragma unroll
+    for (int t = 0; t < NR; ++t) {
+      v[t] = make_double2(z[t].x, z[t].y);
+      if (lane + 32 * t < n) w.v[lane + 32 * t] = v[t];
+    }
+    herm_matvec(w.ainv, coh + pts[pt] * npairs, n, v, sv, sv + n, mv);
+    double lam;
+    residual(v, mv, lam);
+#pragma unroll
+    for (int t = 0; t < NR; ++t) z[t] = make_float2((float)mv[t].x, (float)mv[t].y);
+    apply_q(w, n, z, true);
+#pragma unroll
+    for (int t = 0; t < NR; ++t)  // D^H: times conj(delta_i)
+      mv[t] = lane + 32 * t < n ? cmulc(make_double2(z[t].x, z[t].y), sd[lane + 32 * t]) : make_double2(0, 0);
+    double yd[NR];
+    unit_y(w.y, n, yd);
+    project(yd, mv);
+#pragma unroll
+    for (int t = 0; t < NR; ++t)
+      if (lane + 32 * t < n) w.x[lane + 32 * t] = mv[t];
+    if (lane == 0) *w.lam = lam;
+    __syncwarp();
+  }
+}
+
+// x <- (R - lambda I)^-1 x of each point, one thread per point: kSolvePoints points per warp, their
+// vectors in shared memory.
+constexpr int kSolvePoints = 16;
+inline size_t solve_smem(int n) { return (size_t)n * (kSolvePoints + 1) * (3 * sizeof(double) + sizeof(double2)); }
+
+constexpr int kSolveThreads = 128;  // to fetch and store; kSolvePoints of them solve
+
+__global__ void __launch_bounds__(kSolveThreads) refine_solve_kernel(PointSet pts, int n, unsigned char* __restrict__ ws) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int P = kSolvePoints, S = P + 1;
+  double2* x0 = reinterpret_cast<double2*>(smem_raw);
+  double* s0 = reinterpret_cast<double*>(x0 + n * S);
+  const int tid = threadIdx.x;
+  const int64_t npt = pts.size();
+  for (int64_t base = (int64_t)blockIdx.x * P; base < npt; base += (int64_t)gridDim.x * P) {
+    const int here = (int)(npt - base < P ? npt - base : P);
+#pragma unroll 4
+    for (int f = tid; f < here * n; f += kSolveThreads) {
+      const int q = f / n, i = f - q * n;
+      const PointPtr<float, double> w(ws, base + q, n);
+      x0[i * S + q] = w.x[i];
+      s0[i * S + q] = (double)w.d[i];
+      const float2 e = w.e[min(i, n - 2)];
+      const double ex = e.x, ey = e.y;
+      s0[(n + i) * S + q] = sqrt(ex * ex + ey * ey);  // entry n - 1 is not used
+    }
+    __syncthreads();
+    if (tid < here) {
+      const PointPtr<float, double> w(ws, base + tid, n);
+      const double tiny = DBL_EPSILON * (double)w.scal[1] + DBL_MIN;
+      // row i of d and b is read before the elimination overwrites it with its reciprocal pivot and
+      // super-diagonal
+      const double *d = s0 + tid, *b = s0 + n * S + tid;
+      tridiag_solve<double>([&](int i) { return d[i * S]; }, [&](int i) { return b[i * S]; }, n, *w.lam, tiny, 1.0,
+                            Strided<double2>{x0 + tid, S}, Strided<double>{s0 + tid, S},
+                            Strided<double>{s0 + n * S + tid, S}, Strided<double>{s0 + 2 * n * S + tid, S});
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int f = tid; f < here * n; f += kSolveThreads) {
+      const int q = f / n, i = f - q * n;
+      const PointPtr<float, double> w(ws, base + q, n);
+      w.x[i] = x0[i * S + q];
+    }
+    __syncthreads();
+  }
+}
+
+template <int NR>
+__global__ void __launch_bounds__(32 * kRefineWarps, 5) refine_check_kernel(
+    const float2* __restrict__ coh, PointSet pts, int n, int ref, unsigned char* __restrict__ ws,
+    uint8_t* __restrict__ sing, float2* __restrict__ ph, float* __restrict__ quality, float* __restrict__ tcoh,
+    double tol) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double2* sv = reinterpret_cast<double2*>(smem_raw) + 2 * n * wid;
+  const int64_t npairs = (int64_t)n * (n - 1) / 2;
+  const int64_t npt = pts.size();
+  for (int64_t pt = (int64_t)blockIdx.x * kRefineWarps + wid; pt < npt; pt += (int64_t)gridDim.x * kRefineWarps) {
+    const int64_t gp = pts[pt];
+    const PointPtr<float, double> w(ws, pt, n);
+    const float2* c = coh + gp * npairs;
+    double2 v[NR], x[NR], dph[NR];
+    double yd[NR];
+    row_phases<double>(w, n, dph);
+    unit_y(w.y, n, yd);
+#pragma unroll
+    for (int t = 0; t < NR; ++t) {
+      const int i = lane + 32 * t;
+      x[t] = i < n ? w.x[i] : make_double2(0, 0);
+      v[t] = i < n ? w.v[i] : make_double2(0, 0);
+    }
+    project(yd, x);
+    float2 z[NR];
+#pragma unroll
+    for (int t = 0; t < NR; ++t) {
+      const double2 q = cmul(x[t], dph[t]);
+      z[t] = make_float2((float)q.x, (float)q.y);
+    }
+    apply_q(w, n, z, false);
+    double vn = 0;
+#pragma unroll
+    for (int t = 0; t < NR; ++t) {
+      v[t] = make_double2(v[t].x - (double)z[t].x, v[t].y - (double)z[t].y);
+      vn += v[t].x * v[t].x + v[t].y * v[t].y;
+    }
+    vn = 1.0 / sqrt(warp_sum(vn));
+#pragma unroll
+    for (int t = 0; t < NR; ++t) v[t] = make_double2(v[t].x * vn, v[t].y * vn);
+    double2 mv[NR];
+    herm_matvec(w.ainv, c, n, v, sv, sv + n, mv);
+    double lam;
+    const double rn = residual(v, mv, lam);
     // phase error bound of the refined vector (v has unit length)
     double vmin = 1e300;
-    for (int i = lane; i < n; i += 32) vmin = fmin(vmin, sqrt(v[i].x * v[i].x + v[i].y * v[i].y));
+#pragma unroll
+    for (int t = 0; t < NR; ++t)
+      if (lane + 32 * t < n) vmin = fmin(vmin, sqrt(v[t].x * v[t].x + v[t].y * v[t].y));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) vmin = fmin(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
     // |r'| / (gap min|v_i|) <= tol with gap = lambda_2(R) - lam - margin holds exactly when
     // lambda_2(R) >= sig = lam + margin + |r'| / (tol min|v_i|): one Sturm count at sig
     // (rounded up to FP32) answers it, without locating lambda_2
+    const float eps = Lim<float>::eps(), tnorm = w.scal[1];
+    const float pivmin = fmaxf(Lim<float>::tiny(), eps * eps * tnorm * tnorm) + Lim<float>::tiny();
     const double sig = lam + 4.0 * (double)eps * (double)n * (double)tnorm + rn / (tol * vmin);
-    for (int i = lane; i + 1 < n; i += 32) b2[i] = b[i] * b[i];  // b2 was the solves' scratch
+    float* d = reinterpret_cast<float*>(sv);
+    float* b2 = d + n;
+    for (int i = lane; i < n; i += 32) {
+      d[i] = w.d[i];
+      if (i + 1 < n) {
+        const double ex = w.e[i].x, ey = w.e[i].y;
+        const float b = (float)sqrt(ex * ex + ey * ey);
+        b2[i] = b * b;
+      }
+    }
     __syncwarp();
     float sg = (float)sig;
     if ((double)sg < sig) sg = nextafterf(sg, 3.4e38f);
-    const bool gap_ok = sig < 3.0e38 && sturm_count(d, b2, n, (T)sg, pivmin) <= 1;  // NaN: false
+    const bool gap_ok = sig < 3.0e38 && sturm_count(d, b2, n, sg, pivmin) <= 1;  // NaN: false
     const bool singular = (sing[pt] & kRouteSingular) != 0;
     const bool small_pivot = (sing[pt] & kRouteCond) != 0;  // the sweep's inverse is not trusted
     const bool ok = singular || (!small_pivot && gap_ok);
-    // normalise to the reference image
-    const double2 zr = v[ref];
-    for (int i = lane; i < n; i += 32) {
-      const double2 q = cmulc(v[i], zr);
-      const double a = sqrt(q.x * q.x + q.y * q.y);
-      float2 o = make_float2((float)(q.x / a), (float)(q.y / a));
-      if (singular) o = make_float2(fnan, fnan);
-      ph[gp * n + i] = o;
-      t1[i] = make_double2(o.x, o.y);
-    }
     __syncwarp();
+    write_phases(v, n, ref, singular, ph + gp * n, sv);
     if (lane == 0) {
-      quality[gp] = singular ? fnan : (float)lam;
+      quality[gp] = singular ? __int_as_float(0x7fffffff) : (float)lam;
       sing[pt] = singular ? kRouteSingular : (ok ? 0 : kRouteCond);
     }
-    if (tcoh) {  // |sum_q coh_q/|coh_q| conj(ph_m) ph_j| / n_pairs
-      double tx = 0, ty = 0;
-      int mm = 0, jj = 1 + lane;
-      while (jj >= n && mm < n - 1) { mm += 1; jj = jj - n + mm + 1; }
-      for (int64_t q = lane; q < npairs; q += 32) {
-        const int m0 = mm, j0 = jj;
-        jj += 32;
-        while (jj >= n && mm < n - 1) { mm += 1; jj = jj - n + mm + 1; }
-        const float2 g = c[q];
-        const double ga = sqrt((double)g.x * g.x + (double)g.y * g.y);
-        const double2 q2 = cmul(make_double2(g.x / ga, g.y / ga), cmulc(t1[j0], t1[m0]));
-        tx += q2.x;
-        ty += q2.y;
-      }
-      tx = warp_sum(tx);
-      ty = warp_sum(ty);
-      if (lane == 0) tcoh[gp] = (float)(sqrt(tx * tx + ty * ty) / (double)npairs);
+    if (tcoh) {
+      const float t = temp_coh_of(c, sv, n);
+      if (lane == 0) tcoh[gp] = t;
     }
     __syncwarp();
   }
@@ -1731,16 +1805,37 @@ int run_big_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, void
 // One pass of the three kernels over a sub-batch (pts.list == nullptr: all pts.n_pc points;
 // else the listed ones, whose count is read on the device), inverse and reduction both in
 // T. cond_max > 0 flags the points whose condition estimate exceeds it.
-template <typename T, int NR, int W>
+// Eigenpair of each point's tridiagonal.
+template <typename T, typename TA, int G>
+int launch_tri_eig(PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
+  const size_t smem = eig_smem<T>(n, G);
+  auto kernel = tri_eig_kernel<T, TA, G>;
+  if (int rc = allow_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
+  const int occ = std::max(1, occupancy(kernel, kEigThreads, smem));
+  const int64_t ctas = (pts.n_pc + kEigThreads / G - 1) / (kEigThreads / G);
+  kernel<<<(unsigned)std::min<int64_t>(ctas, (int64_t)sm_count() * occ), kEigThreads, smem, s>>>(pts, n, ws);
+  return check_launch("emi eigenpair");
+}
+
+template <typename T, typename TA>
+int run_tri_eig(PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
+  // Lanes per point by the arithmetic alone: another number of sections moves the last bits of the
+  // eigenvalue, and a point's result does not depend on the batch that it is in. FP32: 8 rounds of 8
+  // cheap counts; FP64: 13 rounds of 16, whose divisions make each round long.
+  return launch_tri_eig<T, TA, sizeof(T) == 4 ? 8 : 16>(pts, n, ws, s);
+}
+
+template <typename T, int NR>
 int launch_tail(const float2* c, PointSet pts, int n, int ref, float2* ph, float* quality, float* tcoh,
-                const unsigned char* ws, const uint8_t* sing, cudaStream_t s) {
-  const size_t tsmem = W * tail_warp_bytes<T>(n);
-  auto kernel = tail_kernel<T, T, NR, W>;
-  if (int rc_ = allow_smem(reinterpret_cast<const void*>(kernel), tsmem)) return rc_;
-  const int tocc = std::max(1, occupancy(kernel, 32 * W, tsmem));
-  const int64_t tgrid = std::min<int64_t>((pts.n_pc + W - 1) / W, (int64_t)sm_count() * tocc);
+                unsigned char* ws, const uint8_t* sing, cudaStream_t s) {
   KernelTimer kt(pts.list ? "emi tail rerun" : sizeof(T) == 8 ? "emi tail fp64" : "emi tail fp32", s);
-  kernel<<<(unsigned)tgrid, 32 * W, tsmem, s>>>(c, pts, n, ref, ws, sing, ph, quality, tcoh);
+  if (int rc = run_tri_eig<T, T>(pts, n, ws, s)) return rc;
+  const size_t tsmem = kTailWarps * (size_t)n * sizeof(double2);
+  auto kernel = tail_kernel<T, T, NR>;
+  if (int rc = allow_smem(reinterpret_cast<const void*>(kernel), tsmem)) return rc;
+  const int tocc = std::max(1, occupancy(kernel, 32 * kTailWarps, tsmem));
+  const int64_t tgrid = std::min<int64_t>((pts.n_pc + kTailWarps - 1) / kTailWarps, (int64_t)sm_count() * tocc);
+  kernel<<<(unsigned)tgrid, 32 * kTailWarps, tsmem, s>>>(c, pts, n, ref, ws, sing, ph, quality, tcoh);
   return check_launch("emi tail");
 }
 
@@ -1751,14 +1846,15 @@ int run_pass(const float2* c, PointSet pts, int n, int ref, float2* ph, float* q
     if (n > kMaxFastN) {
       if (int rc = run_big_inverse(c, pts, n, ws, sing, slices, s)) return rc;
       if (int rc = run_big_reduce(c, pts, n, ws, slices, s)) return rc;
-      return n <= 160   ? launch_tail<T, 5, 4>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s)
-             : n <= 256 ? launch_tail<T, 8, 4>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s)
-                        : launch_tail<T, 16, 4>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s);
+      return n <= 256 ? launch_tail<T, 8>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s)
+                      : launch_tail<T, 16>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s);
     }
   }
   if (int rc = run_inverse<T, T>(c, pts, n, ws, sing, cond_max, s)) return rc;
   if (int rc = run_reduce<T, T>(c, pts, n, ws, s)) return rc;
-  return launch_tail<T, 4, kTailWarps>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s);
+  return n <= 32   ? launch_tail<T, 1>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s)
+         : n <= 64 ? launch_tail<T, 2>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s)
+                   : launch_tail<T, 4>(c, pts, n, ref, ph, quality, tcoh, ws, sing, s);
 }
 
 template <int NB>
@@ -1782,6 +1878,29 @@ int run_sweep(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t* 
   }
 }
 
+template <int NR>
+int launch_refine(const float2* c, PointSet pts, int n, int ref, float2* ph, float* quality, float* tcoh,
+                  unsigned char* ws, uint8_t* sing, double tol, cudaStream_t s) {
+  KernelTimer kt("emi refine tail", s);
+  if (int rc = run_tri_eig<float, double>(pts, n, ws, s)) return rc;
+  const size_t wsmem = kRefineWarps * 3 * (size_t)n * sizeof(double2), ssmem = solve_smem(n);
+  auto ka = refine_residual_kernel<NR>;
+  auto kb = refine_check_kernel<NR>;
+  if (int rc = allow_smem(reinterpret_cast<const void*>(ka), wsmem)) return rc;
+  if (int rc = allow_smem(reinterpret_cast<const void*>(kb), wsmem)) return rc;
+  if (int rc = allow_smem(reinterpret_cast<const void*>(refine_solve_kernel), ssmem)) return rc;
+  auto grid = [&](auto kernel, int threads, size_t smem, int points) {
+    const int occ = std::max(1, occupancy(kernel, threads, smem));
+    return (unsigned)std::min<int64_t>((pts.n_pc + points - 1) / points, (int64_t)sm_count() * occ);
+  };
+  ka<<<grid(ka, 32 * kRefineWarps, wsmem, kRefineWarps), 32 * kRefineWarps, wsmem, s>>>(c, pts, n, ws);
+  refine_solve_kernel<<<grid(refine_solve_kernel, kSolveThreads, ssmem, kSolvePoints), kSolveThreads, ssmem, s>>>(
+      pts, n, ws);
+  kb<<<grid(kb, 32 * kRefineWarps, wsmem, kRefineWarps), 32 * kRefineWarps, wsmem, s>>>(c, pts, n, ref, ws, sing, ph,
+                                                                                       quality, tcoh, tol);
+  return check_launch("emi refine tail", 3);
+}
+
 // The refined pass: FP64 inverse (symmetric sweep), FP32 reduction, FP64-refined tail;
 // sing[] ends with the points whose sweep met a small pivot or whose refined error bound
 // exceeds `tol` flagged kRouteCond.
@@ -1789,14 +1908,9 @@ int run_refine_pass(const float2* c, PointSet pts, int n, int ref, float2* ph, f
                     unsigned char* ws, uint8_t* sing, double tol, cudaStream_t s) {
   if (int rc = run_sweep(c, pts, n, ws, sing, s)) return rc;
   if (int rc = run_reduce<float, double>(c, pts, n, ws, s)) return rc;
-  const size_t tsmem = kRefineWarps * refine_warp_bytes(n);
-  if (int rc_ = allow_smem(reinterpret_cast<const void*>(tail_refine_kernel<float>), tsmem)) return rc_;
-  const int tocc = std::max(1, occupancy(tail_refine_kernel<float>, 32 * kRefineWarps, tsmem));
-  const int64_t tgrid = std::min<int64_t>((pts.n_pc + kRefineWarps - 1) / kRefineWarps, (int64_t)sm_count() * tocc);
-  KernelTimer kt("emi refine tail", s);
-  tail_refine_kernel<float><<<(unsigned)tgrid, 32 * kRefineWarps, tsmem, s>>>(c, pts, n, ref, ws, sing, ph,
-                                                                                quality, tcoh, tol);
-  return check_launch("emi refine tail");
+  return n <= 32   ? launch_refine<1>(c, pts, n, ref, ph, quality, tcoh, ws, sing, tol, s)
+         : n <= 64 ? launch_refine<2>(c, pts, n, ref, ph, quality, tcoh, ws, sing, tol, s)
+                   : launch_refine<4>(c, pts, n, ref, ph, quality, tcoh, ws, sing, tol, s);
 }
 
 size_t point_bytes_max(int n) {
