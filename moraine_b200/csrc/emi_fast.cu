@@ -368,9 +368,17 @@ struct PointSet {
   __device__ __forceinline__ int64_t operator[](int64_t i) const { return list ? (int64_t)list[off + i] : i; }
 };
 
+// CTAs per SM that the registers are cut to: left alone the unrolled steps take up to 254 registers
+// and one CTA waits out its pivot chain alone. 4,000 points, one CTA (natural) against this: FP64,
+// N = 64 1.5 and 0.70 ms, N = 100 3.46 and 2.89, where the spills of a third CTA cost more than it
+// gives, as those of a second do above 112; FP32, N = 64 two, three and four CTAs 0.71, 0.57, 0.51.
+template <typename T, int NB> constexpr int gj_ctas() {
+  return sizeof(T) == 4 ? (NB <= 7 ? 4 : 3) : NB <= 3 ? 5 : NB == 4 ? 4 : NB == 5 ? 3 : NB <= 7 ? 2 : 1;
+}
+
 // TW: arithmetic of the reduction that reads the workspace (the point stride depends on it).
 template <typename T, int NB, int CX, typename TW>
-__global__ void __launch_bounds__(16 * CX, 1) inverse_kernel(const float2* __restrict__ coh, PointSet pts, int n,
+__global__ void __launch_bounds__(16 * CX, gj_ctas<T, NB>()) inverse_kernel(const float2* __restrict__ coh, PointSet pts, int n,
                                                           unsigned char* __restrict__ ws, uint8_t* __restrict__ sing,
                                                           float cond_max) {
   constexpr int NC = GjGrid<NB, CX>::NC;
@@ -408,6 +416,84 @@ __global__ void __launch_bounds__(16 * CX, 1) inverse_kernel(const float2* __res
     }
     if (tid == 0) sing[pt] = flag;
     __syncthreads();
+  }
+}
+
+// ----------------------------------------------------------------- kernel 1a: inverse, N <= 32
+// The same Gauss-Jordan with one warp per point: lane i holds row i in registers (the padding is
+// identity and never pivots), the pivot is a warp argmax over the lanes' entries of column k, and the
+// pivot row goes to all lanes by shuffles. No barrier, and as many points per SM as it has warps:
+// on the 16 x 16 grid a 17 x 17 matrix used 289 of the CTA's 1,024 entries and waited for a
+// barrier per step. FP64, N = 17, 1,003 points: 23 us against 42.
+constexpr int kWarpInvWarps = 4;
+
+template <typename T, int NM, typename TW>
+__global__ void __launch_bounds__(32 * kWarpInvWarps) warp_inverse_kernel(const float2* __restrict__ coh, PointSet pts,
+                                                                          int n, unsigned char* __restrict__ ws,
+                                                                          uint8_t* __restrict__ sing, float cond_max) {
+  const int lane = threadIdx.x & 31;
+  const int64_t npairs = (int64_t)n * (n - 1) / 2;
+  const int64_t npt = pts.size();
+  for (int64_t pt = (int64_t)blockIdx.x * kWarpInvWarps + (threadIdx.x >> 5); pt < npt;
+       pt += (int64_t)gridDim.x * kWarpInvWarps) {
+    const float2* c = coh + pts[pt] * npairs;
+    T a[NM];
+#pragma unroll
+    for (int j = 0; j < NM; ++j) {
+      float2 g = make_float2(lane == j ? 1.f : 0.f, 0.f);
+      if (lane < n && j < n && lane != j) g = c[lane < j ? triu_index(lane, j, n) : triu_index(j, lane, n)];
+      a[j] = (T)sqrt((double)g.x * g.x + (double)g.y * g.y);
+    }
+    auto norm = [&]() {  // max over the rows of the sum of |a_ij|
+      T r = 0;
+#pragma unroll
+      for (int j = 0; j < NM; ++j)
+        if (j < n) r += fabs(a[j]);
+      if (lane >= n) r = 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
+      return r;
+    };
+    const T anorm = cond_max > 0.f ? norm() : T(0);
+    bool used = lane >= n, singular = false;
+    int step = 0;       // of this row
+    int piv_mine = 0;   // lane k: pivot row of step k
+#pragma unroll
+    for (int k = 0; k < NM; ++k) {
+      if (k >= n) break;
+      T best = used ? T(-1) : fabs(a[k]) == fabs(a[k]) ? fabs(a[k]) : T(-0.5);  // NaN ranks last but is taken
+      int p = used ? 32 : lane;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const T ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, p, o);
+        if (ob > best || (ob == best && oi < p)) { best = ob; p = oi; }
+      }
+      T pv = __shfl_sync(0xffffffffu, a[k], p);
+      if (pv == T(0)) { singular = true; pv = T(1); }
+      const T rp = recip(pv);
+      const bool is_p = lane == p;
+      if (is_p) { used = true; step = k; }
+      if (lane == k) piv_mine = p;
+      // a -= f r everywhere, with f_p = pv - 1 so that the pivot row becomes r
+      const T fi = a[k], f = is_p ? pv - T(1) : fi;
+#pragma unroll
+      for (int j = 0; j < NM; ++j) a[j] -= f * (__shfl_sync(0xffffffffu, a[j], p) * rp);
+      a[k] = is_p ? rp : -fi * rp;
+    }
+    uint8_t flag = singular ? kRouteSingular : 0;
+    if (cond_max > 0.f && !singular) {
+      const T cond = anorm * norm();
+      if (!(cond <= (T)cond_max)) flag = kRouteCond;
+    }
+    T* out = PointPtr<TW, T>(ws, pt, n).ainv;
+#pragma unroll
+    for (int j = 0; j < NM; ++j) {  // row `step` of the inverse; column j belongs to pivot row j's step
+      if (j >= n) break;
+      const int pc = __shfl_sync(0xffffffffu, piv_mine, j);
+      if (lane < n && step >= pc) out[tri_up(pc, step, n)] = a[j];  // inv[step][pc], kept once
+    }
+    if (lane == 0) sing[pt] = flag;
   }
 }
 
@@ -1692,8 +1778,8 @@ __global__ void route_kernel(const uint8_t* __restrict__ sing, int64_t nb, int64
 }
 
 // Column groups of the Gauss-Jordan grid. 32 groups (512 threads, half the registers per
-// thread) measured no faster than 16 in FP32 or FP64: one point per SM either way, and its
-// serial pivot steps set the pace. With look-ahead pivoting the 512-thread tile stayed in
+// thread) measured no faster than 16 in FP32 or FP64 with one point per SM, whose serial pivot
+// steps set the pace. With look-ahead pivoting the 512-thread tile stayed in
 // local memory (128 registers per thread), twice as slow.
 template <typename T>
 constexpr int gj_cx() { return 16; }
@@ -1710,6 +1796,18 @@ int launch_inverse(const float2* coh, PointSet pts, int64_t grid_cap, int n, uns
 }
 
 // inv(|Gamma|) in arithmetic TA into a workspace laid out for a reduction in T.
+template <typename T, int NM, typename TW>
+int launch_warp_inverse(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t* sing, float cond_max,
+                        cudaStream_t s) {
+  auto kernel = warp_inverse_kernel<T, NM, TW>;
+  const int occ = std::max(1, occupancy(kernel, 32 * kWarpInvWarps, 0));
+  const int64_t ctas = (pts.n_pc + kWarpInvWarps - 1) / kWarpInvWarps;
+  KernelTimer kt(pts.list ? "emi inverse rerun" : sizeof(T) == 8 ? "emi inverse fp64" : "emi inverse fp32", s);
+  kernel<<<(unsigned)std::min<int64_t>(ctas, (int64_t)sm_count() * occ), 32 * kWarpInvWarps, 0, s>>>(c, pts, n, ws,
+                                                                                                    sing, cond_max);
+  return check_launch("emi inverse");
+}
+
 // Most images with the reduction's FP64 triangle in shared memory.
 constexpr int kReduceIn = 158;
 
@@ -1745,7 +1843,9 @@ int run_inverse(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t
                 cudaStream_t s) {
   const int64_t cap = pts.n_pc;  // grid bound: the most points this pass can see
   switch ((n + 15) / 16) {
-    case 1: case 2: return launch_inverse<TA, 2, T>(c, pts, cap, n, ws, sing, cond_max, s);
+    case 1: return launch_warp_inverse<TA, 16, T>(c, pts, n, ws, sing, cond_max, s);
+    case 2: return n <= 24 ? launch_warp_inverse<TA, 24, T>(c, pts, n, ws, sing, cond_max, s)
+                           : launch_warp_inverse<TA, 32, T>(c, pts, n, ws, sing, cond_max, s);
     case 3: return launch_inverse<TA, 3, T>(c, pts, cap, n, ws, sing, cond_max, s);
     case 4: return launch_inverse<TA, 4, T>(c, pts, cap, n, ws, sing, cond_max, s);
     case 5: return launch_inverse<TA, 5, T>(c, pts, cap, n, ws, sing, cond_max, s);
