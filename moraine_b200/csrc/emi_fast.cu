@@ -829,20 +829,21 @@ __global__ void __launch_bounds__(256, 2) sweep_kernel(const float2* __restrict_
 // separate passes over M): FP32, N = 17, 2,047 points 146 us, now 37; N = 50, 35,627 points 8.4 ms,
 // now 3.4; N = 100, 286,294 points 199 ms, now 178; FP64, N = 17, 1,003 points 157 us, now 38; N = 100,
 // 4,001 points 6.2 ms, now 5.8.
-// Shared memory: the triangle, 16 entries that reads past the end of its last row may touch, (u, w)
-// of step k-1 and u_k with kRowPad entries in front (rows above the first of a strip), and each
-// warp's part of M u.
+// The vectors of a step, one record per row: kRowPad zero records in front (rows above the first of a
+// strip) and kColPad behind (columns past the last). u, w: of step k-1; c: u_k.
 constexpr int kRowPad = 8, kColPad = 16;
+template <typename C> struct Rec {
+  C u, w, c;
+};
+
+// Shared memory: the step's records, each warp's part of M u, and the triangle with kColPad entries
+// that reads past the end of its last row may touch.
 __host__ __device__ inline size_t reduce_tri(int n) { return (size_t)n * (n + 1) / 2 + kColPad; }
 template <typename T>
 __host__ __device__ inline size_t reduce_smem(int n, int warps, bool tri_in) {
-  return ((tri_in ? reduce_tri(n) : 0) + 3 * (size_t)(n + kRowPad + kColPad) + (size_t)warps * n) *
-         sizeof(typename C2<T>::type);
+  return (n + kRowPad + kColPad) * sizeof(Rec<typename C2<T>::type>) +
+         ((tri_in ? reduce_tri(n) : 0) + (size_t)warps * n) * sizeof(typename C2<T>::type);
 }
-
-template <typename C> struct alignas(2 * sizeof(C)) Pair {
-  C u, w;
-};
 
 template <typename T, typename TA, int QC, int R, int W, bool kTriIn = true>
 __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
@@ -853,20 +854,14 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, lc = lane & 15, wid = tid >> 5;
   constexpr int nw = W;
-  Pair<C>* uw = reinterpret_cast<Pair<C>*>(smem_raw) + kRowPad;  // u_{k-1}, w_{k-1}
-  C* uc = reinterpret_cast<C*>(uw + n + kColPad) + kRowPad;      // u_k
-  C* part = uc + n + kColPad;                                    // [warps][n]: each warp's part of M u
+  Rec<C>* rec = reinterpret_cast<Rec<C>*>(smem_raw) + kRowPad;
+  C* part = reinterpret_cast<C*>(rec + n + kColPad);  // [warps][n]: each warp's part of M u
   C* L = kTriIn ? part + nw * n : slices + blockIdx.x * reduce_tri(n);
   const int64_t npairs = (int64_t)n * (n - 1) / 2;
   const int64_t npt = pts.size();
-  for (int e = tid; e < kRowPad; e += blockDim.x) {
-    uw[-1 - e] = {mk<T>(0, 0), mk<T>(0, 0)};
-    uc[-1 - e] = mk<T>(0, 0);
-  }
-  for (int e = tid; e < kColPad; e += blockDim.x) {
-    uw[n + e] = {mk<T>(0, 0), mk<T>(0, 0)};
-    uc[n + e] = mk<T>(0, 0);
-    L[tri(n) + e] = mk<T>(0, 0);
+  for (int e = tid; e < kRowPad + kColPad; e += blockDim.x) {
+    rec[e < kRowPad ? -1 - e : n + e - kRowPad] = {mk<T>(0, 0), mk<T>(0, 0), mk<T>(0, 0)};
+    if (e < kColPad) L[tri(n) + e] = mk<T>(0, 0);
   }
   for (int64_t pt = blockIdx.x; pt < npt; pt += gridDim.x) {
     const float2* c = coh + pts[pt] * npairs;
@@ -908,10 +903,10 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
           const int i = lane + 32 * t;
           wr[t].x -= K * u[t].x;
           wr[t].y -= K * u[t].y;
-          if (i < n) uw[i] = {u[t], wr[t]};
+          if (i < n) { rec[i].u = u[t]; rec[i].w = wr[t]; }
         }
         __syncwarp();
-        const Pair<C> at_k = uw[k];
+        const C uk = rec[k].u, wk = rec[k].w;
         C x[Q];
         T xn2 = 0;
 #pragma unroll
@@ -920,7 +915,7 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
           x[t] = mk<T>(0, 0);
           if (i >= k && i < n) {
             x[t] = L[tri(i) + k];
-            rank2(x[t], u[t], at_k.w, wr[t], at_k.u);
+            rank2(x[t], u[t], wk, wr[t], uk);
           }
           if (i >= k + 2) xn2 += x[t].x * x[t].x + x[t].y * x[t].y;
         }
@@ -961,7 +956,7 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
           }
           u[t] = i == k + 1 ? v1 : x[t];
           if (i <= k || tau == T(0)) u[t] = mk<T>(0, 0);
-          if (i < n) uc[i] = u[t];
+          if (i < n) rec[i].c = u[t];
           if (i > k && i < n && k + 2 < n) refl[i] = u[t];
         }
         if (lane == 0) {
@@ -977,16 +972,14 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
       C acc[QC];  // column sums, of columns k + 1 + lc + 16 q
 #pragma unroll
       for (int q = 0; q < QC; ++q) acc[q] = mk<T>(0, 0);
-      const Pair<C>* cuw = uw + (k + 1 + lc);
-      const C* cuc = uc + (k + 1 + lc);
+      const Rec<C>* crec = rec + (k + 1 + lc);
       for (int top = n - 1 - 2 * R * wid; top > k; top -= 2 * R * nw) {
         const int hi = top - R * (lane >> 4);  // this half-warp's strip: rows hi - R + 1 .. hi
-        Pair<C> rv[R];
-        C rc[R], sum[R];
+        Rec<C> rv[R];
+        C sum[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          rv[r] = uw[hi - r];
-          rc[r] = uc[hi - r];
+          rv[r] = rec[hi - r];
           sum[r] = mk<T>(0, 0);
         }
         C* row0 = L + tri(hi) + (k + 1 + lc);
@@ -995,8 +988,7 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
         for (int q = 0; q < QC; ++q) {
           const int j0 = k + 1 + 16 * q;
           if (j0 > top) break;
-          const Pair<C> cv = cuw[16 * q];
-          const C cc = cuc[16 * q];
+          const Rec<C> cv = crec[16 * q];
           if (j0 + 15 < top - (2 * R - 1)) {  // all lanes left of every diagonal of the two strips
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -1004,8 +996,8 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
               C a = *e;
               rank2(a, rv[r].u, cv.w, rv[r].w, cv.u);
               *e = a;
-              cmac(sum[r], a, cc);
-              cmacc(acc[q], a, rc[r]);
+              cmac(sum[r], a, cv.c);
+              cmacc(acc[q], a, rv[r].c);
             }
           } else {
             const int left = hi - (j0 + lc);  // of row hi's diagonal
@@ -1018,8 +1010,8 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
               // half of the diagonal in either part, nothing beyond it
               a.x = left > r ? a.x : left == r ? T(0.5) * a.x : T(0);
               a.y = left > r ? a.y : T(0);
-              cmac(sum[r], a, cc);
-              cmacc(acc[q], a, rc[r]);
+              cmac(sum[r], a, cv.c);
+              cmacc(acc[q], a, rv[r].c);
             }
           }
         }
@@ -1031,10 +1023,10 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
 #pragma unroll
       for (int q = 0; q < QC; ++q) {
         const int j = k + 1 + lc + 16 * q;
-        acc[q] = cadd(acc[q], shfl_xor_c(acc[q], 16));
+        C col = cadd(acc[q], shfl_xor_c(acc[q], 16));
         if (lane < 16 && j < n) {
-          if (((n - 1 - j) / (2 * R)) % nw == wid) acc[q] = cadd(acc[q], mine[j]);  // a row of this warp's strips
-          mine[j] = acc[q];
+          if (((n - 1 - j) / (2 * R)) % nw == wid) col = cadd(col, mine[j]);  // a row of this warp's strips
+          mine[j] = col;
         }
       }
       __syncthreads();
