@@ -827,8 +827,9 @@ __global__ void __launch_bounds__(256, 2) sweep_kernel(const float2* __restrict_
 // divisions) and the short strips of B, hidden only by the other CTAs of the SM. The previous form
 // (256 threads, three barriers, groups of four threads on mirrored row pairs, row and column parts in
 // separate passes over M): FP32, N = 17, 2,047 points 146 us, now 37; N = 50, 35,627 points 8.4 ms,
-// now 3.4; N = 100, 286,294 points 199 ms, now 178; FP64, N = 17, 1,003 points 157 us, now 38; N = 100,
-// 4,001 points 6.2 ms, now 5.8.
+// now 3.5; N = 100, 286,294 points 199 ms, now 164; FP64, N = 17, 1,003 points 157 us, now 38; N = 100,
+// 4,001 points 6.2 ms, now 5.4. FP32 in packed pairs (fma.f32x2 on rows and columns laid out twice)
+// was slower, 204 ms: its sums and doubled vectors cost registers and shared memory.
 // The vectors of a step, one record per row: kRowPad zero records in front (rows above the first of a
 // strip) and kColPad behind (columns past the last). u, w: of step k-1; c: u_k.
 constexpr int kRowPad = 8, kColPad = 16;
@@ -836,13 +837,15 @@ template <typename C> struct Rec {
   C u, w, c;
 };
 
-// Shared memory: the step's records, each warp's part of M u, and the triangle with kColPad entries
-// that reads past the end of its last row may touch.
-__host__ __device__ inline size_t reduce_tri(int n) { return (size_t)n * (n + 1) / 2 + kColPad; }
+// Shared memory: the step's records, each warp's column sums, the row sums, and the triangle.
+// Entries of the triangle and those that reads outside it may touch (their values are dropped): 15 past
+// its last row, and up to entry 31 from the rows above the first of a strip (tri(k - 6) + k + 16).
+constexpr int kTriPad = 32;
+__host__ __device__ inline size_t reduce_tri(int n) { return (size_t)n * (n + 1) / 2 + kTriPad; }
 template <typename T>
 __host__ __device__ inline size_t reduce_smem(int n, int warps, bool tri_in) {
   return (n + kRowPad + kColPad) * sizeof(Rec<typename C2<T>::type>) +
-         ((tri_in ? reduce_tri(n) : 0) + (size_t)warps * n) * sizeof(typename C2<T>::type);
+         ((tri_in ? reduce_tri(n) : 0) + (size_t)(warps + 1) * n) * sizeof(typename C2<T>::type);
 }
 
 template <typename T, typename TA, int QC, int R, int W, bool kTriIn = true>
@@ -855,13 +858,13 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
   const int tid = threadIdx.x, lane = tid & 31, lc = lane & 15, wid = tid >> 5;
   constexpr int nw = W;
   Rec<C>* rec = reinterpret_cast<Rec<C>*>(smem_raw) + kRowPad;
-  C* part = reinterpret_cast<C*>(rec + n + kColPad);  // [warps][n]: each warp's part of M u
-  C* L = kTriIn ? part + nw * n : slices + blockIdx.x * reduce_tri(n);
+  C* part = reinterpret_cast<C*>(rec + n + kColPad);  // [warps][n]: each warp's column sums
+  C* rows = part + nw * n;                             // row sums
+  C* L = kTriIn ? rows + n : slices + blockIdx.x * reduce_tri(n);
   const int64_t npairs = (int64_t)n * (n - 1) / 2;
   const int64_t npt = pts.size();
   for (int e = tid; e < kRowPad + kColPad; e += blockDim.x) {
     rec[e < kRowPad ? -1 - e : n + e - kRowPad] = {mk<T>(0, 0), mk<T>(0, 0), mk<T>(0, 0)};
-    if (e < kColPad) L[tri(n) + e] = mk<T>(0, 0);
   }
   for (int64_t pt = blockIdx.x; pt < npt; pt += gridDim.x) {
     const float2* c = coh + pts[pt] * npairs;
@@ -891,8 +894,9 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
           const int i = lane + 32 * t;
           wr[t] = mk<T>(0, 0);
           if (tau_prev != T(0) && i >= k && i < n) {
-            C p = part[i];
-            for (int q = 1; q < nw; ++q) p = cadd(p, part[q * n + i]);
+            C p = rows[i];
+#pragma unroll
+            for (int q = 0; q < nw; ++q) p = cadd(p, part[q * n + i]);
             wr[t] = mk<T>(tau_prev * p.x, tau_prev * p.y);
             dot += u[t].x * wr[t].x + u[t].y * wr[t].y;
           }
@@ -1017,17 +1021,14 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
         }
         const C tot = half_warp_sum(sum);
         const int i = hi - (lane & 15) / (16 / R);
-        if (lane % (16 / R) == 0 && i > k) mine[i] = tot;
+        if (lane % (16 / R) == 0 && i > k) rows[i] = tot;
       }
-      __syncwarp();
 #pragma unroll
       for (int q = 0; q < QC; ++q) {
-        const int j = k + 1 + lc + 16 * q;
-        C col = cadd(acc[q], shfl_xor_c(acc[q], 16));
-        if (lane < 16 && j < n) {
-          if (((n - 1 - j) / (2 * R)) % nw == wid) col = cadd(col, mine[j]);  // a row of this warp's strips
-          mine[j] = col;
-        }
+        const int j0 = k + 1 + 16 * q;
+        if (j0 >= n) break;
+        const C col = cadd(acc[q], shfl_xor_c(acc[q], 16));
+        if (lane < 16 && j0 + lane < n) mine[j0 + lane] = col;
       }
       __syncthreads();
     }
@@ -1801,7 +1802,7 @@ int launch_warp_inverse(const float2* c, PointSet pts, int n, unsigned char* ws,
 }
 
 // Most images with the reduction's FP64 triangle in shared memory.
-constexpr int kReduceIn = 158;
+constexpr int kReduceIn = 157;
 
 template <int Q, bool kIn>
 int launch_big_inverse(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t* sing, void* slices,
@@ -1864,13 +1865,14 @@ int launch_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, cudaS
 
 template <typename T, typename TA>
 int run_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
-  // Warps per point and rows per half-warp strip. Up to 64 images one warp (FP64: two above 32)
-  // needs no or little waiting on other warps and an SM holds many points; above, shared memory
-  // holds two to four points per SM, and more warps each hide their latencies: N = 100, FP32, 1, 2, 4,
-  // 8 warps of 4 rows: 243, 222, 178, 285 ms for 286,294 points; FP64, 4 and 8 warps of 4 rows 6.5 and
-  // 6.2, of 2 rows (128 registers, two CTAs of 8 warps) 6.4 and 5.8 ms for 4,001 points.
+  // Warps per point and rows per half-warp strip. Up to 64 images one warp needs no waiting on other
+  // warps and an SM holds many points (FP64, N = 50, 4,001 points: one warp 0.78 ms, two 1.02);
+  // above, shared memory holds two to four points per SM, and more warps each hide their latencies:
+  // N = 100, FP32, 1, 2, 4, 8 warps of 4 rows: 243, 222, 178, 285 ms for 286,294 points; FP64, 4 and 8
+  // warps of 4 rows 6.5 and 6.2, of 2 rows (128 registers, two CTAs of 8 warps) 6.4 and 5.8 ms for
+  // 4,001 points.
   constexpr bool f64 = sizeof(T) == 8;
-  constexpr int W4 = f64 ? 2 : 1, W8 = f64 ? 8 : 4, R8 = f64 ? 2 : 4;
+  constexpr int W4 = 1, W8 = f64 ? 8 : 4, R8 = f64 ? 2 : 4;
   switch ((n + 15) / 16) {
     case 1: return launch_reduce<T, TA, 1, 4, 1>(c, pts, n, ws, s);
     case 2: return launch_reduce<T, TA, 2, 4, 1>(c, pts, n, ws, s);

@@ -167,8 +167,28 @@ def test_temp_coh_all_pairs_shapes(cuda, n):
 
 
 # ----------------------------------------------------------------------------- EMI
+@pytest.mark.parametrize("rows", [2, 4])
+def test_reduction_reads_stay_inside(rows):
+    """Every read of the reduction's strips (rows above the first active one and columns past the
+    edge included) lies inside the triangle and its 32 spare entries, and inside the padded
+    records of the step."""
+    def tri(i):
+        return i * (i + 1) // 2
+    for n in (*range(3, 40), 64, 100, 128, 158, 512):
+        for k in range(n - 2):
+            tops = range(k + 1, n) if n < 40 else {k + 1, k + 2, k + 5, min(k + 17, n - 1), n - 1}
+            for top in (t for t in tops if k < t < n):
+                for hi in (top, top - rows):
+                    blocks = (top - (k + 1)) // 16
+                    assert k + 1 + 16 * blocks + 15 < n + 16
+                    for r in range(rows):
+                        row = tri(hi) - (r * hi - r * (r - 1) // 2)
+                        assert -8 <= hi - r < n and row == tri(hi - r)
+                        assert 0 <= row + k + 1 and row + k + 16 + 16 * blocks < tri(n) + 32
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [2, 3, 15, 16, 17, 32, 33, 48, 49, 64, 65, 80, 97, 113, 128, 129, 144, 145, 158, 159,
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 6, 15, 16, 17, 32, 33, 48, 49, 64, 65, 80, 97, 113, 128, 129, 144, 145, 157, 158, 159,
                                160, 161, 192, 193, 257])
 def test_emi_block_shapes(cuda, n):
     """EMI at the edges of its kernels' tiles, warps and matrix placements against LAPACK FP64; a
