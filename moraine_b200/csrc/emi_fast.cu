@@ -1717,7 +1717,9 @@ int occupancy(K kernel, int threads, size_t smem) {
 template <typename T>
 int64_t sub_batch(int n) {
   const PointWs<T> w(n);  // FP64 sub-batches also fit the refined layout (it is smaller)
-  const int64_t def = (int64_t)std::max<size_t>(1024, std::min<size_t>(1 << 17, (size_t)(1ull << 32) / (w.bytes + 1)));
+  // above 128 images 2 GiB: a wave of one point per SM is enough there
+  const size_t most = n > kMaxFastN ? (size_t)1 << 31 : (size_t)1 << 32, least = n > kMaxFastN ? 296 : 1024;
+  const int64_t def = (int64_t)std::max<size_t>(least, std::min<size_t>(1 << 17, most / (w.bytes + 1)));
   const int64_t cap = g_sub_batch_cap.load();
   return cap > 0 ? std::min(cap, def) : def;
 }
