@@ -159,11 +159,11 @@ EMI_TRAFFIC_PER_POINT = {(100, "fp64"): 356_500, (100, "fp32"): 239_900}
 # scene model (profiles/*_c2_512.md); the traffic of these kernels scales with the units, so a
 # full-size launch gets units x bytes. Keyed by (kernel, N); DS points, pixels for the KS merge.
 KERNEL_TRAFFIC_PER_UNIT = {
-    ("emi reduce fp32", 100): (2.768748e9 + 1.384547e9) / 34_510,   # prof512_reduce_f32c
-    ("emi refine tail", 100): (10.324045e9 + 31.297536e6) / 34_510,  # prof512_tail_refine_c
-    ("emi sweep fp64", 100): (1.368710e9 + 1.348463e9) / 34_510,     # prof512_sweep2
-    ("gram fp64", 100): (1.502556e9 + 2.682337e9) / 69_019,          # prof512_gram_b
-    ("ks merge", 100): (109.437696e6 + 38.131456e6) / 262_144,       # prof512_ks_kept
+    ("emi reduce fp32", 100): (2.774624e9 + 1.388484e9) / 34_510,
+    ("emi refine tail", 100): (11.547766e9 + 366.030e6) / 34_510,  # its four kernels
+    ("emi sweep fp64", 100): (1.368710e9 + 1.348463e9) / 34_510,
+    ("gram fp64", 100): (1.447099e9 + 2.684820e9) / 69_019,
+    ("ks merge", 100): (110.203648e6 + 38.718720e6) / 262_144,
 }
 
 
@@ -196,7 +196,8 @@ def stage_rooflines(cfg, stage: dict, n_ds: int, res, peaks: dict, fp32: float, 
     """Achieved rate of every stage against the bound that limits it.
 
     Algorithmic work per unit (unit = pixel for the raster stages, DS point for the rest):
-      ks_select   4N + W + 4 bytes per pixel (rmli in, mask and count out), W(2N-1) merge steps
+      ks_select   4N + W + 4 bytes per pixel (rmli in, mask and count out); W(2N-1) steps of the
+                  merge that defines the statistic
       coherence   8 S Q + 3 S N flops per DS point (S = its SHP count, Q = N(N-1)/2)
       emi_tcoh    2.7 N^3 + 80 N^2 flops per DS point (Cholesky + inverse of |Gamma|, complex
                   factorisation of M, inverse-iteration solves)
@@ -210,7 +211,7 @@ def stage_rooflines(cfg, stage: dict, n_ds: int, res, peaks: dict, fp32: float, 
         ms = stage["ks_select"] + stage.get("intensity", 0.0)
         byts = npix * (4 * n + cfg.az_win * cfg.r_win + 4) + npix * n * 12
         gbs = byts / (ms / 1e3) / 1e9
-        out["ks_select"] = {"kernel": "intensity_kernel + sort_keys_kernel + ks_merge_kernel", "bound": "hbm",
+        out["ks_select"] = {"kernel": "intensity_kernel + sort_keys_kernel + ks_select_kernel", "bound": "hbm",
                             "achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm, "traffic": None,
                             "ms": ms, "merge_steps_per_s": npix * cfg.az_win * cfg.r_win * (2 * n - 1) / (ms / 1e3),
                             "peak_source": peaks["source"]}
@@ -223,7 +224,8 @@ def stage_rooflines(cfg, stage: dict, n_ds: int, res, peaks: dict, fp32: float, 
         tc = precision in ("bf16", "bf16x3")
         g64 = precision == "fp64"
         peak = peaks.get("bf16_tflops") if tc else (fp32 / 2 if g64 else fp32)
-        out["coherence"] = {"kernel": "gram_tc_kernel" if tc else "gram_kernel", "bound": "tensor" if tc else
+        out["coherence"] = {"kernel": "gram_tc_kernel" if tc else
+                            ("gram64_kernel" if g64 and n <= 104 else "gram_kernel"), "bound": "tensor" if tc else
                             ("fp64-simt" if g64 else "fp32-simt"), "achieved": tf, "peak": peak, "unit": "TFLOP/s",
                             "frac": tf / peak, "traffic": None, "ms": ms,
                             "peak_source": peaks["source"] + " bf16" if tc else
@@ -236,7 +238,7 @@ def stage_rooflines(cfg, stage: dict, n_ds: int, res, peaks: dict, fp32: float, 
         tpp = EMI_TRAFFIC_PER_POINT.get((n, chain.emi_precision))
         f64 = chain.emi_precision == "fp64" or n > 128
         peak = fp32 / 2 if f64 else fp32  # the FP64 pipe of B200 runs at half the FP32 rate
-        out["emi_tcoh"] = {"kernel": "mr_emi: inverse_kernel + reduce_kernel + tail_kernel", "bound":
+        out["emi_tcoh"] = {"kernel": "mr_emi: inverse or sweep, reduce_kernel, tri_eig_kernel, tail or refine kernels", "bound":
                            "fp64-simt" if f64 else "fp32-simt",
                            "achieved": tf, "peak": peak, "unit": "TFLOP/s", "frac": tf / peak,
                            "traffic": tpp * n_ds / calls if tpp else None, "ms": ms,
@@ -253,8 +255,8 @@ def kernel_rooflines(cfg, ktimes: dict, n_ds: int, res, peaks: dict, fp32: float
     per unit, and the bound:
       ks sort keys      pixel: 4N bytes in, 4K out (K = keys per pixel)          HBM
       ks merge          pixel: 4N + W + 4 bytes (keys in, mask and count out)     HBM (as asked;
-                        its real limit is shared memory: the bank conflicts of its
-                        data-dependent merge reads, W(2N-1) merge steps per pixel)
+                        its real limit is shared-memory bandwidth, W 2(N - k_th + 1)
+                        compares per pixel; W(2N-1) steps is the merge it stands for)
       gram fp32/fp64    DS point: 8 S Q + 3 S N flops (S its SHP count)          FP32 / FP64 pipe
       emi inverse/sweep DS point: N^3/3 + N^3 flops (factorisation and inverse of |Gamma|)
       emi reduce        DS point: 4N^3/3 flops (the complex factorisation of M)
