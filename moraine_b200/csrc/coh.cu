@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kMaxGramThreads, sizeof(A) == 8 ? 2 : 3) gram_
 // points of 166 SHPs at N = 150).
 // N = 100, 11 x 21 window, 20,000 points: 5.2 ms against 6.4 (one CTA of 256 threads, samples
 // widened at each use) and 5.5 with gram_kernel<double>; N = 64 1.9 against 3.3 and 2.8; N = 50,
-// 35,627 points: 2.5 against 4.6; N = 17, 2,047 points: 47 against 126 us. The exact sums |z|^2 and the
+// 35,627 points: 2.5 against 4.6. The exact sums |z|^2 and the
 // rounding test of `normalised` are 0.4 ms of the 5.2: without them a few coherences in 10^8 round
 // to the other float, which the EMI of a nearly singular point magnifies to milliradians.
 constexpr int kGramWarps = 4;
@@ -541,13 +541,23 @@ GramPlan cut_gram64(int n, int cap) {
   return plan;
 }
 
-// The cut into at most kGramWarps runs with the least warp time (warps times the longest run), short
-// runs where two are equal. n <= kDmmaImages always has one (runs of 13).
-GramPlan plan_gram64(int n) {
+// The cut into at most kGramWarps runs whose longest run is the shortest: the least time for a
+// point, and the more room for CTAs. n <= kDmmaImages always has one (runs of 13). Up to 24 images
+// one warp can hold all blocks of a point; it wastes no step on an idle warp, but a point takes
+// longer, so it is taken where every SM has more than 32 points (11 x 21 window, 20,000 points: N =
+// 17 438 against 550 us, N = 24 448 against 567; 5,000 points 152 against 153 and 156 against 155;
+// 2,000 points of a 15 x 31 window, N = 24: 165 against 114). One warp or few long runs above 24
+// images lost at every size: N = 32 (one run of 6 against three of 2), 200 points 167 against 75 us,
+// 20,000 points 701 against 663; N = 72 (three runs of 10 against four of up to 8), 200 points 220
+// against 162 us, 20,000 points 3.95 against 2.40 ms.
+constexpr int kOneWarpImages = 24;
+
+GramPlan plan_gram64(int n, bool many) {
+  if (n <= kOneWarpImages && many) return cut_gram64(n, 4);
   GramPlan best{};
-  for (int cap = 4; cap <= 13; ++cap) {
+  for (int cap = 1; cap <= 13; ++cap) {
     const GramPlan p = cut_gram64(n, cap);
-    if (p.runs <= kGramWarps && (!best.runs || p.warps * p.slots < best.warps * best.slots)) best = p;
+    if (p.runs <= kGramWarps && (!best.runs || p.slots < best.slots)) best = p;
   }
   return best;
 }
@@ -625,7 +635,7 @@ int launch_gram64(const float2* rslc, int nlines, int width, int n, const int32_
     return launch_gram<double, false>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win, r_win, coh,
                                       nullptr, s, dcount, doff);
   const int nr = (n + 15) / 16;
-  const GramPlan plan = plan_gram64(n);
+  const GramPlan plan = plan_gram64(n, n_pc > (int64_t)sm_count() * 32);
   const int threads = 32 * plan.warps;
   const int kc = plan.warps == 1 ? 8 : 16;  // one-warp CTAs stage fewer rows, so that more of them fit an SM
   const size_t smem = (size_t)kc * ((16 * nr + 4) * sizeof(double2) + n * sizeof(float2)) + 32 * nr * sizeof(double) +

@@ -123,6 +123,23 @@ def test_coherence_block_shapes(cuda, n):
         np.testing.assert_array_equal(coh, np.conj(np.swapaxes(coh, -1, -2)))
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 8, 9, 16, 17, 24, 25, 32, 33, 40, 41, 56, 57, 65, 72, 73, 81, 97, 104])
+def test_coherence_does_not_depend_on_the_batch(cuda, n):
+    """A few points (blocks of images spread over the warps) and enough of them to fill the device
+    several times over: the same floats."""
+    rng = np.random.default_rng(n)
+    nl, w, azw, rw = 13, 17, 9, 11
+    z = (rng.normal(size=(nl, w, n)) + 1j * rng.normal(size=(nl, w, n))).astype(np.complex64)
+    idx = np.stack([rng.integers(0, nl, 23), rng.integers(0, w, 23)], 1).astype(np.int32)
+    mask = rng.random((23, azw, rw)) < 0.6
+    mask[:, azw // 2, rw // 2] = True
+    few = mb.emperical_co_pc(z, idx, mask, precision="fp64")
+    np.testing.assert_allclose(few, O.emperical_co_pc(z, idx, mask), atol=1e-7, rtol=0)
+    many = mb.emperical_co_pc(z, np.tile(idx, (300, 1)), np.tile(mask, (300, 1, 1)), precision="fp64")
+    np.testing.assert_array_equal(many, np.tile(few, (300, 1)))
+
+
 # ----------------------------------------------------------------------------- streaming statistics
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 16, 17, 32, 33, 64, 65, 129, 300])
