@@ -821,9 +821,10 @@ __global__ void __launch_bounds__(256, 2) sweep_kernel(const float2* __restrict_
 //      lanes, and the columns' sums of conj(M_ij) u_i, which stay in the lane that owns column j
 //      (lanes run along columns k + 1 + lane % 16 + 16 q) until the warp is through its strips.
 // Every element is read and written once per step and a row's vectors are read once per strip;
-// partial sums are added in a fixed order, so results do not depend on timing. Blocks of 16 columns
-// that meet the diagonal run unmasked over the next rows' entries, keep what is theirs and count half
-// of the diagonal in either part. Bound by latency: the chain of A (two warp sums, roots and
+// partial sums are added in a fixed order, so results do not depend on timing. In blocks of 16 columns
+// that meet the diagonal a lane reads and writes only entries of its own row (what lies past the
+// diagonal belongs to the next row, and to another half-warp) and counts half of the diagonal in
+// either part. Bound by latency: the chain of A (two warp sums, roots and
 // divisions) and the short strips of B, hidden only by the other CTAs of the SM. The previous form
 // (256 threads, three barriers, groups of four threads on mirrored row pairs, row and column parts in
 // separate passes over M): FP32, N = 17, 2,047 points 146 us, now 37; N = 50, 35,627 points 8.4 ms,
@@ -838,10 +839,7 @@ template <typename C> struct Rec {
 };
 
 // Shared memory: the step's records, each warp's column sums, the row sums, and the triangle.
-// Entries of the triangle and those that reads outside it may touch (their values are dropped): 15 past
-// its last row, and up to entry 31 from the rows above the first of a strip (tri(k - 6) + k + 16).
-constexpr int kTriPad = 32;
-__host__ __device__ inline size_t reduce_tri(int n) { return (size_t)n * (n + 1) / 2 + kTriPad; }
+__host__ __device__ inline size_t reduce_tri(int n) { return (size_t)n * (n + 1) / 2; }
 template <typename T>
 __host__ __device__ inline size_t reduce_smem(int n, int warps, bool tri_in) {
   return (n + kRowPad + kColPad) * sizeof(Rec<typename C2<T>::type>) +
@@ -1008,9 +1006,10 @@ __global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
 #pragma unroll
             for (int r = 0; r < R; ++r) {
               C* e = row0 - (r * hi - r * (r - 1) / 2) + 16 * q;
-              C a = *e;  // past the diagonal: the next row's, not kept
+              const bool own = left >= r;  // else the next row's entry, which its own half-warp may be writing
+              C a = own ? *e : mk<T>(0, 0);
               rank2(a, rv[r].u, cv.w, rv[r].w, cv.u);
-              if (left >= r) *e = a;
+              if (own) *e = a;
               // half of the diagonal in either part, nothing beyond it
               a.x = left > r ? a.x : left == r ? T(0.5) * a.x : T(0);
               a.y = left > r ? a.y : T(0);

@@ -1,5 +1,8 @@
 """Kernels and dispatch rules at the sizes where they can go wrong: host emulations of their
 index logic (CPU), and the device against the oracle or the general path (GPU)."""
+import re
+from pathlib import Path
+
 import numpy as np
 import pytest
 import torch
@@ -236,3 +239,42 @@ def test_emi_block_shapes(cuda, n):
     if n > 128:
         _, _, route = mb.emi(coh, ref=ref, precision="refine", return_route=True)
         assert (route == 1).all()
+
+
+# ----------------------------------------------------------------------------- EMI: ownership, memory
+def _emi_source():
+    return (Path(mb.__file__).parent / "csrc" / "emi_fast.cu").read_text()
+
+
+def test_reduction_entries_have_one_owner():
+    """The reduction's walk with the constants of its source: in every step each entry of the
+    trailing triangle is read and written by one lane, no lane touches another's (blocks that meet
+    the diagonal included), and every record read exists."""
+    src = _emi_source()
+    row_pad, col_pad = (int(re.search(rf"\b{name} = (\d+)", src).group(1)) for name in ("kRowPad", "kColPad"))
+    guarded = re.search(r"const bool own = left >= r;[^\n]*\n\s*C a = own \? \*e :", src) is not None
+    shapes = {int(r) for r in re.findall(r"launch_reduce<double, double, \d+, (\d+), \d+", src)} | {2, 4}
+    lc = np.arange(16)
+    for rows in sorted(shapes):
+        for n in (*range(2, 44), 63, 64, 65, 97, 108, 112, 113, 128, 157, 158, 161, 512):
+            for k in range(n - 2) if n < 44 else (0, 1, 2, 15, 16, 17, n // 2, n - 20, n - 4, n - 3):
+                seen = np.zeros((n, n), int)
+                for top in range(n - 1, k, -2 * rows):
+                    for hi in (top, top - rows):
+                        assert hi - rows + 1 >= -row_pad
+                        for j0 in range(k + 1, top + 1, 16):
+                            assert j0 + 15 < n + col_pad
+                            for i in range(hi, hi - rows, -1):
+                                if j0 + 15 < top - (2 * rows - 1):
+                                    assert i > j0 + 15  # all of the block left of the diagonal
+                                    seen[i, j0:j0 + 16] += 1
+                                    continue
+                                own = j0 + lc <= i
+                                touched = own if guarded else np.ones(16, bool)
+                                assert not (touched & ~own).any(), "an entry of another row is read"
+                                if own.any():
+                                    assert i > k
+                                    seen[i, (j0 + lc)[own]] += 1
+                trail = np.arange(n) > k
+                want = np.tril(np.ones((n, n), int)) * trail[:, None] * trail[None, :]
+                assert np.array_equal(seen, want)
