@@ -847,7 +847,7 @@ __host__ __device__ inline size_t reduce_smem(int n, int warps, bool tri_in) {
 }
 
 template <typename T, typename TA, int QC, int R, int W, bool kTriIn = true>
-__global__ void __launch_bounds__(32 * W, W >= 4 && QC <= 8 ? 16 / W : 1)
+__global__ void __launch_bounds__(32 * W, W >= 3 && QC <= 8 ? (sizeof(T) == 8 ? 2 : 16 / W) : 1)
     reduce_kernel(const float2* __restrict__ coh, PointSet pts, int n, unsigned char* __restrict__ ws,
                   typename C2<T>::type* __restrict__ slices) {
   using C = typename C2<T>::type;
@@ -1881,7 +1881,18 @@ int run_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, cudaStre
     case 4: return launch_reduce<T, TA, 4, 4, W4>(c, pts, n, ws, s);
     case 5: return launch_reduce<T, TA, 5, R8, W8>(c, pts, n, ws, s);
     case 6: return launch_reduce<T, TA, 6, R8, W8>(c, pts, n, ws, s);
-    case 7: return launch_reduce<T, TA, 7, R8, W8>(c, pts, n, ws, s);
+    case 7:
+      if constexpr (f64) {
+        // The most warps with which two CTAs fit an SM's 228 KB (1 KB of each CTA is reserved): 8 up to
+        // 107 images, 6 up to 109, 4 up to 111, 3 at 112. One CTA of 8 warps against these, 3,000
+        // points: N = 108 7.44 and 4.46 ms, N = 110 (4 warps) 7.64 and 4.96, N = 112 7.86 and 5.78.
+        auto two_fit = [&](int warps) { return 2 * (reduce_smem<T>(n, warps, true) + 1024) <= 228 * 1024; };
+        if (!two_fit(8))
+          return two_fit(6)   ? launch_reduce<T, TA, 7, 2, 6>(c, pts, n, ws, s)
+                 : two_fit(4) ? launch_reduce<T, TA, 7, 4, 4>(c, pts, n, ws, s)
+                              : launch_reduce<T, TA, 7, 4, 3>(c, pts, n, ws, s);
+      }
+      return launch_reduce<T, TA, 7, R8, W8>(c, pts, n, ws, s);
     default: return launch_reduce<T, TA, 8, R8, W8>(c, pts, n, ws, s);
   }
 }

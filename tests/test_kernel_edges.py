@@ -278,3 +278,9 @@ def test_reduction_entries_have_one_owner():
                 trail = np.arange(n) > k
                 want = np.tril(np.ones((n, n), int)) * trail[:, None] * trail[None, :]
                 assert np.array_equal(seen, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [107, 108, 109, 110, 111, 112])
+def test_emi_where_the_reduction_changes_its_warps(cuda, n):
+    test_emi_block_shapes(cuda, n)
