@@ -225,7 +225,7 @@ def stage_rooflines(cfg, stage: dict, n_ds: int, res, peaks: dict, fp32: float, 
         g64 = precision == "fp64"
         peak = peaks.get("bf16_tflops") if tc else (fp32 / 2 if g64 else fp32)
         out["coherence"] = {"kernel": "gram_tc_kernel" if tc else
-                            ("gram64_kernel" if g64 and n <= 104 else "gram_kernel"), "bound": "tensor" if tc else
+                            ("gram64_kernel" if g64 and n <= 128 and not 56 < n <= 60 else "gram_kernel"), "bound": "tensor" if tc else
                             ("fp64-simt" if g64 else "fp32-simt"), "achieved": tf, "peak": peak, "unit": "TFLOP/s",
                             "frac": tf / peak, "traffic": None, "ms": ms,
                             "peak_source": peaks["source"] + " bf16" if tc else

@@ -341,17 +341,14 @@ __global__ void __launch_bounds__(kMaxGramThreads, sizeof(A) == 8 ? 2 : 3) gram_
 // read once or twice per step and its other addresses are a base and a constant (nothing issues
 // beside a DMMA, so every instruction counts: with a next-block rule per slot it took 5.9 ms
 // below, on m8n8k4 7.9 ms). Four warps of 13 blocks hold 104 images in one pass over the SHPs,
-// two such CTAs per SM; smaller runs leave room for more CTAs. Above that the accumulators
-// need several passes, which measured slower than gram_kernel<double> (6.4 against 5.2 ms for 5,224
-// points of 166 SHPs at N = 150).
+// two such CTAs per SM, eight of 9 hold 128; smaller runs leave room for more warps (plan_gram64).
 // N = 100, 11 x 21 window, 20,000 points: 5.2 ms against 6.4 (one CTA of 256 threads, samples
 // widened at each use) and 5.5 with gram_kernel<double>; N = 64 1.9 against 3.3 and 2.8; N = 50,
 // 35,627 points: 2.5 against 4.6. The exact sums |z|^2 and the
 // rounding test of `normalised` are 0.4 ms of the 5.2: without them a few coherences in 10^8 round
 // to the other float, which the EMI of a nearly singular point magnifies to milliradians.
-constexpr int kGramWarps = 4;
 constexpr int kMaxRuns = 8;
-constexpr int kDmmaImages = 104;
+constexpr int kDmmaImages = 128;
 
 // Run r: blocks (br1, bc1 ...) c1 of them, then (br2, bc2 ...) up to cnt.
 struct GramRun {
@@ -369,8 +366,13 @@ __device__ __forceinline__ void dmma(double (&d)[4], const double (&a)[4], const
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-template <int SLOTS>
-__global__ void __launch_bounds__(32 * kGramWarps, SLOTS <= 4 ? 4 : SLOTS <= 7 ? 3 : 2) gram64_kernel(
+// CTAs per SM that the registers are cut to, of `warps` warps with `slots` blocks of accumulators each.
+constexpr int gram64_ctas(int slots, int warps) {
+  return warps == 4 ? (slots <= 4 ? 4 : slots <= 7 ? 3 : 2) : warps * slots <= 42 ? 2 : 1;
+}
+
+template <int SLOTS, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, gram64_ctas(SLOTS, WARPS)) gram64_kernel(
     const float2* __restrict__ rslc, int nlines, int width, int n, const int32_t* __restrict__ idx,
     int64_t n_pc, const uint8_t* __restrict__ mask, int mask_stride, int az_win, int r_win,
     float2* __restrict__ coh, const int64_t* __restrict__ dcount, int64_t doff, int kc,
@@ -541,25 +543,72 @@ GramPlan cut_gram64(int n, int cap) {
   return plan;
 }
 
-// The cut into at most kGramWarps runs whose longest run is the shortest: the least time for a
-// point, and the more room for CTAs. n <= kDmmaImages always has one (runs of 13). Up to 24 images
-// one warp can hold all blocks of a point; it wastes no step on an idle warp, but a point takes
-// longer, so it is taken where every SM has more than 32 points (11 x 21 window, 20,000 points: N =
-// 17 438 against 550 us, N = 24 448 against 567; 5,000 points 152 against 153 and 156 against 155;
-// 2,000 points of a 15 x 31 window, N = 24: 165 against 114). One warp or few long runs above 24
-// images lost at every size: N = 32 (one run of 6 against three of 2), 200 points 167 against 75 us,
-// 20,000 points 701 against 663; N = 72 (three runs of 10 against four of up to 8), 200 points 220
-// against 162 us, 20,000 points 3.95 against 2.40 ms.
+// The cut for n images into at most `warps` runs of at most `most` blocks whose longest run is the
+// shortest (runs = 0: there is none).
+GramPlan fit_gram64(int n, int warps, int most) {
+  const int nc = (n + 7) / 8, nr = (n + 15) / 16, blocks = nr * nc - nr * (nr - 1);
+  for (int cap = (blocks + warps - 1) / warps; cap <= most; ++cap) {
+    const GramPlan p = cut_gram64(n, cap);
+    if (p.runs <= warps) return p;
+  }
+  return {};
+}
+
+// A CTA's shape: its warps and the accumulator blocks that each may hold. The first shape that the
+// images fit is taken, in an order by warps resident per SM (16, 12 or 8, by registers) and by how
+// evenly the blocks fill the runs. Times of 4,000 points, 11 x 21 window, in us, with four warps, with
+// gram_kernel<double>, and as dispatched:
+//   up to 72 images  four warps of up to 7    N = 64: 364, 499, 364 (six warps 424, eight 403)
+//   up to 80         eight warps of 4         N = 76: 682, 507, 493
+//   up to 96         six warps of 6 or 7      N = 84: 791, 759, 617;  N = 96: 846, 897, 689
+//   up to 104        four warps of 13         N = 104: 945, 978, 945 (eight warps of 7: 1,023)
+//   up to 128        eight warps of 7 to 9    N = 112: -, 1,242, 1,022;  N = 124: -, 1,366, 1,265
+// From 129 to 144 images eight warps of 11 or 12 blocks lose as often as they win (4,000 points, N = 132
+// 1,750 against 1,502 us with gram_kernel, N = 144 1,809 against 1,885); above, the accumulators need
+// several passes over the SHPs (N = 150, 5,224 points of 166 SHPs: 6.4 against 5.2 ms).
+// 57 to 60 images, padded to 64 here, fill 120 of 128 threads of gram_kernel: N = 60 327 against 361 us.
+// 105 to 108, padded to 112, fill 378 of its 384: N = 105 992 against 1,018 us, but 900 points 269
+// against 253 us: there with more than 16 points per SM.
+// Few points, at most two per SM, end sooner with more warps each whatever the images (200 points,
+// 11 x 21 window, N = 64 58 against 62 us, N = 104 98 against 108; with six per SM that lost: N = 64,
+// 900 points 118 against 111).
+// Up to 24 images one warp can hold all blocks of a point; it wastes no step on an idle warp, but a
+// point takes longer, so it is taken where every SM has more than 32 points (11 x 21 window, 20,000
+// points: N = 17 438 against 550 us, N = 24 448 against 567; 5,000 points 152 against 153 and 156
+// against 155; 2,000 points of a 15 x 31 window, N = 24: 165 against 114).
 constexpr int kOneWarpImages = 24;
 
-GramPlan plan_gram64(int n, bool many) {
-  if (n <= kOneWarpImages && many) return cut_gram64(n, 4);
-  GramPlan best{};
-  for (int cap = 1; cap <= 13; ++cap) {
-    const GramPlan p = cut_gram64(n, cap);
-    if (p.runs <= kGramWarps && (!best.runs || p.slots < best.slots)) best = p;
-  }
-  return best;
+struct GramShape {
+  int warps, slots;
+};
+constexpr GramShape kManyPoints[] = {{4, 7}, {8, 4}, {6, 7}, {4, 13}, {8, 9}};
+constexpr GramShape kFewPoints[] = {{8, 4}, {6, 7}, {8, 9}};
+
+// The plan, and in `shape` the CTA shape of the kernel that holds it.
+GramPlan plan_gram64(int n, int64_t n_pc, int sms, GramShape& shape) {
+  shape = {4, 4};
+  if (n <= kOneWarpImages && n_pc > (int64_t)sms * 32) return cut_gram64(n, 4);
+  GramPlan plan{};
+  auto first = [&](const auto& shapes) {
+    for (const GramShape& s : shapes) {
+      plan = fit_gram64(n, s.warps, s.slots);
+      if (plan.runs) {
+        if (plan.runs > 4) shape = s;
+        else shape = {4, plan.slots};
+        return;
+      }
+    }
+  };
+  if (n_pc <= (int64_t)sms * 2) first(kFewPoints);
+  else first(kManyPoints);
+  return plan;
+}
+
+// Whether gram64_kernel takes n images.
+bool dmma_images(int n, int64_t n_pc, int sms) {
+  if (n > 56 && n <= 60) return false;
+  if (n > 104 && n <= 108 && n_pc > (int64_t)sms * 16) return false;
+  return n <= kDmmaImages;
 }
 
 // Arbitrary pair lists: one thread per (point, pair), serial over the window.
@@ -631,11 +680,13 @@ int launch_gram(const float2* rslc, int nlines, int width, int n, const int32_t*
 int launch_gram64(const float2* rslc, int nlines, int width, int n, const int32_t* idx, int64_t n_pc,
                   const uint8_t* mask, int mask_stride, int az_win, int r_win, float2* coh, cudaStream_t s,
                   const int64_t* dcount = nullptr, int64_t doff = 0) {
-  if (n > kDmmaImages)
+  const int sms = sm_count();
+  if (!dmma_images(n, n_pc, sms))
     return launch_gram<double, false>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win, r_win, coh,
                                       nullptr, s, dcount, doff);
   const int nr = (n + 15) / 16;
-  const GramPlan plan = plan_gram64(n, n_pc > (int64_t)sm_count() * 32);
+  GramShape shape;
+  const GramPlan plan = plan_gram64(n, n_pc, sms, shape);
   const int threads = 32 * plan.warps;
   const int kc = plan.warps == 1 ? 8 : 16;  // one-warp CTAs stage fewer rows, so that more of them fit an SM
   const size_t smem = (size_t)kc * ((16 * nr + 4) * sizeof(double2) + n * sizeof(float2)) + 32 * nr * sizeof(double) +
@@ -647,7 +698,10 @@ int launch_gram64(const float2* rslc, int nlines, int width, int n, const int32_
         rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win, r_win, coh, dcount, doff, kc, plan);
     return check_launch("coherence gram");
   };
-  return plan.slots <= 4 ? go(gram64_kernel<4>) : plan.slots <= 7 ? go(gram64_kernel<7>) : go(gram64_kernel<13>);
+  if (shape.warps == 6) return go(gram64_kernel<7, 6>);
+  if (shape.warps == 8)
+    return plan.slots <= 4 ? go(gram64_kernel<4, 8>) : plan.slots <= 7 ? go(gram64_kernel<7, 8>) : go(gram64_kernel<9, 8>);
+  return plan.slots <= 4 ? go(gram64_kernel<4, 4>) : plan.slots <= 7 ? go(gram64_kernel<7, 4>) : go(gram64_kernel<13, 4>);
 }
 
 }  // namespace

@@ -1,5 +1,6 @@
 """Kernels and dispatch rules at the sizes where they can go wrong: host emulations of their
 index logic (CPU), and the device against the oracle or the general path (GPU)."""
+import math
 import re
 from pathlib import Path
 
@@ -284,3 +285,70 @@ def test_reduction_entries_have_one_owner():
 @pytest.mark.parametrize("n", [107, 108, 109, 110, 111, 112])
 def test_emi_where_the_reduction_changes_its_warps(cuda, n):
     test_emi_block_shapes(cuda, n)
+
+
+# ----------------------------------------------------------------------------- FP64 Gram: one set of floats
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [16, 41, 56, 57, 60, 61, 64, 72, 73, 80, 81, 88, 89, 96, 97, 104, 105, 112, 113, 120, 121, 128])
+def test_fp64_gram_is_the_same_on_every_path(cuda, n):
+    """A few points, enough of them for the other CTA shapes, and the same images inside a stack too
+    long for the tensor instruction: the same floats."""
+    rng = np.random.default_rng(n)
+    nl, w, azw, rw = 13, 17, 9, 11
+    z = (rng.normal(size=(nl, w, 145)) + 1j * rng.normal(size=(nl, w, 145))).astype(np.complex64)
+    idx = np.stack([rng.integers(0, nl, 23), rng.integers(0, w, 23)], 1).astype(np.int32)
+    mask = rng.random((23, azw, rw)) < 0.6
+    mask[:, azw // 2, rw // 2] = True
+    few = mb.emperical_co_pc(np.ascontiguousarray(z[..., :n]), idx, mask, precision="fp64")
+    np.testing.assert_allclose(few, O.emperical_co_pc(np.ascontiguousarray(z[..., :n]), idx, mask), atol=1e-7, rtol=0)
+    many = mb.emperical_co_pc(np.ascontiguousarray(z[..., :n]), np.tile(idx, (30, 1)), np.tile(mask, (30, 1, 1)),
+                              precision="fp64")
+    np.testing.assert_array_equal(many, np.tile(few, (30, 1)))
+    m, j = np.triu_indices(145, 1)
+    inside = j < n
+    wide = mb.emperical_co_pc(z, idx, mask, precision="fp64")
+    np.testing.assert_array_equal(wide[:, inside], few)
+
+
+def _integers_of_square_sum(total, k, rng):
+    """k integers whose squares add up to total."""
+    while True:
+        a = rng.integers(-900, 900, k - 4)
+        rest = total - int((a * a).sum())
+        for _ in range(200):
+            b = rng.integers(0, int(rest ** 0.5), 2)
+            left = rest - int((b * b).sum())
+            for c in range(int(max(left, 0) ** 0.5), 0, -1):
+                d = math.isqrt(left - c * c)
+                if d * d == left - c * c:
+                    return np.concatenate([a, b, [c, d]])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [9, 60, 100, 128, 145])
+def test_fp64_gram_rounds_like_the_quotient(cuda, n):
+    """Integer samples with sums of squares 2^25: every sum is exact, and many quotients lie exactly
+    between two floats, where a product with a rounded reciprocal root would fall to either side."""
+    rng = np.random.default_rng(n)
+    looks, total = 16, 2 ** 25
+    base = _integers_of_square_sum(total, 2 * looks, rng)
+    rows = []
+    for _ in range(n):
+        r = base.copy()
+        a, b = rng.choice(2 * looks, 2, replace=False)
+        r[[a, b]] = r[[b, a]]
+        rows.append(r)
+    x = np.array(rows).reshape(n, looks, 2)
+    zi = x[..., 0] + 1j * x[..., 1]                       # (n, looks)
+    num = zi @ zi.conj().T
+    m, j = np.triu_indices(n, 1)
+    num = num[m, j]
+    f = (1.0 / np.sqrt(float(total))) ** 2
+    product, quotient = (num.real * f).astype(np.float32), (num.real / total).astype(np.float32)
+    assert (product != quotient).sum() > len(m) // 10     # the inputs tell the two apart
+    z = np.zeros((5, 5, n), np.complex64)
+    z.reshape(25, n)[:looks] = zi.T
+    mask = (np.arange(25) < looks).reshape(1, 5, 5)
+    got = mb.emperical_co_pc(z, np.array([[2, 2]], np.int32), mask, precision="fp64")[0]
+    np.testing.assert_array_equal(got.real, quotient)
+    np.testing.assert_array_equal(got.imag, (num.imag / total).astype(np.float32))
