@@ -104,7 +104,13 @@ __device__ __forceinline__ void copy8(float2* dst, const float2* src) {
 // each, take as long as their 64 FP64 FMAs). FP32, N = 50, 15 x 31 window, 30,011 points: 1.65 ms
 // against 2.9 with a separate pass for |z|^2 and 256-thread CTAs; N = 20 raster of 123 x 131: 0.16
 // against 0.38 ms. FP64 at N = 150, 8,000 points of 95 SHPs: 4.7 against 5.0 ms.
-constexpr int kMaxGramThreads = 192;
+//
+// A CTA has up to 192 threads, or up to 256 (fewer of them per SM) where that takes a round less: FP32
+// at any number of points (N = 80, 4,000 points, 11 x 21 window: 444 against 331 us; N = 112 735 and
+// 620; N = 200 2,129 and 1,736; with the same rounds at N = 68 the 256 lost, 74 against 76 % of the
+// time of the kernel before), FP64 with at most two points per SM (N = 152, 200 points: 210 against
+// 184 us; but 4,000 points 1,999 against 2,172).
+constexpr int kGramThreads = 192, kWideGramThreads = 256;
 
 template <typename A> struct GramAcc;
 template <> struct GramAcc<float> {
@@ -157,8 +163,8 @@ __device__ __forceinline__ void load_block(const double2* row, int nb, int b, do
   for (int r = 0; r < 4; ++r) z[r] = row[r * nb + b];
 }
 
-template <typename A, bool kFull>
-__global__ void __launch_bounds__(kMaxGramThreads, sizeof(A) == 8 ? 2 : 3) gram_kernel(
+template <typename A, bool kFull, int MT>
+__global__ void __launch_bounds__(MT, (sizeof(A) == 8 ? 2 : 3) - (MT == kWideGramThreads)) gram_kernel(
     const float2* __restrict__ rslc, int nlines, int width, int n, const int32_t* __restrict__ idx,
     int64_t n_pc, const uint8_t* __restrict__ mask, int mask_stride, int az_win, int r_win,
     float2* __restrict__ coh, float2* __restrict__ cov, const int64_t* __restrict__ dcount, int64_t doff, int kc) {
@@ -657,24 +663,38 @@ unsigned gram_grid(K kernel, int threads, size_t smem, int64_t n_pc) {
   return (unsigned)std::min<int64_t>(n_pc, (int64_t)sm_count() * occ * 8);
 }
 
-template <typename A, bool kFull>
-int launch_gram(const float2* rslc, int nlines, int width, int n, const int32_t* idx, int64_t n_pc,
-                const uint8_t* mask, int mask_stride, int az_win, int r_win, float2* coh, float2* cov,
-                cudaStream_t s, const int64_t* dcount = nullptr, int64_t doff = 0) {
+template <typename A, bool kFull, int MT>
+int launch_gram_of(const float2* rslc, int nlines, int width, int n, const int32_t* idx, int64_t n_pc,
+                   const uint8_t* mask, int mask_stride, int az_win, int r_win, float2* coh, float2* cov,
+                   cudaStream_t s, const int64_t* dcount, int64_t doff) {
   using C = typename cplx<A>::type;
   constexpr bool kWide = sizeof(A) == 8;
   const int nb = (n + 3) / 4, nblk = nb * (nb + 1) / 2;
   // no more warps than the blocks fill; all but the last round run full
-  const int threads = std::min(kMaxGramThreads, (nblk + 31) / 32 * 32);
+  const int threads = std::min(MT, (nblk + 31) / 32 * 32);
   const size_t row = (size_t)(kWide ? 1 : 2) * 4 * nb * sizeof(C);
   const int kc = chunk_rows(kWide ? 16 : 32, row);
   const size_t smem = kc * row + (kWide ? ((size_t)kc * n + 1) / 2 * 2 * sizeof(float2) : 0) + (kWide ? 2 : 1) * 4 * nb * sizeof(A) +
                       (size_t)az_win * r_win * sizeof(int);
-  if (int rc = allow_smem(reinterpret_cast<const void*>(gram_kernel<A, kFull>), smem)) return rc;
+  if (int rc = allow_smem(reinterpret_cast<const void*>(gram_kernel<A, kFull, MT>), smem)) return rc;
   KernelTimer kt(kWide ? "gram fp64" : "gram fp32", s);
-  gram_kernel<A, kFull><<<gram_grid(gram_kernel<A, kFull>, threads, smem, n_pc), threads, smem, s>>>(
+  gram_kernel<A, kFull, MT><<<gram_grid(gram_kernel<A, kFull, MT>, threads, smem, n_pc), threads, smem, s>>>(
       rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win, r_win, coh, cov, dcount, doff, kc);
   return check_launch("coherence gram");
+}
+
+template <typename A, bool kFull>
+int launch_gram(const float2* rslc, int nlines, int width, int n, const int32_t* idx, int64_t n_pc,
+                const uint8_t* mask, int mask_stride, int az_win, int r_win, float2* coh, float2* cov,
+                cudaStream_t s, const int64_t* dcount = nullptr, int64_t doff = 0) {
+  const int nb = (n + 3) / 4, nblk = nb * (nb + 1) / 2;
+  auto rounds = [&](int threads) { return (nblk + threads - 1) / threads; };
+  const bool wide = rounds(kWideGramThreads) < rounds(kGramThreads) &&
+                    (sizeof(A) == 4 || n_pc <= (int64_t)sm_count() * 2);
+  return wide ? launch_gram_of<A, kFull, kWideGramThreads>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win,
+                                                           r_win, coh, cov, s, dcount, doff)
+              : launch_gram_of<A, kFull, kGramThreads>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win,
+                                                       r_win, coh, cov, s, dcount, doff);
 }
 
 int launch_gram64(const float2* rslc, int nlines, int width, int n, const int32_t* idx, int64_t n_pc,

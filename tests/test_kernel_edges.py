@@ -352,3 +352,33 @@ def test_fp64_gram_rounds_like_the_quotient(cuda, n):
     got = mb.emperical_co_pc(z, np.array([[2, 2]], np.int32), mask, precision="fp64")[0]
     np.testing.assert_array_equal(got.real, quotient)
     np.testing.assert_array_equal(got.imag, (num.imag / total).astype(np.float32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [76, 80, 88, 89, 109, 124, 136, 152, 174])
+def test_gram_where_the_threads_change(cuda, n):
+    """Where a CTA of more threads saves a round: against the oracle, and FP64 the same floats with
+    few points and with many."""
+    test_coherence_block_shapes(cuda, n)
+    rng = np.random.default_rng(n)
+    z = (rng.normal(size=(9, 11, n)) + 1j * rng.normal(size=(9, 11, n))).astype(np.complex64)
+    idx = np.stack([rng.integers(0, 9, 13), rng.integers(0, 11, 13)], 1).astype(np.int32)
+    mask = rng.random((13, 5, 7)) < 0.6
+    mask[:, 2, 3] = True
+    for precision in ("fp32", "fp64"):
+        few = mb.emperical_co_pc(z, idx, mask, precision=precision)
+        many = mb.emperical_co_pc(z, np.tile(idx, (30, 1)), np.tile(mask, (30, 1, 1)), precision=precision)
+        np.testing.assert_array_equal(many, np.tile(few, (30, 1)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [80, 109])
+def test_raster_where_the_threads_change(cuda, n):
+    rng = np.random.default_rng(n)
+    z = (rng.normal(size=(5, 7, n)) + 1j * rng.normal(size=(5, 7, n))).astype(np.complex64)
+    is_shp = rng.random((5, 7, 5, 7)) < 0.5
+    is_shp[..., 2, 3] = True
+    cov_ref, coh_ref = O.emperical_co(z, is_shp)
+    cov, coh = mb.emperical_co(z, is_shp)
+    np.testing.assert_allclose(coh, coh_ref, atol=2e-6, rtol=0)
+    np.testing.assert_allclose(cov, cov_ref, atol=2e-6 * np.abs(cov_ref).max(), rtol=0)
