@@ -382,3 +382,9 @@ def test_raster_where_the_threads_change(cuda, n):
     cov, coh = mb.emperical_co(z, is_shp)
     np.testing.assert_allclose(coh, coh_ref, atol=2e-6, rtol=0)
     np.testing.assert_allclose(cov, cov_ref, atol=2e-6 * np.abs(cov_ref).max(), rtol=0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [128, 129, 255, 256, 257, 511, 512])
+def test_amp_disp_one_pixel_at_a_time(cuda, n):
+    test_amp_disp_group_shapes(cuda, n)
