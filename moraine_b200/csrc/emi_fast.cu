@@ -290,7 +290,9 @@ template <typename C> __device__ __forceinline__ C half_warp_sum(const C (&r)[4]
 // Per point: inv(|Gamma|) in the arithmetic TA of the inverse, packed upper triangle by
 // rows like the compressed coherence ((m, j >= m) at tri_up(m, j)); then, in the arithmetic
 // T of the reduction, the reflectors (column k rows k+1..n-1, packed by column, nq complex
-// T), d and tau (n T each), e (n complex T).
+// T), d and tau (n T each), e (n complex T). The reduction has all of M in its triangle before it
+// writes the first reflector, so the reflectors take the inverse's place, except where the refined
+// tail reads the inverse again.
 __host__ __device__ __forceinline__ int64_t tri_up(int m, int j, int n) {
   return (int64_t)m * n - ((int64_t)m * (m - 1)) / 2 + (j - m);
 }
@@ -302,11 +304,15 @@ struct PointWs {
     using C = typename C2<T>::type;
     np = (size_t)n * (n + 1) / 2;
     nq = (size_t)n * (n - 1) / 2;
-    bytes = align16(np * sizeof(TA)) + align16(nq * sizeof(C)) + align16(2 * (size_t)n * sizeof(T)) +
+    bytes = (kRefined ? align16(np * sizeof(TA)) + align16(nq * sizeof(C)) : front(np * sizeof(TA), nq * sizeof(C))) +
+            align16(2 * (size_t)n * sizeof(T)) +
             align16((size_t)n * sizeof(C)) + align16(((size_t)n + 2) * sizeof(T)) +
             (kRefined ? (2 * (size_t)n + 1) * sizeof(double2) : 0);
   }
   static constexpr bool kRefined = sizeof(T) == 4 && sizeof(TA) == 8;
+  static __host__ __device__ __forceinline__ size_t front(size_t ainv, size_t refl) {
+    return align16(ainv > refl ? ainv : refl);
+  }
 };
 
 template <typename T, typename TA = T>
@@ -326,9 +332,10 @@ struct PointPtr {
     const PointWs<T, TA> w(n);
     unsigned char* b = ws + (size_t)pt * w.bytes;
     ainv = reinterpret_cast<TA*>(b);
-    b += align16(w.np * sizeof(TA));
+    if (PointWs<T, TA>::kRefined) b += align16(w.np * sizeof(TA));
     refl = reinterpret_cast<C*>(b);
-    b += align16(w.nq * sizeof(C));
+    b += PointWs<T, TA>::kRefined ? align16(w.nq * sizeof(C))
+                                  : PointWs<T, TA>::front(w.np * sizeof(TA), w.nq * sizeof(C));
     d = reinterpret_cast<T*>(b);
     tau = d + n;
     b += align16(2 * (size_t)n * sizeof(T));
@@ -1711,15 +1718,27 @@ int occupancy(K kernel, int threads, size_t smem) {
   return occ;
 }
 
-// Most points of a sub-batch: its per-point workspace within 4 GiB (about 34,600 points at
-// N = 100), so that each launch has enough points to keep every SM busy to its end.
+size_t point_bytes_max(int n) {
+  return std::max({PointWs<float>(n).bytes, PointWs<double>(n).bytes, PointWs<float, double>(n).bytes});
+}
+
+// Most points of a sub-batch. Up to 128 images: per-point workspace within 4 GiB (about 50,000 points
+// at N = 100), so that each launch has enough points to keep every SM busy to its end. Above, where a
+// point has an SM to itself: whole waves of one point per SM, as many as 256 MiB hold, at least one.
+// A sub-batch more costs its eigenpair and tail kernels' latency, 0.27 ms at N = 150: 5,224 points take
+// 42.4 ms in one sub-batch (1,372 MiB with the inverse kept beside the reflectors), 43.2 as set here
+// (235 MiB), 44.3 in waves of five (131 MiB).
 template <typename T>
 int64_t sub_batch(int n) {
-  const PointWs<T> w(n);  // FP64 sub-batches also fit the refined layout (it is smaller)
-  // above 128 images 2 GiB: a wave of one point per SM is enough there
-  const size_t most = n > kMaxFastN ? (size_t)1 << 31 : (size_t)1 << 32, least = n > kMaxFastN ? 296 : 1024;
-  const int64_t def = (int64_t)std::max<size_t>(least, std::min<size_t>(1 << 17, most / (w.bytes + 1)));
   const int64_t cap = g_sub_batch_cap.load();
+  int64_t def;
+  if (n > kMaxFastN) {
+    const int64_t sms = sm_count(), wave = sms * (int64_t)PointWs<double>(n).bytes;
+    def = std::max<int64_t>(1, ((int64_t)1 << 28) / wave) * sms;
+  } else {
+    const size_t bytes = sizeof(T) == 4 ? PointWs<float>(n).bytes : point_bytes_max(n);
+    def = (int64_t)std::max<size_t>(1024, std::min<size_t>(1 << 17, ((size_t)1 << 32) / bytes));
+  }
   return cap > 0 ? std::min(cap, def) : def;
 }
 
@@ -2019,15 +2038,11 @@ int run_refine_pass(const float2* c, PointSet pts, int n, int ref, float2* ph, f
                    : launch_refine<4>(c, pts, n, ref, ph, quality, tcoh, ws, sing, tol, s);
 }
 
-size_t point_bytes_max(int n) {
-  return std::max({PointWs<float>(n).bytes, PointWs<double>(n).bytes, PointWs<float, double>(n).bytes});
-}
-
 }  // namespace
 
 size_t fast_workspace_bytes(int64_t n_pc, int n) {
-  if (n > kMaxFastN)
-    return SubWs::bytes(std::min<int64_t>(n_pc, sub_batch<double>(n)), PointWs<double>(n).bytes, n_pc) +
+  if (n > kMaxFastN)  // FP64 only: no list of points to redo
+    return SubWs::bytes(std::min<int64_t>(n_pc, sub_batch<double>(n)), PointWs<double>(n).bytes, 0) +
            std::min<int64_t>(n_pc, sm_count()) * slice_bytes(n);
   const int64_t s32 = std::min<int64_t>(n_pc, sub_batch<float>(n));
   const int64_t s64 = std::min<int64_t>(n_pc, sub_batch<double>(n));
@@ -2044,11 +2059,13 @@ int fast_run(const float2* coh, int64_t n_pc, int n, int ref, int precision, flo
   auto* ws = static_cast<unsigned char*>(workspace);
   // a mixed or refined sub-batch must hold its points in FP64 when all of them are routed
   const bool wide = f64 || mixed || refine;
-  // sub-batches of equal size (none left nearly empty at the end)
   const int64_t cap = wide ? sub_batch<double>(n) : sub_batch<float>(n);
+  // sub-batches of equal size (none left nearly empty at the end); above 128 images full waves of one
+  // point per SM and the rest
   const int64_t nsub = (n_pc + cap - 1) / cap;
-  const int64_t sub = nsub > 0 ? (n_pc + nsub - 1) / nsub : 0;
-  const SubWs w(ws, sub, wide ? point_bytes_max(n) : PointWs<float>(n).bytes, n_pc);
+  const int64_t sub = n > kMaxFastN ? std::min(cap, n_pc) : nsub > 0 ? (n_pc + nsub - 1) / nsub : 0;
+  const size_t point = n > kMaxFastN ? PointWs<double>(n).bytes : wide ? point_bytes_max(n) : PointWs<float>(n).bytes;
+  const SubWs w(ws, sub, point, n > kMaxFastN ? 0 : n_pc);
   const int64_t npairs = (int64_t)n * (n - 1) / 2;
   const bool routed = mixed || refine;
   if (routed) MR_CUDA_TRY(cudaMemsetAsync(w.count, 0, sizeof(int32_t), s));

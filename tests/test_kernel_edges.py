@@ -388,3 +388,40 @@ def test_raster_where_the_threads_change(cuda, n):
 @pytest.mark.parametrize("n", [128, 129, 255, 256, 257, 511, 512])
 def test_amp_disp_one_pixel_at_a_time(cuda, n):
     test_amp_disp_group_shapes(cuda, n)
+
+
+@pytest.mark.parametrize("n", [129, 150, 157, 158, 160, 200, 257, 400, 512])
+def test_emi_workspace_of_long_stacks_is_bounded(n):
+    """Above 128 images a sub-batch holds 256 MiB of points (reflectors and a few vectors each) or one
+    point per SM, and a matrix per SM beside them, whatever the number of points (148 SMs)."""
+    from moraine_b200 import _lib
+    lib = _lib.load()
+    point, matrix = 8 * n * n + 48 * n + 64, 8 * n * n + 8 * n + 16
+    for points in (1, 7, 148, 296, 740, 1000, 5224, 10 ** 6):
+        most = min(points * point, max(2 ** 28, 148 * point)) + min(points, 148) * matrix + 8192
+        assert lib.mr_emi_workspace_bytes(points, n) <= most
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [129, 158, 200])
+def test_emi_of_long_stacks_in_sub_batches(cuda, n):
+    """More points than a sub-batch holds, and sub-batches that are no whole waves: the same floats."""
+    from moraine_b200 import _lib
+    rng = np.random.default_rng(n)
+    r, s = np.triu_indices(n, 1)
+    z = rng.normal(size=(9, n + 30, n)) + 1j * rng.normal(size=(9, n + 30, n))
+    z += 0.8 * rng.normal(size=(9, n + 30, 1)) * np.exp(1j * rng.uniform(0, 6, (9, 1, n)))
+    c = np.einsum("pli,plj->pij", z, z.conj())
+    d = np.sqrt(np.einsum("pii->pi", c).real)
+    coh = torch.from_numpy((c / (d[:, :, None] * d[:, None, :]))[:, r, s].astype(np.complex64)).to(cuda)
+    ref_ph, ref_q = mb.emi(coh)
+    assert np.isfinite(ref_q.cpu().numpy()).all()
+    lib = _lib.load()
+    try:
+        for points, cap in ((2500, 0), (40, 7), (300, 148), (149, 0)):
+            assert lib.mr_set_emi_sub_batch(cap) == 0
+            pick = torch.arange(points, device=cuda) % 9
+            ph, q = mb.emi(coh[pick].contiguous())
+            assert torch.equal(ph, ref_ph[pick]) and torch.equal(q, ref_q[pick])
+    finally:
+        lib.mr_set_emi_sub_batch(0)
