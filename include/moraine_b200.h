@@ -117,14 +117,15 @@ int mr_ks_test(const float* rmli, int nlines, int width, int nimages, int az_hal
 
 /* Replaces moraine.shp.select_shp (moraine/shp.py:309-323): is_shp = p < p_max (p
  * widened to double; NaN gives 0), shp_num = per-pixel count. */
-/* Tile plans of the KS merge: with autotuning on (off by default), the first mr_ks_test for a
- * (device, nimages, window, raster size within a factor of 4) times the plans for several
+/* Tile plans of the KS kernels: with autotuning on (off by default), the first mr_ks_test for a
+ * (device, nimages, window, kernel, raster size within a factor of 4) times the plans for several
  * shared-memory budgets on its own input, three times each (synchronising the stream; never
  * inside a stream capture), and keeps the one with the fastest median; results do not depend
- * on the plan. Timings are most reliable when nothing else runs on the device, e.g. in a
- * first call before a server starts its slots. mr_ks_plan reports the plan in use (for the
- * largest raster size tuned so far). No reference counterpart (the reference kernel has no
- * tiles). */
+ * on the plan. The kernels: the selection (neither p nor dist asked for) and the statistic. Timings
+ * are most reliable when nothing else runs on the device, e.g. in a first call before a server starts
+ * its slots. mr_ks_plan reports the plan in use for the selection, or for the statistic where only
+ * that kernel's rows fit shared memory (for the largest raster size tuned so far). No reference
+ * counterpart (the reference kernel has no tiles). */
 void mr_set_autotune(int on);
 int mr_ks_plan(int nimages, int az_half_win, int r_half_win, int* tile_rows, int* tile_cols,
                int* az_chunk);

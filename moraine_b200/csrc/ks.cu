@@ -703,13 +703,20 @@ extern "C" int mr_ks_plan(int nimages, int az_half_win, int r_half_win, int* til
                           int* az_chunk) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
-  mr::KsPlan plan = mr::plan_ks(nimages, az_half_win, r_half_win, true);
+  // of the selection kernel; of the statistic kernel, whose rows are shorter, where only that fits
+  // (mr_ks_test takes it there too)
+  bool select = true;
+  mr::KsPlan plan = mr::plan_ks(nimages, az_half_win, r_half_win, select);
+  if (plan.th == 0) {
+    select = false;
+    plan = mr::plan_ks(nimages, az_half_win, r_half_win, select);
+  }
   {
     // the tuned plan of the largest raster size class seen for this shape, if any
     std::lock_guard<std::mutex> lk(mr::g_tune_mu);
     for (const auto& kv : mr::g_tuned)
       if (std::get<0>(kv.first) == dev && std::get<1>(kv.first) == nimages && std::get<2>(kv.first) == az_half_win &&
-          std::get<3>(kv.first) == r_half_win)
+          std::get<3>(kv.first) == r_half_win && std::get<4>(kv.first) == select)
         plan = kv.second;
   }
   if (tile_rows) *tile_rows = plan.th;

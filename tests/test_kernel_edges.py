@@ -425,3 +425,51 @@ def test_emi_of_long_stacks_in_sub_batches(cuda, n):
             assert torch.equal(ph, ref_ph[pick]) and torch.equal(q, ref_q[pick])
     finally:
         lib.mr_set_emi_sub_batch(0)
+
+
+# ----------------------------------------------------------------------------- KS plans
+def _ks_plan(n, azh, rh):
+    import ctypes
+
+    from moraine_b200 import _lib
+    th, tw, azc = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+    rc = _lib.load().mr_ks_plan(n, azh, rh, ctypes.byref(th), ctypes.byref(tw), ctypes.byref(azc))
+    return rc, (th.value, tw.value, azc.value)
+
+
+@pytest.mark.parametrize("n,rh", [(512, 47), (512, 48), (511, 48), (509, 49), (5, 1280), (100, 230)])
+def test_ks_plan_where_only_the_statistic_fits(n, rh):
+    """A shape that mr_ks_test takes has a plan: one pixel and its row of 2 rh + 1 neighbours fit 200 KiB
+    at the statistic kernel's row length."""
+    assert (2 * rh + 2) * ((n + 1) | 1) * 4 <= 200 * 1024
+    rc, plan = _ks_plan(n, 0, rh)
+    assert rc == 0 and min(plan) >= 1
+
+
+def test_ks_plan_refuses_what_fits_neither():
+    assert _ks_plan(512, 0, 60)[0] == -3
+
+
+@pytest.mark.gpu
+def test_ks_plan_is_the_selections(cuda):
+    """Tuning the statistic kernel (p asked for) leaves the reported selection plan alone."""
+    n, azh, rh = 23, 3, 6
+    before = _ks_plan(n, azh, rh)
+    x = torch.rand((40, 50, n), device=cuda)
+    mb.ks_test(x, azh, rh)
+    assert _ks_plan(n, azh, rh) == before
+    _select(x, azh, rh, 0.05)
+    rc, plan = _ks_plan(n, azh, rh)
+    assert rc == 0 and min(plan) >= 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,rh", [(512, 48), (5, 1280)])
+def test_ks_selection_where_only_the_statistic_fits(cuda, n, rh):
+    rng = np.random.default_rng(n)
+    x = rng.exponential(size=(3, 110, n)).astype(np.float32)
+    x[:, 60:] *= 1.6
+    ref, num = O.select_shp(O.ks_test(x, 0, rh), 0.05)
+    got, got_num = _select(torch.from_numpy(x).to(cuda), 0, rh, 0.05)
+    np.testing.assert_array_equal(got.astype(bool), ref)
+    np.testing.assert_array_equal(got_num, num)
