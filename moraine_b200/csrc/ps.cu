@@ -40,52 +40,42 @@ __device__ __forceinline__ float abs_c64_fast(float2 z) {
 }
 
 // kPx pixels per group of G lanes and step, lanes over a pixel's dates (contiguous, image axis
-// innermost; NPL per lane at a time). Sums of a - a_0 and (a - a_0)^2 in FP64, a_0 the pixel's first
+// innermost; NPL per lane). Sums of a - a_0 and (a - a_0)^2 in FP64, a_0 the pixel's first
 // amplitude: the variance about the mean in one pass without cancellation on near-constant (PS)
 // pixels, both sums of all kPx pixels reduced together. Bound by HBM and, below 32 dates a
 // pixel, by the lane sums: 700 x 701 x 30 takes 70 us (with FP64 roots and two sums per
-// pixel one after the other over 16 slots a lane: 383 us). Above 128 dates a pixel keeps a warp
-// busy by itself, and four at a time only leave fewer warps: 40 x 43 x 256 takes 19 us with one and
-// 23 with four, 350 x 353 x 256 119 and 181.
-template <int G, int NPL, int kPx>
+// pixel one after the other over 16 slots a lane: 383 us).
+constexpr int kPx = 4;
+
+template <int G, int NPL>
 __global__ void __launch_bounds__(256) amp_disp_kernel(const float2* __restrict__ z, int64_t npix, int n,
                                                        float* __restrict__ out) {
   const int lane = threadIdx.x & (G - 1);
   const int64_t groups = (int64_t)gridDim.x * (256 / G);
   for (int64_t p0 = ((int64_t)blockIdx.x * (256 / G) + threadIdx.x / G) * kPx; p0 - kPx * (threadIdx.x % 32 / G) < npix;
        p0 += groups * kPx) {  // the test is the same for a whole warp
-    float a0[kPx];
-    double v[2 * kPx];
-    auto add = [&](int k0, bool first) {  // dates k0 .. k0 + G NPL - 1
-      float a[kPx][NPL];
+    float a[kPx][NPL], a0[kPx];
 #pragma unroll
-      for (int q = 0; q < kPx; ++q)
+    for (int q = 0; q < kPx; ++q)
 #pragma unroll
-        for (int t = 0; t < NPL; ++t) {
-          const int k = k0 + lane + G * t;
-          a[q][t] = (k < n && p0 + q < npix) ? abs_c64_fast(z[(p0 + q) * n + k]) : 0.f;
-        }
-#pragma unroll
-      for (int q = 0; q < kPx; ++q) {
-        if (first) {
-          a0[q] = __shfl_sync(0xffffffffu, a[q][0], 0, G);
-          v[2 * q] = v[2 * q + 1] = 0.0;
-        }
-#pragma unroll
-        for (int t = 0; t < NPL; ++t) {
-          const double d = k0 + lane + G * t < n ? (double)a[q][t] - (double)a0[q] : 0.0;
-          v[2 * q] += d;
-          v[2 * q + 1] += d * d;
-        }
+      for (int t = 0; t < NPL; ++t) {
+        const int k = lane + G * t;
+        a[q][t] = (k < n && p0 + q < npix) ? abs_c64_fast(z[(p0 + q) * n + k]) : 0.f;
       }
-    };
-    add(0, true);
-    if constexpr (kPx == 1) {
-#pragma unroll 1
-      for (int k0 = G * NPL; k0 < n; k0 += G * NPL) add(k0, false);
+    double v[2 * kPx];
+#pragma unroll
+    for (int q = 0; q < kPx; ++q) {
+      a0[q] = __shfl_sync(0xffffffffu, a[q][0], 0, G);
+      v[2 * q] = v[2 * q + 1] = 0.0;
+#pragma unroll
+      for (int t = 0; t < NPL; ++t) {
+        const double d = lane + G * t < n ? (double)a[q][t] - (double)a0[q] : 0.0;
+        v[2 * q] += d;
+        v[2 * q + 1] += d * d;
+      }
     }
-    // 2 kPx sums over G >= 8 lanes: each halving hands half of them to the other half of the lanes,
-    // so that lane l ends with sum l / (G / (2 kPx)) of the group
+    // eight sums over G >= 8 lanes: each halving hands half of them to the other half of the lanes,
+    // so that lane l ends with sum l / (G / 8) of the group
     int live = 2 * kPx;
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) {
@@ -103,11 +93,8 @@ __global__ void __launch_bounds__(256) amp_disp_kernel(const float2* __restrict_
       }
     }
     const int q = lane / (G / kPx);  // pixel of the sum that this lane holds
-    const double sq = __shfl_xor_sync(0xffffffffu, v[0], G / (2 * kPx), G);
-    float first = a0[0];
-#pragma unroll
-    for (int e = 1; e < kPx; ++e)
-      if (q == e) first = a0[e];
+    const double sq = __shfl_xor_sync(0xffffffffu, v[0], G / 8, G);
+    const float first = q == 0 ? a0[0] : q == 1 ? a0[1] : q == 2 ? a0[2] : a0[3];
     if (lane % (G / kPx) == 0 && p0 + q < npix) {
       const double m1 = v[0] / n, var = sq / n - m1 * m1;
       // one rounding: near-constant PS pixels keep their digits
@@ -116,11 +103,47 @@ __global__ void __launch_bounds__(256) amp_disp_kernel(const float2* __restrict_
   }
 }
 
-template <int G, int NPL, int kPx = 4>
+// Above 128 dates: one pixel per warp and step, eight dates per lane at a time. A pixel keeps a warp
+// busy by itself there, and four at a time only leave fewer warps: 40 x 43 x 300 takes 19 us against 27
+// with four (16 dates per lane unrolled), 350 x 353 x 512 227 against 479.
+__global__ void __launch_bounds__(256) amp_disp_long_kernel(const float2* __restrict__ z, int64_t npix, int n,
+                                                            float* __restrict__ out) {
+  constexpr int kDates = 8;
+  const int lane = threadIdx.x & 31;
+  for (int64_t p = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); p < npix; p += (int64_t)gridDim.x * 8) {
+    const float2* zp = z + p * n;
+    float first = 0.f;
+    double s1 = 0.0, s2 = 0.0;
+#pragma unroll 1
+    for (int k0 = 0; k0 < n; k0 += 32 * kDates) {
+      float a[kDates];
+#pragma unroll
+      for (int t = 0; t < kDates; ++t) {
+        const int k = k0 + lane + 32 * t;
+        a[t] = k < n ? abs_c64_fast(zp[k]) : 0.f;
+      }
+      if (k0 == 0) first = __shfl_sync(0xffffffffu, a[0], 0);
+#pragma unroll
+      for (int t = 0; t < kDates; ++t) {
+        const double d = k0 + lane + 32 * t < n ? (double)a[t] - (double)first : 0.0;
+        s1 += d;
+        s2 += d * d;
+      }
+    }
+    s1 = warp_sum(s1);
+    s2 = warp_sum(s2);
+    if (lane == 0) {
+      const double m1 = s1 / n, var = s2 / n - m1 * m1;
+      out[p] = (float)(sqrt(var < 0.0 ? 0.0 : var) / ((double)first + m1));
+    }
+  }
+}
+
+template <int G, int NPL>
 void launch_amp_disp(const float2* z, int64_t npix, int n, float* out, cudaStream_t s) {
   const int64_t blocks = (npix + (256 / G) * kPx - 1) / ((256 / G) * kPx);
-  amp_disp_kernel<G, NPL, kPx><<<(unsigned)std::min<int64_t>(blocks, (int64_t)sm_count() * 64), 256, 0, s>>>(
-      z, npix, n, out);
+  amp_disp_kernel<G, NPL><<<(unsigned)std::min<int64_t>(blocks, (int64_t)sm_count() * 64), 256, 0, s>>>(z, npix, n,
+                                                                                                      out);
 }
 
 // calamp: per-block (sum, count) of the non-NaN amplitudes in double, then one block adds
@@ -186,13 +209,14 @@ extern "C" int mr_amp_disp(const mr_complex64* rslc, int64_t npix, int nimages, 
   MR_REQUIRE(rslc && amp_disp, "amp_disp: NULL pointer");
   const auto* z = reinterpret_cast<const float2*>(rslc);
   cudaStream_t s = as_stream(stream);
-  // as many lanes per pixel as it has dates, up to a warp; above 128 dates one pixel at a time
+  // as many lanes per pixel as it has dates, up to a warp
   if (nimages <= 8) launch_amp_disp<8, 1>(z, npix, nimages, amp_disp, s);
   else if (nimages <= 16) launch_amp_disp<16, 1>(z, npix, nimages, amp_disp, s);
   else if (nimages <= 32) launch_amp_disp<32, 1>(z, npix, nimages, amp_disp, s);
   else if (nimages <= 64) launch_amp_disp<32, 2>(z, npix, nimages, amp_disp, s);
   else if (nimages <= 128) launch_amp_disp<32, 4>(z, npix, nimages, amp_disp, s);
-  else launch_amp_disp<32, 8, 1>(z, npix, nimages, amp_disp, s);
+  else amp_disp_long_kernel<<<(unsigned)std::min<int64_t>((npix + 7) / 8, (int64_t)sm_count() * 64), 256, 0, s>>>(
+      z, npix, nimages, amp_disp);
   return check_launch("amp_disp");
 }
 
