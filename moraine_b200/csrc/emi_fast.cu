@@ -291,31 +291,28 @@ template <typename C> __device__ __forceinline__ C half_warp_sum(const C (&r)[4]
 // rows like the compressed coherence ((m, j >= m) at tri_up(m, j)); then, in the arithmetic
 // T of the reduction, the reflectors (column k rows k+1..n-1, packed by column, nq complex
 // T), d and tau (n T each), e (n complex T). The reduction has all of M in its triangle before it
-// writes the first reflector, so the reflectors take the inverse's place, except where the refined
-// tail reads the inverse again.
+// writes the first reflector, so above 128 images (kBig), where the workspace is kept small, the
+// reflectors take the inverse's place: n (n + 1) / 2 reals in n (n - 1) / 2 pairs of them. (Up to 128
+// images that would save a third of 4 GiB, and the refined tail reads the inverse again.)
 __host__ __device__ __forceinline__ int64_t tri_up(int m, int j, int n) {
   return (int64_t)m * n - ((int64_t)m * (m - 1)) / 2 + (j - m);
 }
 
-template <typename T, typename TA = T>
+template <typename T, typename TA = T, bool kBig = false>
 struct PointWs {
   size_t np, nq, bytes;
   __host__ __device__ explicit PointWs(int n) {
     using C = typename C2<T>::type;
     np = (size_t)n * (n + 1) / 2;
     nq = (size_t)n * (n - 1) / 2;
-    bytes = (kRefined ? align16(np * sizeof(TA)) + align16(nq * sizeof(C)) : front(np * sizeof(TA), nq * sizeof(C))) +
-            align16(2 * (size_t)n * sizeof(T)) +
+    bytes = (kBig ? 0 : align16(np * sizeof(TA))) + align16(nq * sizeof(C)) + align16(2 * (size_t)n * sizeof(T)) +
             align16((size_t)n * sizeof(C)) + align16(((size_t)n + 2) * sizeof(T)) +
             (kRefined ? (2 * (size_t)n + 1) * sizeof(double2) : 0);
   }
   static constexpr bool kRefined = sizeof(T) == 4 && sizeof(TA) == 8;
-  static __host__ __device__ __forceinline__ size_t front(size_t ainv, size_t refl) {
-    return align16(ainv > refl ? ainv : refl);
-  }
 };
 
-template <typename T, typename TA = T>
+template <typename T, typename TA = T, bool kBig = false>
 struct PointPtr {
   using C = typename C2<T>::type;
   TA* ainv;
@@ -329,13 +326,12 @@ struct PointPtr {
   double2* x;  // right-hand side and solution of the projected solve,
   double* lam; // Rayleigh quotient
   __device__ PointPtr(unsigned char* ws, int64_t pt, int n) {
-    const PointWs<T, TA> w(n);
+    const PointWs<T, TA, kBig> w(n);
     unsigned char* b = ws + (size_t)pt * w.bytes;
     ainv = reinterpret_cast<TA*>(b);
-    if (PointWs<T, TA>::kRefined) b += align16(w.np * sizeof(TA));
+    if (!kBig) b += align16(w.np * sizeof(TA));
     refl = reinterpret_cast<C*>(b);
-    b += PointWs<T, TA>::kRefined ? align16(w.nq * sizeof(C))
-                                  : PointWs<T, TA>::front(w.np * sizeof(TA), w.nq * sizeof(C));
+    b += align16(w.nq * sizeof(C));
     d = reinterpret_cast<T*>(b);
     tau = d + n;
     b += align16(2 * (size_t)n * sizeof(T));
@@ -615,7 +611,7 @@ __global__ void __launch_bounds__(kBigThreads, 1) big_inverse_kernel(const float
       }
       __syncthreads();
     }
-    double* out = PointPtr<double, double>(ws, pt, n).ainv;
+    double* out = PointPtr<double, double, true>(ws, pt, n).ainv;
     for (int i = wid; i < n; i += W) {
       const int kr = step_of_row[i];
       for (int j = lane; j < n; j += 32) {
@@ -873,7 +869,7 @@ __global__ void __launch_bounds__(32 * W, W >= 3 && QC <= 8 ? (sizeof(T) == 8 ? 
   }
   for (int64_t pt = blockIdx.x; pt < npt; pt += gridDim.x) {
     const float2* c = coh + pts[pt] * npairs;
-    PointPtr<T, TA> w(ws, pt, n);
+    PointPtr<T, TA, (QC > 8)> w(ws, pt, n);
     // M along the upper triangle (inverse and coherence both contiguous there), a warp per row;
     // M_jm = conj(M_mj)
     for (int m = wid; m < n; m += nw) {
@@ -1043,8 +1039,8 @@ __global__ void __launch_bounds__(32 * W, W >= 3 && QC <= 8 ? (sizeof(T) == 8 ? 
 }
 
 // Reflector k of a point (its scalar and the lane's entries, of rows lane + 32 t) into registers.
-template <typename T, typename TA, int NR>
-__device__ __forceinline__ void load_refl(const PointPtr<T, TA>& w, int n, int k, int lane,
+template <typename T, typename TA, bool kBig, int NR>
+__device__ __forceinline__ void load_refl(const PointPtr<T, TA, kBig>& w, int n, int k, int lane,
                                           typename C2<T>::type (&u)[NR], T& tau) {
   tau = w.tau[k];
   const typename C2<T>::type* src = w.refl + refl_off(k, n) - (k + 1);
@@ -1058,8 +1054,8 @@ __device__ __forceinline__ void load_refl(const PointPtr<T, TA>& w, int n, int k
 // z <- H_k z for the reflectors of the workspace, k ascending (forward, Q^H z) or descending (back,
 // Q z), z in registers (row lane + 32 t). A ring of D reflectors is on its way while one is applied,
 // so that the serial chain does not wait on memory. One warp.
-template <typename T, typename TA, int NR>
-__device__ __forceinline__ void apply_q(const PointPtr<T, TA>& w, int n, typename C2<T>::type (&z)[NR], bool forward) {
+template <typename T, typename TA, bool kBig, int NR>
+__device__ __forceinline__ void apply_q(const PointPtr<T, TA, kBig>& w, int n, typename C2<T>::type (&z)[NR], bool forward) {
   using C = typename C2<T>::type;
   constexpr int D = NR * sizeof(C) <= 16 ? 4 : NR * sizeof(C) <= 64 ? 2 : 1;
   const int lane = threadIdx.x & 31, steps = n - 2;
@@ -1094,8 +1090,8 @@ __device__ __forceinline__ void apply_q(const PointPtr<T, TA>& w, int n, typenam
 
 // Phases of the real tridiagonal R = D^H T D: delta_0 = 1, delta_{k+1} = delta_k e_k / |e_k|, as a warp
 // prefix product; lane l gets delta of rows l + 32 t. One warp.
-template <typename V, typename T, typename TA, int NR>
-__device__ __forceinline__ void row_phases(const PointPtr<T, TA>& w, int n, typename C2<V>::type (&dl)[NR]) {
+template <typename V, typename T, typename TA, bool kBig, int NR>
+__device__ __forceinline__ void row_phases(const PointPtr<T, TA, kBig>& w, int n, typename C2<V>::type (&dl)[NR]) {
   using C = typename C2<V>::type;
   const int lane = threadIdx.x & 31;
   C carry = mk<V>(1, 0);
@@ -1199,7 +1195,7 @@ constexpr int kEigThreads = 128;
 
 template <typename T> inline size_t eig_smem(int n, int g) { return 6 * (size_t)n * (kEigThreads / g + 1) * sizeof(T); }
 
-template <typename T, typename TA, int G>
+template <typename T, typename TA, int G, bool kBig>
 __global__ void __launch_bounds__(kEigThreads) tri_eig_kernel(PointSet pts, int n, unsigned char* __restrict__ ws) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int P = kEigThreads / G, S = P + 1;
@@ -1212,7 +1208,7 @@ __global__ void __launch_bounds__(kEigThreads) tri_eig_kernel(PointSet pts, int 
 #pragma unroll 4
     for (int f = tid; f < here * n; f += kEigThreads) {
       const int q = f / n, i = f - q * n;
-      const PointPtr<T, TA> w(ws, base + q, n);
+      const PointPtr<T, TA, kBig> w(ws, base + q, n);
       d0[i * S + q] = w.d[i];
       const typename C2<T>::type e = w.e[min(i, n - 2)];
       b0[i * S + q] = sqrt(e.x * e.x + e.y * e.y);  // entry n - 1 is not used
@@ -1274,7 +1270,7 @@ __global__ void __launch_bounds__(kEigThreads) tri_eig_kernel(PointSet pts, int 
     }
     __syncwarp();
     if (live) {
-      const PointPtr<T, TA> w(ws, base + p, n);
+      const PointPtr<T, TA, kBig> w(ws, base + p, n);
       const T scale = du[0];
       for (int i = g; i < n; i += G) w.y[i] = y[i] * scale;
       if (g == 0) {
@@ -1378,7 +1374,7 @@ __global__ void __launch_bounds__(32 * kTailWarps) tail_kernel(const float2* __r
   const int64_t npt = pts.size();
   for (int64_t pt = (int64_t)blockIdx.x * kTailWarps + wid; pt < npt; pt += (int64_t)gridDim.x * kTailWarps) {
     const int64_t gp = pts[pt];
-    const PointPtr<T, TA> w(ws, pt, n);
+    const PointPtr<T, TA, (NR > 4)> w(ws, pt, n);
     C z[NR];
     row_phases<T>(w, n, z);
 #pragma unroll
@@ -1722,7 +1718,7 @@ size_t point_bytes_max(int n) {
   return std::max({PointWs<float>(n).bytes, PointWs<double>(n).bytes, PointWs<float, double>(n).bytes});
 }
 
-// Most points of a sub-batch. Up to 128 images: per-point workspace within 4 GiB (about 50,000 points
+// Most points of a sub-batch. Up to 128 images: per-point workspace within 4 GiB (about 34,000 points
 // at N = 100), so that each launch has enough points to keep every SM busy to its end. Above, where a
 // point has an SM to itself: whole waves of one point per SM, as many as 256 MiB hold, at least one.
 // A sub-batch more costs its eigenpair and tail kernels' latency, 0.27 ms at N = 150: 5,224 points take
@@ -1733,7 +1729,7 @@ int64_t sub_batch(int n) {
   const int64_t cap = g_sub_batch_cap.load();
   int64_t def;
   if (n > kMaxFastN) {
-    const int64_t sms = sm_count(), wave = sms * (int64_t)PointWs<double>(n).bytes;
+    const int64_t sms = sm_count(), wave = sms * (int64_t)PointWs<double, double, true>(n).bytes;
     def = std::max<int64_t>(1, ((int64_t)1 << 28) / wave) * sms;
   } else {
     const size_t bytes = sizeof(T) == 4 ? PointWs<float>(n).bytes : point_bytes_max(n);
@@ -1931,10 +1927,10 @@ int run_big_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, void
 // else the listed ones, whose count is read on the device), inverse and reduction both in
 // T. cond_max > 0 flags the points whose condition estimate exceeds it.
 // Eigenpair of each point's tridiagonal.
-template <typename T, typename TA, int G>
+template <typename T, typename TA, int G, bool kBig>
 int launch_tri_eig(PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
   const size_t smem = eig_smem<T>(n, G);
-  auto kernel = tri_eig_kernel<T, TA, G>;
+  auto kernel = tri_eig_kernel<T, TA, G, kBig>;
   if (int rc = allow_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
   const int occ = std::max(1, occupancy(kernel, kEigThreads, smem));
   const int64_t ctas = (pts.n_pc + kEigThreads / G - 1) / (kEigThreads / G);
@@ -1942,19 +1938,19 @@ int launch_tri_eig(PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
   return check_launch("emi eigenpair");
 }
 
-template <typename T, typename TA>
+template <typename T, typename TA, bool kBig = false>
 int run_tri_eig(PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
   // Lanes per point by the arithmetic alone: another number of sections moves the last bits of the
   // eigenvalue, and a point's result does not depend on the batch that it is in. FP32: 8 rounds of 8
   // cheap counts; FP64: 13 rounds of 16, whose divisions make each round long.
-  return launch_tri_eig<T, TA, sizeof(T) == 4 ? 8 : 16>(pts, n, ws, s);
+  return launch_tri_eig<T, TA, sizeof(T) == 4 ? 8 : 16, kBig>(pts, n, ws, s);
 }
 
 template <typename T, int NR>
 int launch_tail(const float2* c, PointSet pts, int n, int ref, float2* ph, float* quality, float* tcoh,
                 unsigned char* ws, const uint8_t* sing, cudaStream_t s) {
   KernelTimer kt(pts.list ? "emi tail rerun" : sizeof(T) == 8 ? "emi tail fp64" : "emi tail fp32", s);
-  if (int rc = run_tri_eig<T, T>(pts, n, ws, s)) return rc;
+  if (int rc = run_tri_eig<T, T, (NR > 4)>(pts, n, ws, s)) return rc;
   const size_t tsmem = kTailWarps * (size_t)n * sizeof(double2);
   auto kernel = tail_kernel<T, T, NR>;
   if (int rc = allow_smem(reinterpret_cast<const void*>(kernel), tsmem)) return rc;
@@ -2042,7 +2038,7 @@ int run_refine_pass(const float2* c, PointSet pts, int n, int ref, float2* ph, f
 
 size_t fast_workspace_bytes(int64_t n_pc, int n) {
   if (n > kMaxFastN)  // FP64 only: no list of points to redo
-    return SubWs::bytes(std::min<int64_t>(n_pc, sub_batch<double>(n)), PointWs<double>(n).bytes, 0) +
+    return SubWs::bytes(std::min<int64_t>(n_pc, sub_batch<double>(n)), PointWs<double, double, true>(n).bytes, 0) +
            std::min<int64_t>(n_pc, sm_count()) * slice_bytes(n);
   const int64_t s32 = std::min<int64_t>(n_pc, sub_batch<float>(n));
   const int64_t s64 = std::min<int64_t>(n_pc, sub_batch<double>(n));
@@ -2064,7 +2060,8 @@ int fast_run(const float2* coh, int64_t n_pc, int n, int ref, int precision, flo
   // point per SM and the rest
   const int64_t nsub = (n_pc + cap - 1) / cap;
   const int64_t sub = n > kMaxFastN ? std::min(cap, n_pc) : nsub > 0 ? (n_pc + nsub - 1) / nsub : 0;
-  const size_t point = n > kMaxFastN ? PointWs<double>(n).bytes : wide ? point_bytes_max(n) : PointWs<float>(n).bytes;
+  const size_t point = n > kMaxFastN ? PointWs<double, double, true>(n).bytes
+                       : wide        ? point_bytes_max(n) : PointWs<float>(n).bytes;
   const SubWs w(ws, sub, point, n > kMaxFastN ? 0 : n_pc);
   const int64_t npairs = (int64_t)n * (n - 1) / 2;
   const bool routed = mixed || refine;
