@@ -473,3 +473,22 @@ def test_ks_selection_where_only_the_statistic_fits(cuda, n, rh):
     got, got_num = _select(torch.from_numpy(x).to(cuda), 0, rh, 0.05)
     np.testing.assert_array_equal(got.astype(bool), ref)
     np.testing.assert_array_equal(got_num, num)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "refine", "mixed"])
+@pytest.mark.parametrize("n", [2, 3, 5, 17, 33])
+def test_emi_singular_point_of_a_short_stack(cuda, n, precision):
+    """|Gamma| = ones meets an exact zero pivot at every size, two images included: NaN for that point,
+    and nothing else changes."""
+    rng = np.random.default_rng(n)
+    q = n * (n - 1) // 2
+    coh = (0.3 * np.exp(1j * rng.uniform(0, 6, (6, q))) * rng.uniform(0.2, 1, (6, q))).astype(np.complex64)
+    ph, quality = mb.emi(coh, precision=precision)
+    assert np.isfinite(quality).all()
+    coh[3] = 1.0
+    ph2, quality2 = mb.emi(coh, precision=precision)
+    assert np.isnan(ph2[3]).all() and np.isnan(quality2[3])
+    keep = np.arange(6) != 3
+    np.testing.assert_array_equal(ph2[keep], ph[keep])
+    np.testing.assert_array_equal(quality2[keep], quality[keep])
