@@ -156,8 +156,8 @@ EMI_TRAFFIC_PER_POINT = {(100, "fp64"): 356_500, (100, "fp32"): 239_900}
 
 # DRAM bytes per unit of one kernel (dram__bytes_read.sum + dram__bytes_write.sum of one launch
 # / the units it processed), from one-kernel ncu captures on the 512 x 512 x 100 crop of the c2
-# scene model (profiles/*_c2_512.md); the traffic of these kernels scales with the units, so a
-# full-size launch gets units x bytes. Keyed by (kernel, N); DS points, pixels for the KS merge.
+# scene model; the traffic of these kernels scales with the units, so a full-size launch gets
+# units x bytes. Keyed by (kernel, N); DS points, pixels for the KS step ("ks merge": the selection).
 KERNEL_TRAFFIC_PER_UNIT = {
     ("emi reduce fp32", 100): (2.774624e9 + 1.388484e9) / 34_510,
     ("emi refine tail", 100): (11.547766e9 + 366.030e6) / 34_510,  # its four kernels

@@ -96,7 +96,7 @@ def load() -> ctypes.CDLL:
             fn = getattr(lib, name)
             fn.restype = res
             fn.argtypes = args
-        # tune the KS merge tiles on first use of each (device, nimages, window): one stream
+        # tune the KS tiles on first use of each (device, nimages, window, kernel): one stream
         # synchronisation, then the fastest plan; results do not depend on it
         lib.mr_set_autotune(1)
         _lib = lib

@@ -14,8 +14,8 @@
 //   2. M = inv(|Gamma|) o Gamma;
 //   3. Householder reduction M = Q T Q^H, T Hermitian tridiagonal, then a diagonal unitary
 //      scaling T = D R D^H with R real symmetric tridiagonal;
-//   4. lambda_min(R) by Sturm-count multisection on one warp;
-//   5. its eigenvector y by inverse iteration on R - lambda I (pivoted tridiagonal LU);
+//   4. lambda_min(R) by Sturm-count multisection, a group of lanes per point;
+//   5. its eigenvector y by two inverse iterations on R - lambda I (pivoted tridiagonal LU);
 //   6. v = Q D y.
 // The kernels are in emi_fast.cu: in the arithmetic asked for up to 128 images, in FP64 above.
 #include <algorithm>

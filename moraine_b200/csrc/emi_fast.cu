@@ -16,7 +16,7 @@
 //                          reduction to a Hermitian tridiagonal -> workspace (d, e, tau,
 //                          reflectors).
 //   tri_eig_kernel         smallest eigenpair of the real tridiagonal: Sturm counts and inverse
-//                          iteration, several points per warp.
+//                          iteration (two solves), several points per warp.
 //   tail_kernel            one warp per point: back-transformation, normalisation, temporal
 //                          coherence.
 //   refine_*_kernel        the refined EMI's tail: one FP64 Newton correction of the FP32
@@ -831,8 +831,8 @@ __global__ void __launch_bounds__(256, 2) sweep_kernel(const float2* __restrict_
 // divisions) and the short strips of B, hidden only by the other CTAs of the SM. The previous form
 // (256 threads, three barriers, groups of four threads on mirrored row pairs, row and column parts in
 // separate passes over M): FP32, N = 17, 2,047 points 146 us, now 37; N = 50, 35,627 points 8.4 ms,
-// now 3.5; N = 100, 286,294 points 199 ms, now 164; FP64, N = 17, 1,003 points 157 us, now 38; N = 100,
-// 4,001 points 6.2 ms, now 5.4. FP32 in packed pairs (fma.f32x2 on rows and columns laid out twice)
+// now 3.6; N = 100, 286,294 points 199 ms, now 165; FP64, N = 17, 1,003 points 157 us, now 37; N = 100,
+// 4,001 points 6.2 ms, now 5.1. FP32 in packed pairs (fma.f32x2 on rows and columns laid out twice)
 // was slower, 204 ms: its sums and doubled vectors cost registers and shared memory.
 // The vectors of a step, one record per row: kRowPad zero records in front (rows above the first of a
 // strip) and kColPad behind (columns past the last). u, w: of step k-1; c: u_k.
@@ -1804,7 +1804,6 @@ int launch_inverse(const float2* coh, PointSet pts, int64_t grid_cap, int n, uns
   return check_launch("emi inverse");
 }
 
-// inv(|Gamma|) in arithmetic TA into a workspace laid out for a reduction in T.
 template <typename T, int NM, typename TW>
 int launch_warp_inverse(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t* sing, float cond_max,
                         cudaStream_t s) {
@@ -1847,6 +1846,7 @@ size_t slice_bytes(int n) {
   return align16(std::max((size_t)n * n * sizeof(double), reduce_tri(n) * sizeof(double2)));
 }
 
+// inv(|Gamma|) in arithmetic TA into a workspace laid out for a reduction in T.
 template <typename TA, typename T>
 int run_inverse(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t* sing, float cond_max,
                 cudaStream_t s) {
@@ -1883,7 +1883,8 @@ template <typename T, typename TA>
 int run_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
   // Warps per point and rows per half-warp strip. Up to 64 images one warp needs no waiting on other
   // warps and an SM holds many points (FP64, N = 50, 4,001 points: one warp 0.78 ms, two 1.02);
-  // above, shared memory holds two to four points per SM, and more warps each hide their latencies:
+  // above, shared memory holds two to four points per SM, and more warps each hide their latencies
+  // (times of a build before the row sums had their own array; it takes 165 and 5.1 ms now):
   // N = 100, FP32, 1, 2, 4, 8 warps of 4 rows: 243, 222, 178, 285 ms for 286,294 points; FP64, 4 and 8
   // warps of 4 rows 6.5 and 6.2, of 2 rows (128 registers, two CTAs of 8 warps) 6.4 and 5.8 ms for
   // 4,001 points.
@@ -1923,9 +1924,6 @@ int run_big_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, void
   return launch_reduce<double, double, 32, 2, 8, false>(c, pts, n, ws, s, sl);
 }
 
-// One pass of the three kernels over a sub-batch (pts.list == nullptr: all pts.n_pc points;
-// else the listed ones, whose count is read on the device), inverse and reduction both in
-// T. cond_max > 0 flags the points whose condition estimate exceeds it.
 // Eigenpair of each point's tridiagonal.
 template <typename T, typename TA, int G, bool kBig>
 int launch_tri_eig(PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
@@ -1941,8 +1939,10 @@ int launch_tri_eig(PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
 template <typename T, typename TA, bool kBig = false>
 int run_tri_eig(PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
   // Lanes per point by the arithmetic alone: another number of sections moves the last bits of the
-  // eigenvalue, and a point's result does not depend on the batch that it is in. FP32: 8 rounds of 8
-  // cheap counts; FP64: 13 rounds of 16, whose divisions make each round long.
+  // eigenvalue, and a point's result does not depend on the batch that it is in. FP32 8 (30,000 points at
+  // N = 100: 4, 8, 16, 32 lanes 354, 275, 402, 673 us; 35,000 at N = 50 121, 146, 253, 400). FP64 16, of
+  // 8, 16 and 32: few points are faster with more lanes (1,003 at N = 17 34, 30, 26 us; 1,332 at N = 150
+  // 187, 165, 154), many with fewer (30,000 at N = 100 942, 904, 1,515; 35,000 at N = 50 339, 549, 893).
   return launch_tri_eig<T, TA, sizeof(T) == 4 ? 8 : 16, kBig>(pts, n, ws, s);
 }
 
@@ -1960,6 +1960,9 @@ int launch_tail(const float2* c, PointSet pts, int n, int ref, float2* ph, float
   return check_launch("emi tail");
 }
 
+// One pass of inverse, reduction, eigenpair and tail over a sub-batch (pts.list == nullptr: all
+// pts.n_pc points; else the listed ones, whose count is read on the device), inverse and reduction
+// both in T. cond_max > 0 flags the points whose condition estimate exceeds it.
 template <typename T>
 int run_pass(const float2* c, PointSet pts, int n, int ref, float2* ph, float* quality, float* tcoh,
              unsigned char* ws, uint8_t* sing, float cond_max, void* slices, cudaStream_t s) {

@@ -499,7 +499,7 @@ KsPlan plan_ks(int n, int azh, int rh, bool select, size_t budget = 200 * 1024) 
         size_t px = (size_t)th * tw + (size_t)(th + azc - 1) * (tw + 2 * rh);
         size_t bytes = px * best.ss * 4;
         if (bytes > budget) continue;
-        // merges per loaded pixel, preferring full warps of reference pixels
+        // pairs per loaded pixel, preferring full warps of reference pixels
         int nchunks = (az_win + azc - 1) / azc;
         double loaded = (double)th * tw + (double)nchunks * (th + azc - 1) * (tw + 2 * rh);
         double score = (double)th * tw / loaded * (th * tw >= 32 ? 1.0 : 0.5);
@@ -562,7 +562,7 @@ extern "C" size_t mr_ks_workspace_bytes(int nlines, int width, int nimages) {
 namespace mr {
 namespace {
 
-// Autotuned merge plans: the heuristic plans for several shared-memory budgets (large
+// Autotuned plans: the heuristic plans for several shared-memory budgets (large
 // tiles with one CTA per SM down to small tiles with several) are timed on the first call
 // for a (device, N, window, raster size class) and the fastest is kept. Each candidate is
 // timed three times and ranked by its median, so that a burst of other work on the device
@@ -620,14 +620,14 @@ int launch_select(const KsJob& j, const KsPlan& plan, unsigned tiles, cudaStream
   }
 }
 
-int launch_merge(const KsJob& j, const KsPlan& plan, cudaStream_t s) {
+int launch_ks(const KsJob& j, const KsPlan& plan, cudaStream_t s) {
   const int64_t tiles = (int64_t)((j.nlines + plan.th - 1) / plan.th) * ((j.width + plan.tw - 1) / plan.tw);
   MR_REQUIRE(tiles < (1ll << 31), "ks_test: image too large");
   const int r_win = 2 * j.rh + 1;
   // offsets per thread: 3 or 4, whichever loads less over a row of r_win offsets (2 per offset
   // and 2 for the reference pixel, the last group padded)
   const bool three = (r_win + 2) / 3 * 8 <= (r_win + 3) / 4 * 10;
-  KernelTimer kt("ks merge", s);
+  KernelTimer kt("ks merge", s);  // the name that this step is timed under, whichever kernel it runs
   if (j.select) {
     if (int rc = three ? launch_select<3>(j, plan, (unsigned)tiles, s) : launch_select<4>(j, plan, (unsigned)tiles, s))
       return rc;
@@ -644,10 +644,10 @@ int launch_merge(const KsJob& j, const KsPlan& plan, cudaStream_t s) {
       const int64_t npix = (int64_t)j.nlines * j.width;
       const int grid = (int)std::min<int64_t>((npix + 7) / 8, (int64_t)sm_count() * 16);
       count_shp_kernel<<<grid, 256, 0, s>>>(j.is_shp, npix, (2 * j.azh + 1) * (2 * j.rh + 1), j.shp_num);
-      return check_launch("ks_test merge", 2);
+      return check_launch("ks_test", 2);
     }
   }
-  return check_launch("ks_test merge");
+  return check_launch("ks_test");
 }
 
 // The plan for this call: tuned when asked and possible (never inside a stream capture).
@@ -672,11 +672,11 @@ int choose_plan(KsPlan& plan, const KsJob& j, cudaStream_t s) {
   KsPlan pick = plan;
   int rc = MR_OK;
   for (const KsPlan& c : plan_candidates(j.n, j.azh, j.rh, j.select)) {
-    if ((rc = launch_merge(j, c, s))) break;  // warm
+    if ((rc = launch_ks(j, c, s))) break;  // warm
     float t[3] = {0.f, 0.f, 0.f};
     for (int r = 0; r < 3 && !rc; ++r) {
       cudaEventRecord(e0, s);
-      if ((rc = launch_merge(j, c, s))) break;
+      if ((rc = launch_ks(j, c, s))) break;
       cudaEventRecord(e1, s);
       if (cudaEventSynchronize(e1) != cudaSuccess) { rc = fail(MR_ERR_CUDA, "ks_test: autotune timing failed"); break; }
       cudaEventElapsedTime(&t[r], e0, e1);
@@ -768,7 +768,7 @@ extern "C" int mr_ks_test(const float* rmli, int nlines, int width, int nimages,
   if (plan.th == 0)
     return fail(MR_ERR_UNSUPPORTED, "ks_test: nimages %d with half windows (%d, %d) does not fit shared memory",
                 nimages, az_half_win, r_half_win);
-  return launch_merge(job, plan, s);
+  return launch_ks(job, plan, s);
 }
 
 extern "C" int mr_select_shp(const float* p, int64_t npix, int win, double p_max, uint8_t* is_shp,

@@ -5,10 +5,11 @@
 // HBM-streaming passes over the same (nlines, width, nimages) complex64 stack the DS chain
 // reads.
 //
-// |z| is the float32 rounding of the double square root of the exact double sum of squares,
-// +inf when either part is infinite: bit-exact with np.abs on complex64 in the reference's
-// Numba build (numpy's own hypotf can differ in the last bit). Means and standard
-// deviations accumulate in double and the ratio rounds once to float32.
+// rslc2amp: |z| is the float32 rounding of the double square root of the exact double sum of
+// squares, +inf when either part is infinite: bit-exact with np.abs on complex64 in the
+// reference's Numba build (numpy's own hypotf can differ in the last bit). amp_disp takes |z| from a
+// compensated FP32 root, which gives another float (by one ulp) for about one amplitude in a million;
+// its means and standard deviations accumulate in double and the ratio rounds once to float32.
 #include <algorithm>
 
 #include "common.cuh"
