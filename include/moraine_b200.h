@@ -253,8 +253,8 @@ int mr_gamma_decode(const void* be, int64_t n, int dtype, void* out, int64_t out
 size_t mr_emi_workspace_bytes(int64_t n_pc, int nimages);
 
 /* EMI runs in sub-batches of points (per-point state in the workspace, by default at most 4 GiB of
- * it, about 34,000 points at N = 100; above 128 images 256 MiB, or one point per SM where that is
- * more, and for more than 157 images a matrix per SM beside them). mr_set_emi_sub_batch(m) caps a
+ * it, about 34,000 points at N = 100; above 128 images 256 MiB, or four points per SM where that
+ * is more, and for more than 157 images a matrix per SM beside them). mr_set_emi_sub_batch(m) caps a
  * sub-batch at m points (0 restores the default; negative: MR_ERR_INVALID), which lowers
  * mr_emi_workspace_bytes for later calls; a workspace sized before a larger cap was set is
  * rejected (MR_ERR_WORKSPACE). Process-wide. No reference counterpart. */

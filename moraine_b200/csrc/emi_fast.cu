@@ -1720,17 +1720,18 @@ size_t point_bytes_max(int n) {
 
 // Most points of a sub-batch. Up to 128 images: per-point workspace within 4 GiB (about 34,000 points
 // at N = 100), so that each launch has enough points to keep every SM busy to its end. Above, where a
-// point has an SM to itself: whole waves of one point per SM, as many as 256 MiB hold, at least one.
-// A sub-batch more costs its eigenpair and tail kernels' latency, 0.27 ms at N = 150: 5,224 points take
-// 42.4 ms in one sub-batch (1,372 MiB with the inverse kept beside the reflectors), 43.2 as set here
-// (235 MiB), 44.3 in waves of five (131 MiB).
+// point has an SM to itself: whole waves of one point per SM, as many as 256 MiB hold, at least four
+// (from 200 images on; with the slices less than the dense matrices of two points per SM). A sub-batch
+// more costs its eigenpair and tail kernels' latency, 0.27 ms at N = 150: 5,224 points take 42.3 ms in
+// one sub-batch (1,372 MiB with the inverse kept beside the reflectors), 43.0 as set here (235 MiB),
+// 44.3 in waves of five (131 MiB). 1,000 points at N = 400 543 ms either way (2,026 and 911 MiB).
 template <typename T>
 int64_t sub_batch(int n) {
   const int64_t cap = g_sub_batch_cap.load();
   int64_t def;
   if (n > kMaxFastN) {
     const int64_t sms = sm_count(), wave = sms * (int64_t)PointWs<double, double, true>(n).bytes;
-    def = std::max<int64_t>(1, ((int64_t)1 << 28) / wave) * sms;
+    def = std::max<int64_t>(4, ((int64_t)1 << 28) / wave) * sms;
   } else {
     const size_t bytes = sizeof(T) == 4 ? PointWs<float>(n).bytes : point_bytes_max(n);
     def = (int64_t)std::max<size_t>(1024, std::min<size_t>(1 << 17, ((size_t)1 << 32) / bytes));

@@ -392,13 +392,13 @@ def test_amp_disp_one_pixel_at_a_time(cuda, n):
 
 @pytest.mark.parametrize("n", [129, 150, 157, 158, 160, 200, 257, 400, 512])
 def test_emi_workspace_of_long_stacks_is_bounded(n):
-    """Above 128 images a sub-batch holds 256 MiB of points (reflectors and a few vectors each) or one
-    point per SM, and a matrix per SM beside them, whatever the number of points (148 SMs)."""
+    """Above 128 images a sub-batch holds 256 MiB of points (reflectors and a few vectors each) or four
+    points per SM, and a matrix per SM beside them, whatever the number of points (148 SMs)."""
     from moraine_b200 import _lib
     lib = _lib.load()
     point, matrix = 8 * n * n + 48 * n + 64, 8 * n * n + 8 * n + 16
     for points in (1, 7, 148, 296, 740, 1000, 5224, 10 ** 6):
-        most = min(points * point, max(2 ** 28, 148 * point)) + min(points, 148) * matrix + 8192
+        most = min(points * point, max(2 ** 28, 4 * 148 * point)) + min(points, 148) * matrix + 8192
         assert lib.mr_emi_workspace_bytes(points, n) <= most
 
 
