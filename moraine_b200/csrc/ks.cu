@@ -581,7 +581,10 @@ int size_class(int64_t npix) {
 
 std::vector<KsPlan> plan_candidates(int n, int azh, int rh, bool select) {
   std::vector<KsPlan> out;
-  for (size_t budget : {200u * 1024u, 100u * 1024u, 64u * 1024u, 40u * 1024u, 28u * 1024u, 20u * 1024u}) {
+  for (size_t budget : {200u * 1024u, 100u * 1024u, 64u * 1024u, 40u * 1024u, 28u * 1024u, 20u * 1024u, 12u * 1024u,
+                        6u * 1024u}) {
+    // short series and small windows, of which 20 KiB still hold more than 64 pixels at a time
+    if (budget < 20u * 1024u && (out.empty() || out.back().th * out.back().tw <= 64)) break;
     const KsPlan c = plan_ks(n, azh, rh, select, budget);
     if (c.th == 0) continue;
     bool dup = false;
@@ -625,11 +628,15 @@ int launch_ks(const KsJob& j, const KsPlan& plan, cudaStream_t s) {
   MR_REQUIRE(tiles < (1ll << 31), "ks_test: image too large");
   const int r_win = 2 * j.rh + 1;
   // offsets per thread: 3 or 4, whichever loads less over a row of r_win offsets (2 per offset
-  // and 2 for the reference pixel, the last group padded)
-  const bool three = (r_win + 2) / 3 * 8 <= (r_win + 3) / 4 * 10;
+  // and 2 for the reference pixel, the last group padded); 1 where a row is a single offset, of which
+  // groups of 3 would do each three times, or where groups would leave threads of the tile without any
+  int ko = r_win == 1 ? 1 : (r_win + 2) / 3 * 8 <= (r_win + 3) / 4 * 10 ? 3 : 4;
+  if (plan.azc * ((r_win + ko - 1) / ko) < kKsThreads / (plan.th * plan.tw)) ko = 1;
   KernelTimer kt("ks merge", s);  // the name that this step is timed under, whichever kernel it runs
   if (j.select) {
-    if (int rc = three ? launch_select<3>(j, plan, (unsigned)tiles, s) : launch_select<4>(j, plan, (unsigned)tiles, s))
+    if (int rc = ko == 1   ? launch_select<1>(j, plan, (unsigned)tiles, s)
+                 : ko == 3 ? launch_select<3>(j, plan, (unsigned)tiles, s)
+                           : launch_select<4>(j, plan, (unsigned)tiles, s))
       return rc;
   } else {
     auto go = [&](auto kernel) {
@@ -639,7 +646,7 @@ int launch_ks(const KsJob& j, const KsPlan& plan, cudaStream_t s) {
                                                             j.is_shp);
       return (int)MR_OK;
     };
-    if (int rc = three ? go(ks_stat_kernel<3>) : go(ks_stat_kernel<4>)) return rc;
+    if (int rc = ko == 1 ? go(ks_stat_kernel<1>) : ko == 3 ? go(ks_stat_kernel<3>) : go(ks_stat_kernel<4>)) return rc;
     if (j.shp_num) {
       const int64_t npix = (int64_t)j.nlines * j.width;
       const int grid = (int)std::min<int64_t>((npix + 7) / 8, (int64_t)sm_count() * 16);

@@ -98,6 +98,24 @@ def test_ks_selection_without_p(cuda, n, azh, rh):
     np.testing.assert_array_equal(mb.ks_test(x, azh, rh), p)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,azh,rh", [(5, 4, 0), (17, 0, 0), (41, 5, 0), (100, 1, 1), (200, 0, 5), (512, 1, 1)])
+def test_ks_one_offset_per_thread(cuda, n, azh, rh):
+    """Windows of one column, and windows so small that groups of offsets would leave threads idle."""
+    rng = np.random.default_rng(n)
+    x = rng.exponential(size=(11, 23, n)).astype(np.float32)
+    x[:, 12:] *= 2.5
+    x[3, 5] = x[3, 6]
+    x[5, 9, 0] = np.nan
+    p = O.ks_test(x, azh, rh)
+    np.testing.assert_array_equal(mb.ks_test(x, azh, rh), p)
+    for p_max in (0.05, 0.5, 1.0, 2.5):
+        ref, num = O.select_shp(p, p_max)
+        got, got_num = _select(torch.from_numpy(x).to(cuda), azh, rh, p_max)
+        np.testing.assert_array_equal(got.astype(bool), ref)
+        np.testing.assert_array_equal(got_num, num)
+
+
 # ----------------------------------------------------------------------------- coherence
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [2, 3, 4, 5, 8, 9, 17, 31, 40, 57, 76, 77, 104, 105, 137, 200, 301, 409])
