@@ -8,7 +8,6 @@
 //                          summed in window order (row-major over the az x r window)
 //   moraine/co.py:83-110   raster: cov = sum / n_shp, coh as above, every (m, j)
 #include <algorithm>
-#include <vector>
 
 #include "common.cuh"
 
@@ -518,12 +517,13 @@ __global__ void __launch_bounds__(32 * WARPS, gram64_ctas(SLOTS, WARPS)) gram64_
 
 // Runs of at most `cap` blocks for n images: each block row br has the blocks bc = 2 br .. nc - 1,
 // cut into pieces of cap; what is left of each row is paired with another rest, longest with the
-// longest that still fits.
+// longest that still fits. No heap: the plan is made inside a C entry point, at each call.
 GramPlan cut_gram64(int n, int cap) {
   struct Piece { int br, bc, len; };
   const int nc = (n + 7) / 8, nr = (n + 15) / 16;
   GramPlan plan{};
-  std::vector<Piece> rest;
+  Piece rest[kDmmaImages / 16];  // longest first
+  int left = 0;
   auto add = [&](Piece a, Piece b) {
     if (plan.runs < kMaxRuns)
       plan.run[plan.runs] = {(uint8_t)a.br, (uint8_t)a.bc, (uint8_t)a.len, (uint8_t)b.br, (uint8_t)b.bc,
@@ -534,16 +534,17 @@ GramPlan cut_gram64(int n, int cap) {
   for (int br = 0; br < nr; ++br) {
     int bc = 2 * br;
     for (; nc - bc >= cap; bc += cap) add({br, bc, cap}, {0, 0, 0});
-    if (bc < nc) rest.push_back({br, bc, nc - bc});
+    if (bc >= nc) continue;
+    int at = left++;
+    for (; at > 0 && rest[at - 1].len < nc - bc; --at) rest[at] = rest[at - 1];
+    rest[at] = {br, bc, nc - bc};
   }
-  std::sort(rest.begin(), rest.end(), [](const Piece& a, const Piece& b) { return a.len > b.len; });
-  while (!rest.empty()) {
-    const Piece a = rest.front();
-    rest.erase(rest.begin());
-    auto b = std::find_if(rest.begin(), rest.end(), [&](const Piece& p) { return a.len + p.len <= cap; });
-    if (b == rest.end()) { add(a, {0, 0, 0}); continue; }
-    add(a, *b);
-    rest.erase(b);
+  for (int i = 0; i < left; ++i) {
+    if (rest[i].len == 0) continue;  // taken
+    int j = i + 1;
+    while (j < left && (rest[j].len == 0 || rest[i].len + rest[j].len > cap)) ++j;
+    add(rest[i], j < left ? rest[j] : Piece{0, 0, 0});
+    if (j < left) rest[j].len = 0;
   }
   plan.warps = plan.runs;
   return plan;

@@ -2,6 +2,7 @@
 index logic (CPU), and the device against the oracle or the general path (GPU)."""
 import math
 import re
+import subprocess
 from pathlib import Path
 
 import numpy as np
@@ -326,6 +327,56 @@ def test_fp64_gram_is_the_same_on_every_path(cuda, n):
     inside = j < n
     wide = mb.emperical_co_pc(z, idx, mask, precision="fp64")
     np.testing.assert_array_equal(wide[:, inside], few)
+
+
+_PLAN_CHECK = r"""
+#include <algorithm>
+#include <cstdint>
+#include <cstdio>
+#include <cstdlib>
+#include <new>
+bool closed = false;
+void* operator new(std::size_t n) { if (closed) throw std::bad_alloc(); return std::malloc(n); }
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, std::size_t) noexcept { std::free(p); }
+@SOURCE@
+int main() {
+  int made = 0;
+  closed = true;
+  for (int n = 2; n <= kDmmaImages; ++n)
+    for (int64_t points : {1, 296, 297, 4736, 4737, 1000000}) {
+      GramShape shape;
+      GramPlan plan;
+      try { plan = plan_gram64(n, points, 148, shape); } catch (...) { std::printf("heap at %d\n", n); return 1; }
+      const int nc = (n + 7) / 8, nr = (n + 15) / 16;
+      int seen[8][16] = {};
+      if (plan.runs < 1 || plan.runs > kMaxRuns || plan.warps != plan.runs || plan.runs > shape.warps) return 2;
+      for (int r = 0; r < plan.runs; ++r) {
+        const GramRun& g = plan.run[r];
+        if (g.cnt > plan.slots || plan.slots > shape.slots || g.c1 > g.cnt || !g.cnt) return 3;
+        for (int q = 0; q < g.cnt; ++q) ++seen[q < g.c1 ? g.br1 : g.br2][q < g.c1 ? g.bc1 + q : g.bc2 + q - g.c1];
+      }
+      for (int i = 0; i < 8; ++i)
+        for (int j = 0; j < 16; ++j)
+          if (seen[i][j] != (i < nr && j < nc && j >= 2 * i)) { std::printf("n %d block %d %d: %d\n", n, i, j, seen[i][j]); return 4; }
+      ++made;
+    }
+  std::printf("%d plans\n", made);
+}
+"""
+
+
+def test_gram_plans_hold_each_block_once_without_the_heap(tmp_path):
+    """Every plan of the FP64 tensor kernel deals each block of the triangle to one warp within its CTA
+    shape, and is made without an allocation, which could throw through the C interface."""
+    src = (Path(mb.__file__).parent / "csrc" / "coh.cu").read_text()
+    head = src[src.index("constexpr int kMaxRuns"):src.index("__device__ __forceinline__ void dmma")]
+    plans = src[src.index("GramPlan cut_gram64"):src.index("// Whether gram64_kernel takes n images")]
+    code = tmp_path / "plans.cpp"
+    code.write_text(_PLAN_CHECK.replace("@SOURCE@", "#include <vector>\n" + head + plans))
+    subprocess.run(["g++", "-std=c++17", "-O1", "-o", tmp_path / "plans", code], check=True)
+    out = subprocess.run([tmp_path / "plans"], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout
 
 
 def _integers_of_square_sum(total, k, rng):
