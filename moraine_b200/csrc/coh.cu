@@ -578,7 +578,8 @@ GramPlan fit_gram64(int n, int warps, int most) {
 // against 253 us: there with more than 16 points per SM.
 // Few points, at most two per SM, end sooner with more warps each whatever the images (200 points,
 // 11 x 21 window, N = 64 58 against 62 us, N = 104 98 against 108; with six per SM that lost: N = 64,
-// 900 points 118 against 111).
+// 900 points 118 against 111). At most one per SM: eight warps always (148 points, N = 84 44 against 56 us
+// with six, N = 96 50 against 60; but 296 points, N = 84 81 against 67).
 // Up to 24 images one warp can hold all blocks of a point; it wastes no step on an idle warp, but a
 // point takes longer, so it is taken where every SM has more than 32 points (11 x 21 window, 20,000
 // points: N = 17 438 against 550 us, N = 24 448 against 567; 5,000 points 152 against 153 and 156
@@ -589,7 +590,8 @@ struct GramShape {
   int warps, slots;
 };
 constexpr GramShape kManyPoints[] = {{4, 7}, {8, 4}, {6, 7}, {4, 13}, {8, 9}};
-constexpr GramShape kFewPoints[] = {{8, 4}, {6, 7}, {8, 9}};
+constexpr GramShape kTwoPerSm[] = {{8, 4}, {6, 7}, {8, 9}};
+constexpr GramShape kOnePerSm[] = {{8, 9}};
 
 // The plan, and in `shape` the CTA shape of the kernel that holds it.
 GramPlan plan_gram64(int n, int64_t n_pc, int sms, GramShape& shape) {
@@ -606,7 +608,8 @@ GramPlan plan_gram64(int n, int64_t n_pc, int sms, GramShape& shape) {
       }
     }
   };
-  if (n_pc <= (int64_t)sms * 2) first(kFewPoints);
+  if (n_pc <= sms) first(kOnePerSm);
+  else if (n_pc <= (int64_t)sms * 2) first(kTwoPerSm);
   else first(kManyPoints);
   return plan;
 }

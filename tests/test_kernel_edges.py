@@ -344,7 +344,7 @@ int main() {
   int made = 0;
   closed = true;
   for (int n = 2; n <= kDmmaImages; ++n)
-    for (int64_t points : {1, 296, 297, 4736, 4737, 1000000}) {
+    for (int64_t points : {1, 148, 149, 296, 297, 4736, 4737, 1000000}) {
       GramShape shape;
       GramPlan plan;
       try { plan = plan_gram64(n, points, 148, shape); } catch (...) { std::printf("heap at %d\n", n); return 1; }
