@@ -104,11 +104,11 @@ __device__ __forceinline__ void copy8(float2* dst, const float2* src) {
 // against 2.9 with a separate pass for |z|^2 and 256-thread CTAs; N = 20 raster of 123 x 131: 0.16
 // against 0.38 ms. FP64 at N = 150, 8,000 points of 95 SHPs: 4.7 against 5.0 ms.
 //
-// A CTA has up to 192 threads, or up to 256 (fewer of them per SM) where that takes a round less: FP32
-// at any number of points (N = 80, 4,000 points, 11 x 21 window: 444 against 331 us; N = 112 735 and
-// 620; N = 200 2,129 and 1,736; with the same rounds at N = 68 the 256 lost, 74 against 76 % of the
-// time of the kernel before), FP64 with at most two points per SM (N = 152, 200 points: 210 against
-// 184 us; but 4,000 points 1,999 against 2,172).
+// A CTA has up to 192 threads, or up to 256, two of them per SM, where that takes a round less. FP32: N = 80,
+// 4,000 points, 11 x 21 window 444 against 331 us, N = 112 735 and 620, N = 200 2,129 and 1,736 (with the
+// same rounds the 256 lost: N = 68 74 against 76 % of the time of the kernel before). FP64, 15 x 31 window:
+// 900 points, N = 150 1,153 against 960 us, N = 190 2,058 and 1,792, N = 320 6,457 and 5,549; 3,000 points,
+// N = 174 4,739 and 3,873; one CTA of 256 threads and up to 255 registers was no faster than the 192.
 constexpr int kGramThreads = 192, kWideGramThreads = 256;
 
 template <typename A> struct GramAcc;
@@ -163,7 +163,7 @@ __device__ __forceinline__ void load_block(const double2* row, int nb, int b, do
 }
 
 template <typename A, bool kFull, int MT>
-__global__ void __launch_bounds__(MT, (sizeof(A) == 8 ? 2 : 3) - (MT == kWideGramThreads)) gram_kernel(
+__global__ void __launch_bounds__(MT, sizeof(A) == 8 || MT == kWideGramThreads ? 2 : 3) gram_kernel(
     const float2* __restrict__ rslc, int nlines, int width, int n, const int32_t* __restrict__ idx,
     int64_t n_pc, const uint8_t* __restrict__ mask, int mask_stride, int az_win, int r_win,
     float2* __restrict__ coh, float2* __restrict__ cov, const int64_t* __restrict__ dcount, int64_t doff, int kc) {
@@ -693,8 +693,7 @@ int launch_gram(const float2* rslc, int nlines, int width, int n, const int32_t*
                 cudaStream_t s, const int64_t* dcount = nullptr, int64_t doff = 0) {
   const int nb = (n + 3) / 4, nblk = nb * (nb + 1) / 2;
   auto rounds = [&](int threads) { return (nblk + threads - 1) / threads; };
-  const bool wide = rounds(kWideGramThreads) < rounds(kGramThreads) &&
-                    (sizeof(A) == 4 || n_pc <= (int64_t)sm_count() * 2);
+  const bool wide = rounds(kWideGramThreads) < rounds(kGramThreads);
   return wide ? launch_gram_of<A, kFull, kWideGramThreads>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win,
                                                            r_win, coh, cov, s, dcount, doff)
               : launch_gram_of<A, kFull, kGramThreads>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win,
