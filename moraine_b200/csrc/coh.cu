@@ -86,8 +86,9 @@ __device__ __forceinline__ void copy8(float2* dst, const float2* src) {
 // One CTA per point (grid-stride), a 4 x 4 block of the Gram's upper triangle per thread and
 // round, over the point's SHPs staged kc rows at a time. The launch gives a point only as many
 // warps as its blocks fill; several CTAs share an SM.
-// kFull = false: writes coh (n_pc, Q) in triu order.
-// kFull = true : writes cov and coh (npix, N, N) (raster form), the lower blocks as conjugates.
+// kOut = kTriu  : writes coh (n_pc, Q) in triu order.
+// kOut = kRaster: writes cov and coh (npix, N, N) (raster form), the lower blocks as conjugates;
+//        kRasterPairs: two values to a store (raster_pairs).
 //
 // A staged row holds its images in the arithmetic A, permuted so that the 16-byte words
 // that a thread reads lie 16 bytes from its neighbour's (no bank conflict): image 4 b + r at
@@ -162,13 +163,44 @@ __device__ __forceinline__ void load_block(const double2* row, int nb, int b, do
   for (int r = 0; r < 4; ++r) z[r] = row[r * nb + b];
 }
 
-template <typename A, bool kFull, int MT>
+enum GramOut { kTriu, kRaster, kRasterPairs };
+
+// Columns col and col + 1 of a row of n values, n even and the row 16-byte aligned.
+__device__ __forceinline__ void put2(float2* row, int col, int n, float px, float py, float qx, float qy) {
+  if (col < n) *reinterpret_cast<float4*>(row + col) = make_float4(px, py, qx, qy);
+}
+
+// Rows 4 bm + a and the next of a finished block of coherence (rr, ii) and covariance (ir, ri), and off the
+// diagonal their conjugate transpose.
+__device__ __forceinline__ void write_rows(float2* coh, float2* cov, int n, int bm, int bj, int a,
+                                           const GramAcc<float> (&v)[2][4]) {
+  const int m = 4 * bm + a, j = 4 * bj;
+  if (m >= n) return;
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int b = 0; b < 4; b += 2) {
+      const GramAcc<float> &p = v[r][b], &q = v[r][b + 1];
+      put2(coh + (m + r) * n, j + b, n, p.rr, p.ii, q.rr, q.ii);
+      put2(cov + (m + r) * n, j + b, n, p.ir, p.ri, q.ir, q.ri);
+    }
+  if (bm == bj) return;
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+    if (j + b < n) {
+      const GramAcc<float> &p = v[0][b], &q = v[1][b];
+      put2(coh + (j + b) * n, m, n, p.rr, -p.ii, q.rr, -q.ii);
+      put2(cov + (j + b) * n, m, n, p.ir, -p.ri, q.ir, -q.ri);
+    }
+}
+
+template <typename A, GramOut kOut, int MT>
 __global__ void __launch_bounds__(MT, sizeof(A) == 8 || MT == kWideGramThreads ? 2 : 3) gram_kernel(
     const float2* __restrict__ rslc, int nlines, int width, int n, const int32_t* __restrict__ idx,
     int64_t n_pc, const uint8_t* __restrict__ mask, int mask_stride, int az_win, int r_win,
     float2* __restrict__ coh, float2* __restrict__ cov, const int64_t* __restrict__ dcount, int64_t doff, int kc) {
   using C = typename cplx<A>::type;
-  constexpr bool kWide = sizeof(A) == 8;
+  constexpr bool kWide = sizeof(A) == 8, kFull = kOut != kTriu;
   constexpr int V = 16 / sizeof(C);  // images per 16-byte word
   if (dcount) {  // points doff .. doff + n_pc - 1 of a count held on the device
     const int64_t c = *dcount - doff;
@@ -297,7 +329,24 @@ __global__ void __launch_bounds__(MT, sizeof(A) == 8 || MT == kWideGramThreads ?
         }
         __syncthreads();
       }
-      if (active) {
+      if constexpr (kOut == kRasterPairs) {
+        if (active) {
+          const int64_t o = i * n * n;
+#pragma unroll
+          for (int a = 0; a < 4; a += 2) {
+            GramAcc<float> v[2][4];
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+              for (int b = 0; b < 4; ++b) {
+                const A den = sqrt(amp2[4 * bm + a + r] * amp2[4 * bj + b]);
+                const A re = acc[a + r][b].re(), im = acc[a + r][b].im();
+                v[r][b] = {re / den, im / den, re / (A)S, im / (A)S};
+              }
+            write_rows(coh + o, cov + o, n, bm, bj, a, v);
+          }
+        }
+      } else if (active) {
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
@@ -667,7 +716,7 @@ unsigned gram_grid(K kernel, int threads, size_t smem, int64_t n_pc) {
   return (unsigned)std::min<int64_t>(n_pc, (int64_t)sm_count() * occ * 8);
 }
 
-template <typename A, bool kFull, int MT>
+template <typename A, GramOut kOut, int MT>
 int launch_gram_of(const float2* rslc, int nlines, int width, int n, const int32_t* idx, int64_t n_pc,
                    const uint8_t* mask, int mask_stride, int az_win, int r_win, float2* coh, float2* cov,
                    cudaStream_t s, const int64_t* dcount, int64_t doff) {
@@ -680,24 +729,32 @@ int launch_gram_of(const float2* rslc, int nlines, int width, int n, const int32
   const int kc = chunk_rows(kWide ? 16 : 32, row);
   const size_t smem = kc * row + (kWide ? ((size_t)kc * n + 1) / 2 * 2 * sizeof(float2) : 0) + (kWide ? 2 : 1) * 4 * nb * sizeof(A) +
                       (size_t)az_win * r_win * sizeof(int);
-  if (int rc = allow_smem(reinterpret_cast<const void*>(gram_kernel<A, kFull, MT>), smem)) return rc;
+  if (int rc = allow_smem(reinterpret_cast<const void*>(gram_kernel<A, kOut, MT>), smem)) return rc;
   KernelTimer kt(kWide ? "gram fp64" : "gram fp32", s);
-  gram_kernel<A, kFull, MT><<<gram_grid(gram_kernel<A, kFull, MT>, threads, smem, n_pc), threads, smem, s>>>(
+  gram_kernel<A, kOut, MT><<<gram_grid(gram_kernel<A, kOut, MT>, threads, smem, n_pc), threads, smem, s>>>(
       rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win, r_win, coh, cov, dcount, doff, kc);
   return check_launch("coherence gram");
 }
 
-template <typename A, bool kFull>
+// Two values to a store in the raster form: the transposed blocks' values go to a row each, 32 lines to an
+// instruction, which takes most of the time of long stacks with few SHPs. 50 x 51 pixels, 3 x 3 window, N = 64
+// 155 us one by one and 95 in pairs, N = 80 216 and 145; 15 x 31 window 323 and 309, 460 and 421. Below 24
+// images the pairs' registers cost more than the stores (N = 20, 3 x 3: 20 and 22).
+bool raster_pairs(int n, const float2* coh, const float2* cov) {
+  return n >= 24 && !(n & 1) && !((reinterpret_cast<uintptr_t>(coh) | reinterpret_cast<uintptr_t>(cov)) & 15);
+}
+
+template <typename A, GramOut kOut>
 int launch_gram(const float2* rslc, int nlines, int width, int n, const int32_t* idx, int64_t n_pc,
                 const uint8_t* mask, int mask_stride, int az_win, int r_win, float2* coh, float2* cov,
                 cudaStream_t s, const int64_t* dcount = nullptr, int64_t doff = 0) {
   const int nb = (n + 3) / 4, nblk = nb * (nb + 1) / 2;
   auto rounds = [&](int threads) { return (nblk + threads - 1) / threads; };
   const bool wide = rounds(kWideGramThreads) < rounds(kGramThreads);
-  return wide ? launch_gram_of<A, kFull, kWideGramThreads>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win,
-                                                           r_win, coh, cov, s, dcount, doff)
-              : launch_gram_of<A, kFull, kGramThreads>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win,
-                                                       r_win, coh, cov, s, dcount, doff);
+  return wide ? launch_gram_of<A, kOut, kWideGramThreads>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win,
+                                                          r_win, coh, cov, s, dcount, doff)
+              : launch_gram_of<A, kOut, kGramThreads>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win,
+                                                      r_win, coh, cov, s, dcount, doff);
 }
 
 int launch_gram64(const float2* rslc, int nlines, int width, int n, const int32_t* idx, int64_t n_pc,
@@ -705,7 +762,7 @@ int launch_gram64(const float2* rslc, int nlines, int width, int n, const int32_
                   const int64_t* dcount = nullptr, int64_t doff = 0) {
   const int sms = sm_count();
   if (!dmma_images(n, n_pc, sms))
-    return launch_gram<double, false>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win, r_win, coh,
+    return launch_gram<double, kTriu>(rslc, nlines, width, n, idx, n_pc, mask, mask_stride, az_win, r_win, coh,
                                       nullptr, s, dcount, doff);
   const int nr = (n + 15) / 16;
   GramShape shape;
@@ -765,7 +822,7 @@ extern "C" int mr_emperical_co_pc(const mr_complex64* rslc, int nlines, int widt
   }
   switch (precision) {
     case MR_PREC_FP32:
-      return launch_gram<float, false>(z, nlines, width, nimages, idx, n_pc, mask, mask_stride, az_win, r_win,
+      return launch_gram<float, kTriu>(z, nlines, width, nimages, idx, n_pc, mask, mask_stride, az_win, r_win,
                                        out, nullptr, s);
     case MR_PREC_FP64:
       return launch_gram64(z, nlines, width, nimages, idx, n_pc, mask, mask_stride, az_win, r_win, out, s);
@@ -821,7 +878,7 @@ int gram_counted(const float2* rslc, int nlines, int width, int n, const int32_t
                  int precision, cudaStream_t s) {
   if (n_max <= 0) return MR_OK;
   if (precision == MR_PREC_FP32)
-    return launch_gram<float, false>(rslc, nlines, width, n, idx, n_max, mask, 1, az_win, r_win, coh, nullptr, s,
+    return launch_gram<float, kTriu>(rslc, nlines, width, n, idx, n_max, mask, 1, az_win, r_win, coh, nullptr, s,
                                      dcount, doff);
   if (precision == MR_PREC_FP64)
     return launch_gram64(rslc, nlines, width, n, idx, n_max, mask, 1, az_win, r_win, coh, s, dcount, doff);
@@ -837,8 +894,9 @@ extern "C" int mr_emperical_co(const mr_complex64* rslc, int nlines, int width, 
   MR_REQUIRE(az_win > 0 && r_win > 0 && (az_win & 1) && (r_win & 1), "emperical_co: window must be odd");
   if (nimages > MR_MAX_NIMAGES) return fail(MR_ERR_UNSUPPORTED, "emperical_co: nimages > %d", MR_MAX_NIMAGES);
   if ((int64_t)az_win * r_win > MR_MAX_WINDOW) return fail(MR_ERR_UNSUPPORTED, "emperical_co: window too large");
-  return launch_gram<float, true>(reinterpret_cast<const float2*>(rslc), nlines, width, nimages, nullptr,
-                                  (int64_t)nlines * width, is_shp, 1, az_win, r_win,
-                                  reinterpret_cast<float2*>(coh), reinterpret_cast<float2*>(cov),
-                                  as_stream(stream));
+  auto* c = reinterpret_cast<float2*>(coh);
+  auto* v = reinterpret_cast<float2*>(cov);
+  const auto launch = raster_pairs(nimages, c, v) ? launch_gram<float, kRasterPairs> : launch_gram<float, kRaster>;
+  return launch(reinterpret_cast<const float2*>(rslc), nlines, width, nimages, nullptr, (int64_t)nlines * width, is_shp,
+                1, az_win, r_win, c, v, as_stream(stream), nullptr, 0);
 }

@@ -454,6 +454,30 @@ def test_raster_where_the_threads_change(cuda, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [22, 23, 24, 25, 26, 30, 64, 79, 80, 114])
+def test_raster_written_in_pairs(cuda, n):
+    """Where two values go to a store, and the same floats in buffers that allow one only."""
+    from moraine_b200 import _dev, _lib
+    rng = np.random.default_rng(n)
+    z = (rng.normal(size=(5, 7, n)) + 1j * rng.normal(size=(5, 7, n))).astype(np.complex64)
+    is_shp = rng.random((5, 7, 5, 3)) < 0.5
+    is_shp[..., 2, 1] = True
+    cov_ref, coh_ref = O.emperical_co(z, is_shp)
+    cov, coh = mb.emperical_co(z, is_shp)
+    np.testing.assert_allclose(coh, coh_ref, atol=2e-6, rtol=0)
+    np.testing.assert_allclose(cov, cov_ref, atol=2e-6 * np.abs(cov_ref).max(), rtol=0)
+    zt, mt = torch.from_numpy(z).to(cuda), torch.from_numpy(is_shp.astype(np.uint8)).to(cuda)
+    size = coh.size
+    for cov_at, coh_at in ((0, 1), (1, 0), (1, 1)):
+        out = [torch.zeros(size + 2, dtype=torch.complex64, device=cuda) for _ in range(2)]
+        _lib.call("mr_emperical_co", zt.data_ptr(), 5, 7, n, mt.data_ptr(), 5, 3, out[0].data_ptr() + 8 * cov_at,
+                  out[1].data_ptr() + 8 * coh_at, _dev.stream())
+        for buf, at, want in ((out[0], cov_at, cov), (out[1], coh_at, coh)):
+            np.testing.assert_array_equal(buf[at:at + size].cpu().numpy(), want.reshape(-1))
+            assert not buf[:at].any() and not buf[at + size:].any()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n", [128, 129, 255, 256, 257, 511, 512])
 def test_amp_disp_one_pixel_at_a_time(cuda, n):
     test_amp_disp_group_shapes(cuda, n)
