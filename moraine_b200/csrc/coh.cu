@@ -711,6 +711,7 @@ __global__ void gram_pairs_kernel(const float2* __restrict__ rslc, int nlines, i
 // so their times, differ), each walking its share.
 template <class K>
 unsigned gram_grid(K kernel, int threads, size_t smem, int64_t n_pc) {
+  if (n_pc <= (int64_t)sm_count() * 8) return (unsigned)n_pc;  // whatever the occupancy
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem) != cudaSuccess || occ < 1) occ = 1;
   return (unsigned)std::min<int64_t>(n_pc, (int64_t)sm_count() * occ * 8);

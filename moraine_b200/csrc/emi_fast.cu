@@ -1714,6 +1714,14 @@ int occupancy(K kernel, int threads, size_t smem) {
   return occ;
 }
 
+// CTAs of a launch that walks `ctas` CTAs' worth of points: no more than are resident at once. One per SM
+// always are, so that calls of few points, whose time is their launches', do not ask the runtime.
+template <class K>
+unsigned resident_grid(K kernel, int threads, size_t smem, int64_t ctas) {
+  const int64_t sms = sm_count();
+  return (unsigned)(ctas <= sms ? ctas : std::min<int64_t>(ctas, sms * std::max(1, occupancy(kernel, threads, smem))));
+}
+
 size_t point_bytes_max(int n) {
   return std::max({PointWs<float>(n).bytes, PointWs<double>(n).bytes, PointWs<float, double>(n).bytes});
 }
@@ -1798,10 +1806,9 @@ template <typename T, int NB, typename TW>
 int launch_inverse(const float2* coh, PointSet pts, int64_t grid_cap, int n, unsigned char* ws, uint8_t* sing,
                    float cond_max, cudaStream_t s) {
   constexpr int CX = gj_cx<T>();
-  const int occ = std::max(1, occupancy(inverse_kernel<T, NB, CX, TW>, 16 * CX, 0));
-  const int64_t grid = std::min<int64_t>(grid_cap, (int64_t)sm_count() * occ);
+  const unsigned grid = resident_grid(inverse_kernel<T, NB, CX, TW>, 16 * CX, 0, grid_cap);
   KernelTimer kt(pts.list ? "emi inverse rerun" : sizeof(T) == 8 ? "emi inverse fp64" : "emi inverse fp32", s);
-  inverse_kernel<T, NB, CX, TW><<<(unsigned)grid, 16 * CX, 0, s>>>(coh, pts, n, ws, sing, cond_max);
+  inverse_kernel<T, NB, CX, TW><<<grid, 16 * CX, 0, s>>>(coh, pts, n, ws, sing, cond_max);
   return check_launch("emi inverse");
 }
 
@@ -1809,11 +1816,10 @@ template <typename T, int NM, typename TW>
 int launch_warp_inverse(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t* sing, float cond_max,
                         cudaStream_t s) {
   auto kernel = warp_inverse_kernel<T, NM, TW>;
-  const int occ = std::max(1, occupancy(kernel, 32 * kWarpInvWarps, 0));
   const int64_t ctas = (pts.n_pc + kWarpInvWarps - 1) / kWarpInvWarps;
   KernelTimer kt(pts.list ? "emi inverse rerun" : sizeof(T) == 8 ? "emi inverse fp64" : "emi inverse fp32", s);
-  kernel<<<(unsigned)std::min<int64_t>(ctas, (int64_t)sm_count() * occ), 32 * kWarpInvWarps, 0, s>>>(c, pts, n, ws,
-                                                                                                    sing, cond_max);
+  kernel<<<resident_grid(kernel, 32 * kWarpInvWarps, 0, ctas), 32 * kWarpInvWarps, 0, s>>>(c, pts, n, ws, sing,
+                                                                                          cond_max);
   return check_launch("emi inverse");
 }
 
@@ -1871,12 +1877,10 @@ int launch_reduce(const float2* c, PointSet pts, int n, unsigned char* ws, cudaS
   const size_t rsmem = reduce_smem<T>(n, W, kTriIn);
   auto kernel = reduce_kernel<T, TA, QC, R, W, kTriIn>;
   if (int rc_ = allow_smem(reinterpret_cast<const void*>(kernel), rsmem)) return rc_;
-  const int rocc = occupancy(kernel, 32 * W, rsmem);
-  if (rocc < 1) return fail(MR_ERR_UNSUPPORTED, "emi: %zu bytes of shared memory per CTA do not fit", rsmem);
   KernelTimer kt(pts.list ? "emi reduce rerun" : sizeof(T) == 8 ? "emi reduce fp64" : "emi reduce fp32", s);
   // one slice of the workspace per SM where the triangle is not in shared memory
-  const int64_t most = (int64_t)sm_count() * (kTriIn ? rocc : 1);
-  kernel<<<(unsigned)std::min<int64_t>(pts.n_pc, most), 32 * W, rsmem, s>>>(c, pts, n, ws, slices);
+  const int64_t most = kTriIn ? pts.n_pc : std::min<int64_t>(pts.n_pc, sm_count());
+  kernel<<<resident_grid(kernel, 32 * W, rsmem, most), 32 * W, rsmem, s>>>(c, pts, n, ws, slices);
   return check_launch("emi reduce");
 }
 
@@ -1931,9 +1935,8 @@ int launch_tri_eig(PointSet pts, int n, unsigned char* ws, cudaStream_t s) {
   const size_t smem = eig_smem<T>(n, G);
   auto kernel = tri_eig_kernel<T, TA, G, kBig>;
   if (int rc = allow_smem(reinterpret_cast<const void*>(kernel), smem)) return rc;
-  const int occ = std::max(1, occupancy(kernel, kEigThreads, smem));
   const int64_t ctas = (pts.n_pc + kEigThreads / G - 1) / (kEigThreads / G);
-  kernel<<<(unsigned)std::min<int64_t>(ctas, (int64_t)sm_count() * occ), kEigThreads, smem, s>>>(pts, n, ws);
+  kernel<<<resident_grid(kernel, kEigThreads, smem, ctas), kEigThreads, smem, s>>>(pts, n, ws);
   return check_launch("emi eigenpair");
 }
 
@@ -1955,9 +1958,8 @@ int launch_tail(const float2* c, PointSet pts, int n, int ref, float2* ph, float
   const size_t tsmem = kTailWarps * (size_t)n * sizeof(double2);
   auto kernel = tail_kernel<T, T, NR>;
   if (int rc = allow_smem(reinterpret_cast<const void*>(kernel), tsmem)) return rc;
-  const int tocc = std::max(1, occupancy(kernel, 32 * kTailWarps, tsmem));
-  const int64_t tgrid = std::min<int64_t>((pts.n_pc + kTailWarps - 1) / kTailWarps, (int64_t)sm_count() * tocc);
-  kernel<<<(unsigned)tgrid, 32 * kTailWarps, tsmem, s>>>(c, pts, n, ref, ws, sing, ph, quality, tcoh);
+  const unsigned tgrid = resident_grid(kernel, 32 * kTailWarps, tsmem, (pts.n_pc + kTailWarps - 1) / kTailWarps);
+  kernel<<<tgrid, 32 * kTailWarps, tsmem, s>>>(c, pts, n, ref, ws, sing, ph, quality, tcoh);
   return check_launch("emi tail");
 }
 
@@ -1984,10 +1986,9 @@ int run_pass(const float2* c, PointSet pts, int n, int ref, float2* ph, float* q
 
 template <int NB>
 int launch_sweep(const float2* c, PointSet pts, int n, unsigned char* ws, uint8_t* sing, cudaStream_t s) {
-  const int occ = std::max(1, occupancy(sweep_kernel<NB, float>, 256, 0));
-  const int64_t grid = std::min<int64_t>(pts.n_pc, (int64_t)sm_count() * occ);
+  const unsigned grid = resident_grid(sweep_kernel<NB, float>, 256, 0, pts.n_pc);
   KernelTimer kt(pts.list ? "emi sweep rerun" : "emi sweep fp64", s);
-  sweep_kernel<NB, float><<<(unsigned)grid, 256, 0, s>>>(c, pts, n, ws, sing);
+  sweep_kernel<NB, float><<<grid, 256, 0, s>>>(c, pts, n, ws, sing);
   return check_launch("emi sweep");
 }
 
@@ -2015,8 +2016,7 @@ int launch_refine(const float2* c, PointSet pts, int n, int ref, float2* ph, flo
   if (int rc = allow_smem(reinterpret_cast<const void*>(kb), wsmem)) return rc;
   if (int rc = allow_smem(reinterpret_cast<const void*>(refine_solve_kernel), ssmem)) return rc;
   auto grid = [&](auto kernel, int threads, size_t smem, int points) {
-    const int occ = std::max(1, occupancy(kernel, threads, smem));
-    return (unsigned)std::min<int64_t>((pts.n_pc + points - 1) / points, (int64_t)sm_count() * occ);
+    return resident_grid(kernel, threads, smem, (pts.n_pc + points - 1) / points);
   };
   ka<<<grid(ka, 32 * kRefineWarps, wsmem, kRefineWarps), 32 * kRefineWarps, wsmem, s>>>(c, pts, n, ws);
   refine_solve_kernel<<<grid(refine_solve_kernel, kSolveThreads, ssmem, kSolvePoints), kSolveThreads, ssmem, s>>>(

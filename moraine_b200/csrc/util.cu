@@ -54,6 +54,9 @@ int smem_optin() {
 }
 
 int allow_smem(const void* kernel, size_t bytes) {
+  // 48 KiB need no leave, and no kernel here has more than 16 of static shared memory: two runtime calls
+  // less for small launches, whose time is the host's
+  if (bytes <= 32 * 1024) return MR_OK;
   const int optin = smem_optin();
   if (optin <= 0) return fail(MR_ERR_CUDA, "cannot query the shared-memory limit of the device");
   cudaFuncAttributes fa;
