@@ -5,11 +5,10 @@
 // HBM-streaming passes over the same (nlines, width, nimages) complex64 stack the DS chain
 // reads.
 //
-// rslc2amp: |z| is the float32 rounding of the double square root of the exact double sum of
-// squares, +inf when either part is infinite: bit-exact with np.abs on complex64 in the
-// reference's Numba build (numpy's own hypotf can differ in the last bit). amp_disp takes |z| from a
-// compensated FP32 root, which gives another float (by one ulp) for about one amplitude in a million;
-// its means and standard deviations accumulate in double and the ratio rounds once to float32.
+// |z| is the float32 rounding of the double square root of the exact double sum of squares,
+// +inf when either part is infinite: bit-exact with np.abs on complex64 in the reference's
+// Numba build (numpy's own hypotf can differ in the last bit). Means and standard
+// deviations accumulate in double and the ratio rounds once to float32.
 #include <algorithm>
 
 #include "common.cuh"
@@ -27,9 +26,10 @@ __global__ void rslc2amp_kernel(const float2* __restrict__ z, int64_t n, float* 
     amp[i] = abs_c64(z[i]);
 }
 
-// |z| to within a fraction of a float32 ulp in FP32: x^2 + y^2 as a sum with its rounding errors, the
-// approximate root corrected by its residual. Squares near the ends of the FP32 range, NaN and
-// infinities take the FP64 path.
+// The floats of abs_c64 without its FP64 root: x^2 + y^2 as an FP32 sum with its rounding errors, the
+// approximate root corrected by its residual, together within 2^-41 of |z| (rsqrtf to 2 ulp). Where
+// 2^-40 to either side would round to another float (2e-5 of the samples) the FP64 path decides; so it
+// does for squares near the ends of the FP32 range, NaN and infinities.
 __device__ __forceinline__ float abs_c64_fast(float2 z) {
   const float p = z.x * z.x, h = z.y * z.y;
   const float s = p + h;
@@ -37,7 +37,9 @@ __device__ __forceinline__ float abs_c64_fast(float2 z) {
   const float big = fmaxf(p, h), small = fminf(p, h);
   const float lo = (small - (s - big)) + (fmaf(z.x, z.x, -p) + fmaf(z.y, z.y, -h));
   const float y = rsqrtf(s), r = s * y;
-  return fmaf(fmaf(-r, r, s) + lo, 0.5f * y, r);
+  const float e = fmaf(-r, r, s) + lo, off = s * 0x1p-39f, half = 0.5f * y;
+  const float a = fmaf(e - off, half, r);
+  return a == fmaf(e + off, half, r) ? a : abs_c64(z);
 }
 
 // kPx pixels per group of G lanes and step, lanes over a pixel's dates (contiguous, image axis

@@ -585,3 +585,36 @@ def test_emi_singular_point_of_a_short_stack(cuda, n, precision):
     keep = np.arange(6) != 3
     np.testing.assert_array_equal(ph2[keep], ph[keep])
     np.testing.assert_array_equal(quality2[keep], quality[keep])
+
+
+def _amplitudes_beside_midpoints(count, rng):
+    """complex64 samples x + iy of integers with x^2 + y^2 = m^2 + 1, m odd between 2^24 and 2^25: |z| lies
+    1 / 2m above the middle m between two floats. (x - 1)(x + 1) = (m - y)(m + y) with m - y = a,
+    x = a t + 1, m + y = t (a t + 2)."""
+    t = rng.integers(3, 1500, 4_000_000)
+    a = rng.integers(2 ** 25, 2 ** 26, t.size) // t ** 2 + 1
+    x, b = a * t + 1, t * (a * t + 2)
+    m, y = (a + b) // 2, (b - a) // 2
+    ok = ((a + b) % 2 == 0) & (m % 2 == 1) & (m > 2 ** 24) & (m < 2 ** 25) & (y > 0)
+    ok &= (x == x.astype(np.float32)) & (y == y.astype(np.float32))
+    x, y, m = (v[ok][:count] for v in (x, y, m))
+    assert len(m) == count and (x * x + y * y == m * m + 1).all()
+    return x, y, m
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 9, 30, 100, 129, 300])
+def test_amp_disp_rounds_amplitudes_like_the_double_root(cuda, n):
+    """One date whose |z| lies just beside the middle between two floats, the others a few ulps away: the
+    dispersion shows to which float it was rounded."""
+    x, y, m = _amplitudes_beside_midpoints(400, np.random.default_rng(7))
+    z = (x + 1j * y).astype(np.complex64)
+    a = (m + 1).astype(np.float32)  # the float above the middle
+    assert np.array_equal(a, np.sqrt(x.astype(np.float64) ** 2 + y.astype(np.float64) ** 2).astype(np.float32))
+    rest = (a + 3 * np.spacing(a)).astype(np.float32)
+    stack = np.repeat(rest[:, None], n, axis=1).astype(np.complex64)
+    stack[:, n - 1] = z
+    d = a.astype(np.float64) - rest
+    want = np.sqrt(d * d / n - (d / n) ** 2) / (rest + d / n)
+    got = mb.amp_disp(stack.reshape(20, 20, n)).reshape(-1)
+    np.testing.assert_allclose(got, want, rtol=1e-6)  # another float would be 33 or 25 % off
